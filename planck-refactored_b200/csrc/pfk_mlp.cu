@@ -12,6 +12,17 @@
 //   dZ_L = 2 (Y - T) / (n d_L);  dW_l = H_{l-1}^T bf16(dZ_l);
 //   db_l = column sums of dZ_l;  dH_{l-1} = bf16(dZ_l) W_l^T;
 //   dZ_{l-1} = dH_{l-1} * SiLU'(Z_{l-1}).
+//
+// A training step is 2L + 2 launches for L layers: the input conversion, L
+// forward products (the last one also forms dZ_L and the loss), L - 1
+// products for dH (their epilogue applies SiLU' and leaves dZ), one launch
+// for the weight gradients of every layer, and the update.  Each product
+// leaves its result in both orders (rows of the batch, and transposed), so
+// every product reads both operands as rows of K by 16-byte copies.  On the
+// 112-256-256-232 network (one B200): 2048 rows, a step 135 us against 1675 us
+// before (products staged by 2-byte gathers, bias sums by one thread per
+// column, weight gradients on 8 CTAs, two host synchronisations); forward of
+// 8192 rows 73 us against 250 us (both with the host call).
 // The reference has no counterpart: it is the learned part of the guess
 // hook (scf.cpp:206-240 selects the guess; a learned density enters the SCF
 // as a ReadDensity guess does, scf.cpp:213-216).
@@ -29,29 +40,32 @@ namespace {
 thread_local std::string g_mlp_error;
 
 // ---------------------------------------------------------------------------
-// GEMM on the fifth-generation tensor cores: C[m][n] = sum_k A(m, k) B(k, n),
-// A(m,k) = A[m*lda + k] (or A[k*lda + m] when TA), B(k,n) = B[k*ldb + n] (or
-// B[n*ldb + k] when TB); BF16 operands, FP32 accumulation in tensor memory;
-// the epilogue adds bias[n] and writes C (FP32) and/or H = bf16(SiLU(C)).
+// GEMM on the fifth-generation tensor cores: acc[m][n] = sum_k A[m][k] B[n][k]
+// with both operands stored as rows of K (BF16, row strides lda and ldb, every
+// row start 16-byte aligned), FP32 accumulation in tensor memory, and one of
+// the epilogues below.
 //
-// One CTA of 128 threads per 128 x 64 tile of C.  Per round of 64 in K the
-// threads stage the A tile (128 x 64) and the B tile (64 x 64, as N rows of
-// K) in shared memory, K-major in the no-swizzle core-matrix layout (8 rows x
-// 16 bytes per 128-byte core matrix), zero-filled outside the matrices; one
-// thread issues four tcgen05.mma (M 128, N 64, K 16) into the tile's
-// accumulator in tensor memory and commits them to an mbarrier that every
-// thread waits on before the tiles are overwritten.  The epilogue reads the
-// accumulator back with tcgen05.ld, warp w taking rows 32w .. 32w+31 (the
+// One CTA of 128 threads per 128 x 64 tile.  K goes in rounds of 64 through a
+// ring of TC_STAGES shared-memory stages: cp.async copies 16-byte segments of
+// later rounds while the tensor cores work on the current one (the products
+// here are 2 to 64 rounds deep, so a tile's time is the latency of its loads;
+// the ring keeps three rounds in flight).  Stages hold the operands K-major in
+// the no-swizzle core-matrix layout (8 rows x 16 bytes per 128-byte core
+// matrix), zero-filled outside the matrices; a warp's copies cover 8 rows x 4
+// segments, which is 64 contiguous bytes per row in global memory and 512
+// contiguous bytes in shared memory.  One thread issues four tcgen05.mma
+// (M 128, N 64, K 16) per round and commits them to the stage's mbarrier,
+// which every thread waits on before it refills the stage.  The epilogue reads
+// the accumulator back with tcgen05.ld, warp w taking rows 32w .. 32w+31 (the
 // tensor-memory lanes a warp may access).  Waits are bounded (2 s of
-// %globaltimer); a wait that runs out sets *err, the CTA stops issuing,
-// waits (bounded again) for the round in flight and frees its columns.
+// %globaltimer); a wait that runs out sets *err, the CTA stops issuing, waits
+// (bounded again) for what is in flight and frees its columns.
 // ---------------------------------------------------------------------------
-constexpr int TC_M = 128, TC_N = 64, TC_K = 64;
-constexpr int TC_A_BYTES = TC_M * TC_K * 2, TC_B_BYTES = TC_N * TC_K * 2;
-// 24 KB of tiles, requested as 28 KB so that at most 8 CTAs share an SM and
-// their 8 x 64 accumulator columns fit the SM's 512 tensor-memory columns
-constexpr int TC_SMEM = 28 * 1024;
-static_assert(TC_A_BYTES + TC_B_BYTES <= TC_SMEM, "staged tiles exceed the shared-memory request");
+constexpr int TC_M = 128, TC_N = 64, TC_K = 64, TC_STAGES = 4;
+constexpr int TC_A_BYTES = TC_M * TC_K * 2, TC_B_BYTES = TC_N * TC_K * 2, TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
+// 96 KB of stages: two CTAs share an SM, and their 2 x 64 accumulator columns
+// fit its 512 tensor-memory columns
+constexpr int TC_SMEM = TC_STAGES * TC_STAGE_BYTES;
 constexpr uint32_t TC_TMEM_COLS = 64;
 constexpr unsigned long long TC_WAIT_NS = 2000000000ull;
 // instruction descriptor (kind::f16): D F32 (bits 4-5 = 1), A and B BF16
@@ -59,6 +73,7 @@ constexpr unsigned long long TC_WAIT_NS = 2000000000ull;
 // 17-22, M >> 4 at bits 24-28
 constexpr uint32_t TC_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_N >> 3) << 17) |
                               ((uint32_t)(TC_M >> 4) << 24);
+constexpr int kMaxLayers = 8;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -117,47 +132,104 @@ __device__ __forceinline__ float silu_grad(float z)
     return s * (1.0f + z * (1.0f - s));
 }
 
-// Stages rows row0 .. row0 + ROWS - 1 of a K-major operand tile: element
-// (r, k) = get(row0 + r, k0 + k), zero outside rows < nrows and k < K.  T:
-// the source is stored with the row index contiguous (then consecutive
-// threads take consecutive rows, else consecutive K chunks of a row).
-template <int ROWS, bool T>
-__device__ __forceinline__ void tc_stage(uint32_t sbase, const __nv_bfloat16 *__restrict__ src, int ld, int row0,
-                                         int nrows, int k0, int K)
+// Copies a 16-byte segment to shared memory asynchronously; zero fill when !ok.
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool ok)
 {
-    constexpr int CH = TC_K / 8;
-    for (int c = threadIdx.x; c < ROWS * CH; c += 128) {
-        const int r = T ? c % ROWS : c / CH, kc = T ? c / ROWS : c % CH;
-        const int gr = row0 + r;
-        unsigned w[4];
+    const int n = ok ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
+// One round of an operand tile: rows row0 .. row0 + ROWS - 1, K columns
+// k0 .. k0 + TC_K - 1, zero outside row < nrows and k < kend (kend a multiple
+// of 8, or the storage behind it zero up to the next one).
+template <int ROWS>
+__device__ __forceinline__ void tc_load(uint32_t sbase, const __nv_bfloat16 *__restrict__ src, long long ld, int row0,
+                                        int nrows, int k0, int kend)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int ka = k0 + kc * 8 + 2 * e, kb = ka + 1;
-            __nv_bfloat16 lo = __float2bfloat16(0.0f), hi = lo;
-            if (gr < nrows) {
-                if (ka < K) lo = T ? src[(size_t)ka * ld + gr] : src[(size_t)gr * ld + ka];
-                if (kb < K) hi = T ? src[(size_t)kb * ld + gr] : src[(size_t)gr * ld + kb];
-            }
-            w[e] = pack2(lo, hi);
-        }
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sbase + tc_off(r, kc)), "r"(w[0]), "r"(w[1]),
-                     "r"(w[2]), "r"(w[3])
-                     : "memory");
+    for (int i = 0; i < ROWS / 16; ++i) {
+        // unit u: rows 8 (u >> 1) .. + 7, segments 4 (u & 1) .. + 3
+        const int u = i * 4 + warp;
+        const int r = (u >> 1) * 8 + (lane & 7), kc = (u & 1) * 4 + (lane >> 3);
+        const int gr = row0 + r, gk = k0 + kc * 8;
+        const bool ok = gr < nrows && gk < kend;
+        cp16(sbase + tc_off(r, kc), ok ? src + (size_t)gr * ld + gk : src, ok);
     }
 }
 
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(128) gemm_tc_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
-                                                      int lda, const __nv_bfloat16 *__restrict__ B, int ldb,
-                                                      const float *__restrict__ bias, float *C, __nv_bfloat16 *H,
-                                                      int ldc, int *err)
+// Epilogues.  kEpiHidden: x = acc + bias; Z = x and its transposed SiLU when
+// training, H = bf16(SiLU(x)).  kEpiOut: Y = acc + bias.  kEpiLoss: r = acc +
+// bias - T, d = 2 r scale: G, its transpose, column sums of d, sum of r^2
+// scale.  kEpiBack: d = acc SiLU'(Z): G, its transpose, column sums.
+// kEpiPart: the tile itself (a part of the sum over K).
+enum { kEpiHidden, kEpiOut, kEpiLoss, kEpiBack, kEpiPart };
+
+struct EpiArgs {
+    const float *bias;        // per column
+    float *Z;                 // pre-activations (written: hidden, training; read: back), row stride N
+    const float *T;           // targets, row stride N
+    float *Y;                 // output, row stride N
+    __nv_bfloat16 *R, *RT;    // result rows (stride N; null: not wanted) and transposed (row stride ldt; null: not wanted)
+    long long ldt;
+    float *colpart;           // column sums per row tile: [row tile][N]
+    double *losspart;         // per CTA
+    float scale;
+    bool vec;                 // T or Y is 16-byte aligned
+};
+
+// Sum over the warp's 32 lanes of each of v[0..15]: lane 2c and 2c + 1 return
+// column c's (each step keeps half of the columns and adds the partner
+// lane's halves: 16 shuffles instead of 80).
+__device__ __forceinline__ float colsum16(const float (&v)[16], int lane)
+{
+    float a[8], b[4], c[2], d;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const bool up = lane & 16;
+        a[i] = (up ? v[i + 8] : v[i]) + __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + 8], 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const bool up = lane & 8;
+        b[i] = (up ? a[i + 4] : a[i]) + __shfl_xor_sync(0xffffffffu, up ? a[i] : a[i + 4], 8);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const bool up = lane & 4;
+        c[i] = (up ? b[i + 2] : b[i]) + __shfl_xor_sync(0xffffffffu, up ? b[i] : b[i + 2], 4);
+    }
+    {
+        const bool up = lane & 2;
+        d = (up ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, up ? c[0] : c[1], 2);
+    }
+    return d + __shfl_xor_sync(0xffffffffu, d, 1);
+}
+
+// The whole tile: K loop and epilogue.  part: the tile's FP32 destination (kEpiPart).
+template <int EPI>
+__device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, const __nv_bfloat16 *__restrict__ A,
+                                          long long lda, const __nv_bfloat16 *__restrict__ B, long long ldb, int m0,
+                                          int n0, const EpiArgs &e, float *part, int *err)
 {
     extern __shared__ __align__(128) unsigned char tc_tiles[];
-    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ __align__(8) unsigned long long mbar[TC_STAGES];
     __shared__ uint32_t tmem_slot;
+    __shared__ float colw[4][TC_N];
+    __shared__ double lossw[4];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.y * TC_M, n0 = blockIdx.x * TC_N;
-    const uint32_t sA = smem_u32(tc_tiles), sB = sA + TC_A_BYTES, sbar = smem_u32(&mbar);
+    const uint32_t s0 = smem_u32(tc_tiles), sbar = smem_u32(mbar);
+    const int nk = kend > kbeg ? (kend - kbeg + TC_K - 1) / TC_K : 0;
+    auto load = [&](int kt) {
+        if (kt < nk) {
+            const uint32_t st = s0 + (kt % TC_STAGES) * TC_STAGE_BYTES;
+            tc_load<TC_M>(st, A, lda, m0, M, kbeg + kt * TC_K, kend);
+            tc_load<TC_N>(st + TC_A_BYTES, B, ldb, n0, N, kbeg + kt * TC_K, kend);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");   // one group per round, empty past the end
+    };
+#pragma unroll
+    for (int i = 0; i < TC_STAGES - 1; ++i) load(i);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -166,7 +238,8 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(int M, int N, int K, const
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar) : "memory");
+#pragma unroll
+        for (int i = 0; i < TC_STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar + 8 * i) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -174,20 +247,26 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(int M, int N, int K, const
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
 
-    const int nk = (K + TC_K - 1) / TC_K;
-    uint32_t parity = 0;
     bool failed = false;
+    int issued = 0;
     for (int kt = 0; kt < nk; ++kt) {
-        const int k0 = kt * TC_K;
-        tc_stage<TC_M, TA>(sA, A, lda, m0, M, k0, K);
-        tc_stage<TC_N, !TB>(sB, B, ldb, n0, N, k0, K);
+        bool ok = true;
+        // round kt + TC_STAGES - 1 reuses the stage of round kt - 1
+        if (kt > 0 && kt + TC_STAGES - 1 < nk)
+            ok = tc_wait(sbar + 8 * ((kt - 1) % TC_STAGES), ((kt - 1) / TC_STAGES) & 1);
+        if (ok) load(kt + TC_STAGES - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(TC_STAGES - 1) : "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // staged tiles visible to the tensor cores
-        __syncthreads();
+        if (__syncthreads_or(!ok)) {
+            failed = true;
+            break;
+        }
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t st = s0 + (kt % TC_STAGES) * TC_STAGE_BYTES;
 #pragma unroll
             for (int s = 0; s < TC_K / 16; ++s) {
-                const uint64_t da = tc_desc(sA + s * 256), db = tc_desc(sB + s * 256);
+                const uint64_t da = tc_desc(st + s * 256), db = tc_desc(st + TC_A_BYTES + s * 256);
                 const uint32_t accumulate = (kt > 0 || s > 0) ? 1u : 0u;
                 asm volatile("{\n\t.reg .pred p;\n\t"
                              "setp.ne.b32 p, %4, 0;\n\t"
@@ -195,46 +274,136 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(int M, int N, int K, const
                              "l"(da), "l"(db), "r"(TC_IDESC), "r"(accumulate)
                              : "memory");
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sbar)
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             sbar + 8 * (kt % TC_STAGES))
                          : "memory");
         }
-        const bool ok = tc_wait(sbar, parity);
-        parity ^= 1u;
+        ++issued;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    // the last commit tracks every product before it
+    if (issued > 0) {
+        const bool ok = tc_wait(sbar + 8 * ((issued - 1) % TC_STAGES), ((issued - 1) / TC_STAGES) & 1);
         if (__syncthreads_or(!ok)) {
             failed = true;
-            break;
+            // once more (bounded) before the accumulator columns are released below
+            tc_wait(sbar + 8 * ((issued - 1) % TC_STAGES), ((issued - 1) / TC_STAGES) & 1);
         }
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     if (failed) {
-        if (tid == 0) atomicExch(err, 1);
-        // the round whose wait ran out may still complete: wait for it once
-        // more (bounded) before its accumulator columns are released below
-        tc_wait(sbar, parity ^ 1u);
+        if (tid == 0) {
+            *(volatile int *)err = 1;
+            __threadfence_system();
+        }
     } else {
         const int m = m0 + warp * 32 + lane;
+        double loss = 0.0;
 #pragma unroll 1
-        for (int c = 0; c < TC_N; c += 8) {
-            uint32_t v[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        for (int c = 0; c < TC_N; c += 16) {
+            uint32_t v[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = 0u;
             if (nk > 0) {
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+                             "%11, %12, %13, %14, %15}, [%16];"
                              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                               "=r"(v[7])
+                               "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                               "=r"(v[14]), "=r"(v[15])
                              : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             }
-            if (m < M) {
+            if constexpr (EPI == kEpiPart) {
+                float4 *o = reinterpret_cast<float4 *>(part + (size_t)(warp * 32 + lane) * TC_N + c);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const int n = n0 + c + e;
-                    if (n >= N) continue;
-                    float x = __uint_as_float(v[e]);
-                    if (bias) x += bias[n];
-                    if (C) C[(size_t)m * ldc + n] = x;
-                    if (H) H[(size_t)m * ldc + n] = __float2bfloat16(silu(x));
+                for (int i = 0; i < 4; ++i)
+                    o[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                       __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+            } else {
+                // widths are multiples of 8: each half of the 16 columns is inside or outside
+                float x[16];
+                __nv_bfloat16 h[16];
+    #pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int n = n0 + c + 8 * half;
+                    const bool in = m < M && n < N;
+                    const size_t at = (size_t)m * N + n;
+                    float t[8] = {};
+                    if (EPI == kEpiLoss && in) {
+                        if (e.vec) {
+                            *reinterpret_cast<float4 *>(t) = __ldg(reinterpret_cast<const float4 *>(e.T + at));
+                            *reinterpret_cast<float4 *>(t + 4) = __ldg(reinterpret_cast<const float4 *>(e.T + at + 4));
+                        } else {
+    #pragma unroll
+                            for (int i = 0; i < 8; ++i) t[i] = __ldg(e.T + at + i);
+                        }
+                    }
+                    if (EPI == kEpiBack && in) {
+                        *reinterpret_cast<float4 *>(t) = *reinterpret_cast<const float4 *>(e.Z + at);
+                        *reinterpret_cast<float4 *>(t + 4) = *reinterpret_cast<const float4 *>(e.Z + at + 4);
+                    }
+    #pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int k = 8 * half + i;
+                        float a = __uint_as_float(v[k]);
+                        if (EPI != kEpiBack && in) a += __ldg(e.bias + n + i);
+                        if (EPI == kEpiLoss) {
+                            const float r = a - t[i];
+                            if (in) loss += (double)r * r * e.scale;
+                            a = 2.0f * r * e.scale;
+                        }
+                        if (EPI == kEpiBack) a *= silu_grad(t[i]);
+                        x[k] = in ? a : 0.0f;
+                        if (EPI == kEpiHidden) h[k] = in ? __float2bfloat16(silu(a)) : __float2bfloat16(0.0f);
+                        if (EPI == kEpiLoss || EPI == kEpiBack) h[k] = __float2bfloat16(x[k]);
+                    }
+                    if ((EPI == kEpiHidden && e.Z) || EPI == kEpiOut) {
+                        float *o = EPI == kEpiOut ? e.Y : e.Z;
+                        if (in) {
+                            if (EPI == kEpiHidden || e.vec) {
+                                *reinterpret_cast<float4 *>(o + at) = *reinterpret_cast<const float4 *>(x + 8 * half);
+                                *reinterpret_cast<float4 *>(o + at + 4) = *reinterpret_cast<const float4 *>(x + 8 * half + 4);
+                            } else {
+    #pragma unroll
+                                for (int i = 0; i < 8; ++i) o[at + i] = x[8 * half + i];
+                            }
+                        }
+                    }
+                    if (EPI != kEpiOut) {
+                        if (e.R && in) {
+                            uint4 w;
+                            w.x = pack2(h[8 * half], h[8 * half + 1]);
+                            w.y = pack2(h[8 * half + 2], h[8 * half + 3]);
+                            w.z = pack2(h[8 * half + 4], h[8 * half + 5]);
+                            w.w = pack2(h[8 * half + 6], h[8 * half + 7]);
+                            *reinterpret_cast<uint4 *>(e.R + at) = w;
+                        }
+                        // transposed, zero up to the next multiple of 8 rows: the
+                        // weight-gradient products read whole 16-byte segments
+                        if (e.RT && n < N && m < ((M + 7) & ~7)) {
+    #pragma unroll
+                            for (int i = 0; i < 8; ++i) e.RT[(size_t)(n + i) * e.ldt + m] = h[8 * half + i];
+                        }
+                    }
+                }
+                if constexpr (EPI == kEpiLoss || EPI == kEpiBack) {
+                    const float s = colsum16(x, lane);
+                    if (!(lane & 1)) colw[warp][c + (lane >> 1)] = s;
                 }
             }
+        }
+        if constexpr (EPI == kEpiLoss || EPI == kEpiBack) {
+            if (EPI == kEpiLoss) {
+                for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+                if (lane == 0) lossw[warp] = loss;
+            }
+            __syncthreads();
+            if (tid < TC_N && n0 + tid < N)
+                e.colpart[(size_t)(m0 / TC_M) * N + n0 + tid] =
+                    (colw[0][tid] + colw[1][tid]) + (colw[2][tid] + colw[3][tid]);
+            if (EPI == kEpiLoss && tid == 0)
+                e.losspart[blockIdx.y * gridDim.x + blockIdx.x] = (lossw[0] + lossw[1]) + (lossw[2] + lossw[3]);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -243,65 +412,142 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(int M, int N, int K, const
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
 }
 
-__global__ void to_bf16_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ y, long long n)
+template <int EPI>
+__global__ void __launch_bounds__(128) gemm_tc_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
+                                                      const __nv_bfloat16 *__restrict__ B, EpiArgs e, int *err)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        y[i] = __float2bfloat16(x[i]);
+    gemm_tile<EPI>(M, N, 0, K, A, K, B, K, blockIdx.y * TC_M, blockIdx.x * TC_N, e, nullptr, err);
 }
 
-// dZ = 2 (Y - T) / (n d) (FP32 and BF16), loss += sum (Y - T)^2 / (n d)
-__global__ void mse_grad_kernel(const float *__restrict__ Y, const float *__restrict__ T, long long n, float scale,
-                                float *__restrict__ dZ, __nv_bfloat16 *__restrict__ G, double *loss)
+// The layers as the gradient kernels see them.
+struct Layers {
+    int nl, splits, tiles;                 // tiles: 128 x 64 tiles of all weight matrices
+    int ksplit;                            // batch rows per split (a multiple of TC_K)
+    int din[kMaxLayers], dout[kMaxLayers], tile0[kMaxLayers];
+    long long w_off[kMaxLayers], b_off[kMaxLayers], col_off[kMaxLayers];
+    const __nv_bfloat16 *HT[kMaxLayers], *GT[kMaxLayers];
+};
+
+// Weight gradients of every layer in one launch: CTA (tile, split) sums its
+// 128 x 64 tile of dW_l = H^T G over its share of the batch.  A layer alone is
+// 4 to 8 tiles of 2048 rows on a 148-SM chip; all layers' tiles times the
+// splits fill it, and the update adds the parts in a fixed order.
+__global__ void __launch_bounds__(128) gemm_dw_kernel(Layers L, int n, long long ldt, float *part, int *err)
 {
-    double part = 0.0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float r = Y[i] - T[i];
-        const float d = 2.0f * r * scale;
-        dZ[i] = d;
-        G[i] = __float2bfloat16(d);
-        part += (double)r * r * scale;
+    int l = 0;
+    while (l + 1 < L.nl && (int)blockIdx.x >= L.tile0[l + 1]) ++l;
+    const int tile = blockIdx.x - L.tile0[l], tn = (L.dout[l] + TC_N - 1) / TC_N;
+    const int k0 = blockIdx.y * L.ksplit, k1 = min(n, k0 + L.ksplit);
+    EpiArgs e{};
+    gemm_tile<kEpiPart>(L.din[l], L.dout[l], k0, k1, L.HT[l], ldt, L.GT[l], ldt, tile / tn * TC_M, tile % tn * TC_N, e,
+                        part + ((size_t)blockIdx.y * L.tiles + blockIdx.x) * (TC_M * TC_N), err);
+}
+
+// H = bf16(X) and, with HT, its transpose (zero up to the next multiple of 8
+// rows); 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256) input_kernel(const float *__restrict__ X, int n, int d, __nv_bfloat16 *H,
+                                                    __nv_bfloat16 *HT, long long ldt)
+{
+    __shared__ __nv_bfloat16 tile[32][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5, c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+#pragma unroll
+    for (int i = y; i < 32; i += 8) {
+        const int r = r0 + i, c = c0 + x;
+        const bool in = r < n && c < d;
+        const __nv_bfloat16 v = __float2bfloat16(in ? X[(size_t)r * d + c] : 0.0f);
+        if (in) H[(size_t)r * d + c] = v;
+        tile[i][x] = v;
     }
-    for (int o = 16; o; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, part);
-}
-
-// dZ = dH * SiLU'(Z) (FP32 and BF16)
-__global__ void silu_back_kernel(const float *__restrict__ dH, const float *__restrict__ Z, long long n,
-                                 float *__restrict__ dZ, __nv_bfloat16 *__restrict__ G)
-{
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float d = dH[i] * silu_grad(Z[i]);
-        dZ[i] = d;
-        G[i] = __float2bfloat16(d);
+    if (!HT) return;
+    __syncthreads();
+#pragma unroll
+    for (int i = y; i < 32; i += 8) {
+        const int r = r0 + x, c = c0 + i;
+        if (c < d && r < ((n + 7) & ~7)) HT[(size_t)c * ldt + r] = tile[x][i];
     }
 }
 
-// db[c] = sum_r dZ[r][c]
-__global__ void colsum_kernel(const float *__restrict__ dZ, int rows, int cols, float *__restrict__ db)
+// BF16 weights in both orders (rows of din, rows of dout) from the FP32 ones.
+__global__ void weights_kernel(const float *__restrict__ p, Layers L, __nv_bfloat16 *wb, __nv_bfloat16 *wt)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.0f;
-    for (int r = 0; r < rows; ++r) s += dZ[(size_t)r * cols + c];
-    db[c] = s;
+    const int l = blockIdx.y, din = L.din[l], dout = L.dout[l];
+    const long long nw = (long long)din * dout;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nw; i += (long long)gridDim.x * blockDim.x) {
+        const __nv_bfloat16 w = __float2bfloat16(p[L.w_off[l] + i]);
+        wb[L.w_off[l] + i] = w;
+        wt[L.w_off[l] + (i % dout) * din + i / dout] = w;
+    }
 }
 
-// Adam (bias-corrected) on the FP32 master parameters (the next forward pass
-// rounds the weights to BF16 again).
-__global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ grad, float *__restrict__ m,
-                            float *__restrict__ v, long long n, float lr, float b1, float b2, float eps, float c1,
-                            float c2)
+struct AdamArgs {
+    float lr, b1, b2, eps, c1, c2;
+};
+
+// Gradient of every parameter (the parts of dW, the row tiles' column sums of
+// dZ for the biases, each added in order), then Adam (bias-corrected) on the
+// FP32 parameters and the BF16 weights of the next forward pass; with UPDATE
+// false the gradient vector instead.  Block (0, 0) adds up the loss and
+// leaves it where the host reads it.
+template <bool UPDATE>
+__global__ void __launch_bounds__(256) update_kernel(Layers L, const float *__restrict__ part,
+                                                     const float *__restrict__ colpart, int row_tiles,
+                                                     const double *__restrict__ losspart, int nloss, double *loss_out,
+                                                     float *__restrict__ grad, float *__restrict__ p,
+                                                     float *__restrict__ m, float *__restrict__ v, __nv_bfloat16 *wb,
+                                                     __nv_bfloat16 *wt, AdamArgs a)
 {
+    const int l = blockIdx.y, din = L.din[l], dout = L.dout[l];
+    const int tn = (dout + TC_N - 1) / TC_N;
+    const long long nw = (long long)din * dout, n = nw + dout;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float g = grad[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * g, vi = b2 * v[i] + (1.0f - b2) * g * g;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+        float g = 0.0f;
+        int r = 0, c = 0;
+        if (i < nw) {
+            r = (int)(i / dout);
+            c = (int)(i % dout);
+            const float *q = part + (size_t)(L.tile0[l] + (r / TC_M) * tn + c / TC_N) * (TC_M * TC_N) +
+                             (r % TC_M) * TC_N + c % TC_N;
+            for (int s = 0; s < L.splits; ++s) g += q[(size_t)s * L.tiles * (TC_M * TC_N)];
+        } else {
+            for (int t = 0; t < row_tiles; ++t) g += colpart[L.col_off[l] + (size_t)t * dout + (i - nw)];
+        }
+        const long long at = i < nw ? L.w_off[l] + i : L.b_off[l] + (i - nw);
+        if constexpr (UPDATE) {
+            const float mi = a.b1 * m[at] + (1.0f - a.b1) * g, vi = a.b2 * v[at] + (1.0f - a.b2) * g * g;
+            m[at] = mi;
+            v[at] = vi;
+            const float w = p[at] - a.lr * (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);
+            p[at] = w;
+            if (i < nw) {
+                wb[at] = __float2bfloat16(w);
+                wt[L.w_off[l] + (long long)c * din + r] = __float2bfloat16(w);
+            }
+        } else {
+            grad[at] = g;
+        }
+    }
+    if (blockIdx.x == 0 && blockIdx.y == 0) {
+        __shared__ double part_sum[256];
+        double s = 0.0;
+        for (int i = threadIdx.x; i < nloss; i += 256) s += losspart[i];
+        part_sum[threadIdx.x] = s;
+        __syncthreads();
+        for (int o = 128; o; o >>= 1) {
+            if (threadIdx.x < (unsigned)o) part_sum[threadIdx.x] += part_sum[threadIdx.x + o];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) *loss_out = part_sum[0];
     }
 }
 
 unsigned blocks_for(long long n) { return (unsigned)std::min<long long>((n + 255) / 256, 148 * 16); }
+
+// What the kernels leave for the host, in page-locked memory mapped into the
+// device's address space: read after the stream is synchronised, no copy.
+struct HostSlot {
+    double loss;
+    int tc_err;   // set by a tensor-core wait that ran out
+};
 
 }  // namespace
 
@@ -311,13 +557,17 @@ struct pfk_mlp {
     std::vector<long long> w_off, b_off;      // offsets in the parameter vector
     long long nparam = 0;
     float *p = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;   // FP32 params, grads, Adam moments
-    __nv_bfloat16 *wb = nullptr;              // BF16 copy of the parameter vector (weights used)
-    std::vector<float *> Z;                   // pre-activations per layer [max_batch x d_l]
-    std::vector<__nv_bfloat16 *> Hb;          // BF16 activations per layer (H_0 = input)
-    float *dA = nullptr, *dB = nullptr;       // FP32 scratch for dZ / dH
-    __nv_bfloat16 *G = nullptr;               // BF16 dZ
-    double *loss = nullptr;
-    int *tc_err = nullptr;                    // set by a tensor-core wait that ran out
+    // BF16 weights as rows of din (p's order) and as rows of dout; they change
+    // only together with p (set_params, train_step)
+    __nv_bfloat16 *wb = nullptr, *wt = nullptr;
+    std::vector<float *> Z;                   // pre-activations of the hidden layers [max_batch x d_l]
+    std::vector<__nv_bfloat16 *> H, HT;       // layer inputs (H[0] = network input), rows and transposed
+    std::vector<__nv_bfloat16 *> G, GT;       // BF16 dZ per layer, rows and transposed
+    float *part = nullptr;                    // parts of the weight gradients
+    float *colpart = nullptr;                 // column sums of dZ per row tile, all layers
+    double *losspart = nullptr;
+    HostSlot *slot = nullptr, *d_slot = nullptr;
+    long long ldt = 0;                        // row stride of the transposed buffers (max_batch, rounded up to 8)
     long long step = 0;
     std::string err;
 };
@@ -337,52 +587,129 @@ pfk_status mlp_fail(pfk_mlp *m, const std::string &msg, pfk_status s)
         if (e_ != cudaSuccess) return mlp_fail(m, std::string(#call) + ": " + cudaGetErrorString(e_), PFK_ERR_CUDA); \
     } while (0)
 
-template <bool TA, bool TB>
-void gemm(pfk_mlp *m, int M, int N, int K, const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ldb,
-          const float *bias, float *C, __nv_bfloat16 *H, int ldc, cudaStream_t st)
+int row_tiles(int n) { return (n + TC_M - 1) / TC_M; }
+
+// Weight-gradient tiles of the network, and the splits of the batch for n
+// rows: enough that tiles x splits give every SM a CTA, at least 4 rounds of
+// K each, at most kMaxSplits parts.  Measured on 112-256-256-232 at 2048 rows
+// (20 tiles): 8 splits.
+constexpr int kMaxSplits = 16;
+
+int weight_tiles(const std::vector<int> &d)
 {
-    dim3 grid((N + TC_N - 1) / TC_N, (M + TC_M - 1) / TC_M);
-    gemm_tc_kernel<TA, TB><<<grid, 128, TC_SMEM, st>>>(M, N, K, A, lda, B, ldb, bias, C, H, ldc, m->tc_err);
+    int t = 0;
+    for (size_t l = 0; l + 1 < d.size(); ++l) t += row_tiles(d[l]) * ((d[l + 1] + TC_N - 1) / TC_N);
+    return t;
 }
 
-// Forward pass of n rows already in m->Hb[0]; leaves Y in m->Z[nl-1].
-void forward(pfk_mlp *m, int n, cudaStream_t st)
+int split_cap(int tiles) { return std::max(1, std::min(kMaxSplits, 2 * 148 / tiles)); }
+
+Layers layers_for(const pfk_mlp *m, int n)
 {
-    to_bf16_kernel<<<blocks_for(m->nparam), 256, 0, st>>>(m->p, m->wb, m->nparam);
+    Layers L{};
+    L.nl = m->nl;
+    long long col = 0;
+    int t = 0;
+    for (int l = 0; l < m->nl; ++l) {
+        L.din[l] = m->dims[l];
+        L.dout[l] = m->dims[l + 1];
+        L.tile0[l] = t;
+        t += row_tiles(L.din[l]) * ((L.dout[l] + TC_N - 1) / TC_N);
+        L.w_off[l] = m->w_off[l];
+        L.b_off[l] = m->b_off[l];
+        L.col_off[l] = col;
+        col += (long long)row_tiles(m->max_batch) * L.dout[l];
+        L.HT[l] = m->HT[l];
+        L.GT[l] = m->GT[l];
+    }
+    L.tiles = t;
+    const int rounds = (n + TC_K - 1) / TC_K;
+    const int want = std::max(1, std::min(split_cap(t), rounds / 4));
+    const int per = (rounds + want - 1) / want;
+    L.ksplit = per * TC_K;
+    L.splits = (rounds + per - 1) / per;
+    return L;
+}
+
+bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+template <int EPI>
+void gemm(pfk_mlp *m, int M, int N, int K, const __nv_bfloat16 *A, const __nv_bfloat16 *B, const EpiArgs &e,
+          cudaStream_t st)
+{
+    dim3 grid((N + TC_N - 1) / TC_N, row_tiles(M));
+    gemm_tc_kernel<EPI><<<grid, 128, TC_SMEM, st>>>(M, N, K, A, B, e, &m->d_slot->tc_err);
+}
+
+// Forward pass of n rows of X: to Y, or, with T, to dZ of the last layer and the loss.
+void forward(pfk_mlp *m, int n, const float *X, float *Y, const float *T, cudaStream_t st)
+{
+    const bool train = T != nullptr;
+    const int d0 = m->dims[0];
+    dim3 gi((d0 + 31) / 32, (n + 31) / 32);
+    input_kernel<<<gi, 256, 0, st>>>(X, n, d0, m->H[0], train ? m->HT[0] : nullptr, m->ldt);
+    long long col = 0;
     for (int l = 0; l < m->nl; ++l) {
         const int din = m->dims[l], dout = m->dims[l + 1];
-        const bool last = l == m->nl - 1;
-        gemm<false, false>(m, n, dout, din, m->Hb[l], din, m->wb + m->w_off[l], dout, m->p + m->b_off[l], m->Z[l],
-                           last ? nullptr : m->Hb[l + 1], dout, st);
+        EpiArgs e{};
+        e.bias = m->p + m->b_off[l];
+        e.ldt = m->ldt;
+        const __nv_bfloat16 *w = m->wt + m->w_off[l];
+        if (l + 1 < m->nl) {
+            e.Z = train ? m->Z[l] : nullptr;
+            e.R = m->H[l + 1];
+            e.RT = train ? m->HT[l + 1] : nullptr;
+            gemm<kEpiHidden>(m, n, dout, din, m->H[l], w, e, st);
+        } else if (train) {
+            e.T = T;
+            e.vec = aligned16(T);
+            e.R = m->nl > 1 ? m->G[l] : nullptr;
+            e.RT = m->GT[l];
+            e.colpart = m->colpart + col;
+            e.losspart = m->losspart;
+            e.scale = 1.0f / (float)((long long)n * dout);
+            gemm<kEpiLoss>(m, n, dout, din, m->H[l], w, e, st);
+        } else {
+            e.Y = Y;
+            e.vec = aligned16(Y);
+            gemm<kEpiOut>(m, n, dout, din, m->H[l], w, e, st);
+        }
+        col += (long long)row_tiles(m->max_batch) * dout;
     }
 }
 
-// Gradients of the mean squared error for n rows (inputs in Hb[0], targets T).
-void backward(pfk_mlp *m, int n, const float *T, cudaStream_t st)
+// Gradient parts of the mean squared error after forward(..., T).
+void backward(pfk_mlp *m, int n, const Layers &L, cudaStream_t st)
 {
-    const int L = m->nl;
-    const long long ny = (long long)n * m->dims[L];
-    cudaMemsetAsync(m->loss, 0, sizeof(double), st);
-    mse_grad_kernel<<<blocks_for(ny), 256, 0, st>>>(m->Z[L - 1], T, ny, 1.0f / (float)ny, m->dA, m->G, m->loss);
-    for (int l = L - 1; l >= 0; --l) {
-        const int din = m->dims[l], dout = m->dims[l + 1];
-        // dW_l = H_{l-1}^T G  (din x dout), db_l = colsum(dZ)
-        gemm<true, false>(m, din, dout, n, m->Hb[l], din, m->G, dout, nullptr, m->grad + m->w_off[l], nullptr, dout, st);
-        colsum_kernel<<<(dout + 127) / 128, 128, 0, st>>>(m->dA, n, dout, m->grad + m->b_off[l]);
-        if (l == 0) break;
-        // dH_{l-1} = G W_l^T (n x din), then dZ_{l-1} = dH * SiLU'(Z_{l-1})
-        gemm<false, true>(m, n, din, dout, m->G, dout, m->wb + m->w_off[l], dout, nullptr, m->dB, nullptr, din, st);
-        const long long nh = (long long)n * din;
-        silu_back_kernel<<<blocks_for(nh), 256, 0, st>>>(m->dB, m->Z[l - 1], nh, m->dA, m->G);
+    for (int l = m->nl - 1; l > 0; --l) {
+        // dH_{l-1} = G W_l^T (n x din); dZ_{l-1} = dH * SiLU'(Z_{l-1})
+        EpiArgs e{};
+        e.ldt = m->ldt;
+        e.Z = m->Z[l - 1];
+        e.R = l > 1 ? m->G[l - 1] : nullptr;
+        e.RT = m->GT[l - 1];
+        e.colpart = m->colpart + L.col_off[l - 1];
+        gemm<kEpiBack>(m, n, m->dims[l], m->dims[l + 1], m->G[l], m->wb + m->w_off[l], e, st);
     }
+    gemm_dw_kernel<<<dim3(L.tiles, L.splits), 128, TC_SMEM, st>>>(L, n, m->ldt, m->part, &m->d_slot->tc_err);
+}
+
+template <bool UPDATE>
+void finish(pfk_mlp *m, int n, const Layers &L, const AdamArgs &a, cudaStream_t st)
+{
+    long long most = 0;
+    for (int l = 0; l < m->nl; ++l) most = std::max(most, (long long)L.din[l] * L.dout[l] + L.dout[l]);
+    const int nloss = row_tiles(n) * ((m->dims[m->nl] + TC_N - 1) / TC_N);
+    update_kernel<UPDATE><<<dim3(blocks_for(most), m->nl), 256, 0, st>>>(
+        L, m->part, m->colpart, row_tiles(n), m->losspart, nloss, &m->d_slot->loss, m->grad, m->p, m->m, m->v, m->wb,
+        m->wt, a);
 }
 
 // After a synchronised call: PFK_ERR_CUDA if a GEMM's tensor-core wait ran out.
 pfk_status check_tc(pfk_mlp *m)
 {
-    int e = 0;
-    MLP_CK(cudaMemcpy(&e, m->tc_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) return mlp_fail(m, "tensor-core GEMM: an mbarrier wait ran out (2 s)", PFK_ERR_CUDA);
+    if (*(volatile int *)&m->slot->tc_err)
+        return mlp_fail(m, "tensor-core GEMM: an mbarrier wait ran out (2 s)", PFK_ERR_CUDA);
     return PFK_OK;
 }
 
@@ -426,28 +753,41 @@ pfk_status pfk_mlp_create(int nlayers, const int *dims, int max_batch, int devic
         return s;
     };
     if (cudaSetDevice(device) != cudaSuccess) return bail(mlp_fail(m, "cudaSetDevice failed", PFK_ERR_CUDA));
-    int widest = 0;
-    for (int d : m->dims) widest = std::max(widest, d);
-    bool ok = cudaMalloc(&m->p, sizeof(float) * m->nparam) == cudaSuccess &&
-              cudaMalloc(&m->grad, sizeof(float) * m->nparam) == cudaSuccess &&
-              cudaMalloc(&m->m, sizeof(float) * m->nparam) == cudaSuccess &&
-              cudaMalloc(&m->v, sizeof(float) * m->nparam) == cudaSuccess &&
-              cudaMalloc(&m->wb, sizeof(__nv_bfloat16) * m->nparam) == cudaSuccess &&
-              cudaMalloc(&m->dA, sizeof(float) * (size_t)max_batch * widest) == cudaSuccess &&
-              cudaMalloc(&m->dB, sizeof(float) * (size_t)max_batch * widest) == cudaSuccess &&
-              cudaMalloc(&m->G, sizeof(__nv_bfloat16) * (size_t)max_batch * widest) == cudaSuccess &&
-              cudaMalloc(&m->loss, sizeof(double)) == cudaSuccess &&
-              cudaMalloc(&m->tc_err, sizeof(int)) == cudaSuccess;
+    // transposed buffers: rows of the batch rounded up to whole 16-byte segments
+    m->ldt = ((long long)max_batch + 7) & ~7LL;
+    const size_t rows = max_batch;
+    const int tiles = weight_tiles(m->dims);
+    long long cols = 0;
+    for (int l = 0; l < nlayers; ++l) cols += (long long)row_tiles(max_batch) * dims[l + 1];
+    const size_t nloss = (size_t)row_tiles(max_batch) * ((dims[nlayers] + TC_N - 1) / TC_N);
+    auto get = [](auto **q, size_t count) { return cudaMalloc(reinterpret_cast<void **>(q), sizeof(**q) * count) == cudaSuccess; };
+    bool ok = get(&m->p, m->nparam) && get(&m->grad, m->nparam) && get(&m->m, m->nparam) && get(&m->v, m->nparam) &&
+              get(&m->wb, m->nparam) && get(&m->wt, m->nparam) &&
+              get(&m->part, (size_t)tiles * split_cap(tiles) * TC_M * TC_N) && get(&m->colpart, cols) &&
+              get(&m->losspart, nloss) &&
+              cudaHostAlloc(reinterpret_cast<void **>(&m->slot), sizeof(HostSlot), cudaHostAllocMapped) == cudaSuccess &&
+              cudaHostGetDevicePointer(reinterpret_cast<void **>(&m->d_slot), m->slot, 0) == cudaSuccess;
+    for (auto *b : {&m->H, &m->HT, &m->G, &m->GT}) b->assign(nlayers, nullptr);
     m->Z.assign(nlayers, nullptr);
-    m->Hb.assign(nlayers, nullptr);
     for (int l = 0; ok && l < nlayers; ++l)
-        ok = cudaMalloc(&m->Z[l], sizeof(float) * (size_t)max_batch * dims[l + 1]) == cudaSuccess &&
-             cudaMalloc(&m->Hb[l], sizeof(__nv_bfloat16) * (size_t)max_batch * dims[l]) == cudaSuccess;
+        ok = get(&m->H[l], rows * dims[l]) && get(&m->HT[l], (size_t)m->ldt * dims[l]) &&
+             get(&m->G[l], rows * dims[l + 1]) && get(&m->GT[l], (size_t)m->ldt * dims[l + 1]) &&
+             (l + 1 == nlayers || get(&m->Z[l], rows * dims[l + 1]));
     if (!ok) return bail(mlp_fail(m, "pfk_mlp_create: device allocation failed", PFK_ERR_NOMEM));
-    cudaMemset(m->tc_err, 0, sizeof(int));
+    // the product kernels' shared-memory limits on this device
+    for (const void *k : {(const void *)gemm_tc_kernel<kEpiHidden>, (const void *)gemm_tc_kernel<kEpiOut>,
+                          (const void *)gemm_tc_kernel<kEpiLoss>, (const void *)gemm_tc_kernel<kEpiBack>,
+                          (const void *)gemm_dw_kernel})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess)
+            return bail(mlp_fail(m, "pfk_mlp_create: kernel configuration failed", PFK_ERR_CUDA));
+    m->slot->loss = 0.0;
+    m->slot->tc_err = 0;
     cudaMemset(m->p, 0, sizeof(float) * m->nparam);
     cudaMemset(m->m, 0, sizeof(float) * m->nparam);
     cudaMemset(m->v, 0, sizeof(float) * m->nparam);
+    cudaMemset(m->wb, 0, sizeof(__nv_bfloat16) * m->nparam);
+    cudaMemset(m->wt, 0, sizeof(__nv_bfloat16) * m->nparam);
+    cudaStreamSynchronize(nullptr);
     *out = m;
     return PFK_OK;
 }
@@ -457,13 +797,15 @@ pfk_status pfk_mlp_destroy(pfk_mlp *m)
     if (!m) return PFK_OK;
     cudaSetDevice(m->device);
     cudaDeviceSynchronize();
-    for (void *x : {(void *)m->p, (void *)m->grad, (void *)m->m, (void *)m->v, (void *)m->wb, (void *)m->dA,
-                    (void *)m->dB, (void *)m->G, (void *)m->loss, (void *)m->tc_err})
+    for (void *x : {(void *)m->p, (void *)m->grad, (void *)m->m, (void *)m->v, (void *)m->wb, (void *)m->wt,
+                    (void *)m->part, (void *)m->colpart, (void *)m->losspart})
         if (x) cudaFree(x);
     for (float *z : m->Z)
         if (z) cudaFree(z);
-    for (__nv_bfloat16 *h : m->Hb)
-        if (h) cudaFree(h);
+    for (auto *b : {&m->H, &m->HT, &m->G, &m->GT})
+        for (__nv_bfloat16 *h : *b)
+            if (h) cudaFree(h);
+    if (m->slot) cudaFreeHost(m->slot);
     delete m;
     return PFK_OK;
 }
@@ -479,6 +821,11 @@ pfk_status pfk_mlp_set_params(pfk_mlp *m, const float *params)
     MLP_CK(cudaMemcpy(m->p, params, sizeof(float) * m->nparam, cudaMemcpyHostToDevice));
     MLP_CK(cudaMemset(m->m, 0, sizeof(float) * m->nparam));
     MLP_CK(cudaMemset(m->v, 0, sizeof(float) * m->nparam));
+    long long most = 0;
+    for (int l = 0; l < m->nl; ++l) most = std::max(most, (long long)m->dims[l] * m->dims[l + 1]);
+    weights_kernel<<<dim3(blocks_for(most), m->nl), 256>>>(m->p, layers_for(m, 1), m->wb, m->wt);
+    MLP_CK(cudaGetLastError());
+    MLP_CK(cudaStreamSynchronize(nullptr));   // the calls that use them may run on any stream
     m->step = 0;
     return PFK_OK;
 }
@@ -497,13 +844,9 @@ pfk_status pfk_mlp_forward(pfk_mlp *m, const float *dX, int n, float *dY, void *
     if (s != PFK_OK) return s;
     if (!dY) return mlp_fail(m, "null output", PFK_ERR_INVALID);
     cudaStream_t st = (cudaStream_t)stream;
-    const long long nx = (long long)n * m->dims[0];
-    to_bf16_kernel<<<blocks_for(nx), 256, 0, st>>>(dX, m->Hb[0], nx);
-    forward(m, n, st);
-    MLP_CK(cudaMemcpyAsync(dY, m->Z[m->nl - 1], sizeof(float) * (size_t)n * m->dims[m->nl], cudaMemcpyDeviceToDevice,
-                           st));
-    MLP_CK(cudaStreamSynchronize(st));
+    forward(m, n, dX, dY, nullptr, st);
     MLP_CK(cudaGetLastError());
+    MLP_CK(cudaStreamSynchronize(st));
     return check_tc(m);
 }
 
@@ -514,14 +857,14 @@ pfk_status pfk_mlp_gradients(pfk_mlp *m, const float *dX, const float *dT, int n
     if (s != PFK_OK) return s;
     if (!dT) return mlp_fail(m, "null targets", PFK_ERR_INVALID);
     cudaStream_t st = (cudaStream_t)stream;
-    const long long nx = (long long)n * m->dims[0];
-    to_bf16_kernel<<<blocks_for(nx), 256, 0, st>>>(dX, m->Hb[0], nx);
-    forward(m, n, st);
-    backward(m, n, dT, st);
-    if (grads) MLP_CK(cudaMemcpyAsync(grads, m->grad, sizeof(float) * m->nparam, cudaMemcpyDeviceToHost, st));
-    if (loss) MLP_CK(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
-    MLP_CK(cudaStreamSynchronize(st));
+    const Layers L = layers_for(m, n);
+    forward(m, n, dX, nullptr, dT, st);
+    backward(m, n, L, st);
+    finish<false>(m, n, L, AdamArgs{}, st);
     MLP_CK(cudaGetLastError());
+    if (grads) MLP_CK(cudaMemcpyAsync(grads, m->grad, sizeof(float) * m->nparam, cudaMemcpyDeviceToHost, st));
+    MLP_CK(cudaStreamSynchronize(st));
+    if (loss) *loss = *(volatile double *)&m->slot->loss;
     return check_tc(m);
 }
 
@@ -532,18 +875,16 @@ pfk_status pfk_mlp_train_step(pfk_mlp *m, const float *dX, const float *dT, int 
     if (s != PFK_OK) return s;
     if (!dT || !(lr > 0.0f)) return mlp_fail(m, "null targets or non-positive learning rate", PFK_ERR_INVALID);
     cudaStream_t st = (cudaStream_t)stream;
-    const long long nx = (long long)n * m->dims[0];
-    to_bf16_kernel<<<blocks_for(nx), 256, 0, st>>>(dX, m->Hb[0], nx);
-    forward(m, n, st);
-    backward(m, n, dT, st);
+    const Layers L = layers_for(m, n);
+    forward(m, n, dX, nullptr, dT, st);
+    backward(m, n, L, st);
     m->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f / (1.0f - powf(b1, (float)m->step)), c2 = 1.0f / (1.0f - powf(b2, (float)m->step));
-    adam_kernel<<<blocks_for(m->nparam), 256, 0, st>>>(m->p, m->grad, m->m, m->v, m->nparam, lr, b1, b2, 1e-8f, c1,
-                                                       c2);
-    if (loss) MLP_CK(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
-    MLP_CK(cudaStreamSynchronize(st));
+    finish<true>(m, n, L, AdamArgs{lr, b1, b2, 1e-8f, c1, c2}, st);
     MLP_CK(cudaGetLastError());
+    MLP_CK(cudaStreamSynchronize(st));
+    if (loss) *loss = *(volatile double *)&m->slot->loss;
     return check_tc(m);
 }
 

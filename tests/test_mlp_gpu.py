@@ -83,3 +83,49 @@ def test_training_lowers_the_loss():
     last = net.gradients(Xd, Td)[1]
     assert last < 0.1 * first
     net.close()
+
+
+@pytest.mark.parametrize("dims,n", [([8, 8], 1), ([24, 8], 129), ([64, 64, 64], 8), ([72, 136, 8], 127),
+                                    ([520, 264, 64], 128), ([16, 8, 8, 8, 8, 8, 8, 8, 8], 65), ([128, 192, 200], 1031)])
+def test_tile_edges(dims, n):
+    """Widths and batch sizes around the 128 x 64 tile, the 64-deep round and
+    the four-stage ring (520 is nine rounds; 1031 rows are 17 rounds of the
+    weight gradients in four splits, the last of them short), one to eight
+    layers; targets and outputs that are not 16-byte aligned give the same
+    bits as aligned ones.  Bounds as above: the roundings of Z, H and dZ are
+    the oracle's, the sums differ in order."""
+    torch = pytest.importorskip("torch")
+    net = _net(dims, seed=9, max_batch=n + 3)
+    X, T = _data(dims, n, 10)
+    Xd = torch.from_numpy(X).cuda()
+    flat = torch.zeros(n * dims[-1] + 1, device="cuda")
+    flat[1:] = torch.from_numpy(T).cuda().reshape(-1)
+    Tu = flat[1:].view(n, dims[-1])                 # 4 bytes past a 16-byte boundary
+    Td = Tu.clone()
+    p = net.params()
+    Y = net.forward(Xd).cpu().numpy()
+    Yo = mlp_ref.forward(dims, p, X)[0]
+    assert np.linalg.norm(Y - Yo) < 1e-4 * np.linalg.norm(Yo)
+    Yu = torch.zeros(n * dims[-1] + 1, device="cuda")
+    net._check(net.L.pfk_mlp_forward(net.h, net._ptr(Xd), n, Yu.data_ptr() + 4, None))
+    assert np.array_equal(Yu[1:].view(n, dims[-1]).cpu().numpy(), Y) and float(Yu[0]) == 0.0
+    g, loss = net.gradients(Xd, Td)
+    gu, lossu = net.gradients(Xd, Tu)
+    assert np.array_equal(g, gu) and loss == lossu
+    go, losso = mlp_ref.gradients(dims, p, X, T)
+    assert abs(loss - losso) < 1e-4 * losso
+    o = 0
+    for din, dout in zip(dims[:-1], dims[1:]):
+        for size in (din * dout, dout):
+            a, b = g[o:o + size], go[o:o + size]
+            assert np.linalg.norm(a - b) <= 2e-3 * np.linalg.norm(b) + 1e-12
+            o += size
+    # the update uses these gradients, and the next forward pass its weights
+    net.train_step(Xd, Td, 1e-2)
+    z = np.zeros_like(p, dtype=np.float64)
+    po = mlp_ref.adam(p.astype(np.float64), g.astype(np.float64), z, z, 1, 1e-2)[0]
+    p1 = net.params()
+    assert np.abs(p1 - po).max() < 1e-5
+    Y1o = mlp_ref.forward(dims, p1, X)[0]
+    assert np.linalg.norm(net.forward(Xd).cpu().numpy() - Y1o) < 1e-4 * np.linalg.norm(Y1o)
+    net.close()
