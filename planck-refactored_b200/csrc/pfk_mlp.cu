@@ -19,10 +19,10 @@
 // for the weight gradients of every layer, and the update.  Each product
 // leaves its result in both orders (rows of the batch, and transposed), so
 // every product reads both operands as rows of K by 16-byte copies.  On the
-// 112-256-256-232 network (one B200): 2048 rows, a step 135 us against 1675 us
+// 112-256-256-232 network (one B200): 2048 rows, a step 98 us against 1675 us
 // before (products staged by 2-byte gathers, bias sums by one thread per
 // column, weight gradients on 8 CTAs, two host synchronisations); forward of
-// 8192 rows 73 us against 250 us (both with the host call).
+// 8192 rows 54 us against 250 us (both with the host call).
 // The reference has no counterpart: it is the learned part of the guess
 // hook (scf.cpp:206-240 selects the guess; a learned density enters the SCF
 // as a ReadDensity guess does, scf.cpp:213-216).
@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "planck_fock.h"
@@ -45,7 +46,7 @@ thread_local std::string g_mlp_error;
 // row start 16-byte aligned), FP32 accumulation in tensor memory, and one of
 // the epilogues below.
 //
-// One CTA of 128 threads per 128 x 64 tile.  K goes in rounds of 64 through a
+// One CTA of 256 threads per 128 x 64 tile.  K goes in rounds of 64 through a
 // ring of TC_STAGES shared-memory stages: cp.async copies 16-byte segments of
 // later rounds while the tensor cores work on the current one (the products
 // here are 2 to 64 rounds deep, so a tile's time is the latency of its loads;
@@ -56,12 +57,16 @@ thread_local std::string g_mlp_error;
 // contiguous bytes in shared memory.  One thread issues four tcgen05.mma
 // (M 128, N 64, K 16) per round and commits them to the stage's mbarrier,
 // which every thread waits on before it refills the stage.  The epilogue reads
-// the accumulator back with tcgen05.ld, warp w taking rows 32w .. 32w+31 (the
-// tensor-memory lanes a warp may access).  Waits are bounded (2 s of
+// the accumulator back with tcgen05.ld, warps w and w + 4 taking rows 32w ..
+// 32w+31 (the tensor-memory lanes a warp may access) and 32 columns each: a
+// tile's time is mostly this epilogue (64 values a thread on four warps took
+// 17 us of kernel time for 8192 x 256; with eight warps and overlapped
+// launches the three layers' forward pass went from 73 to 54 us, a training
+// step of 2048 rows from 135 to 98 us).  Waits are bounded (2 s of
 // %globaltimer); a wait that runs out sets *err, the CTA stops issuing, waits
 // (bounded again) for what is in flight and frees its columns.
 // ---------------------------------------------------------------------------
-constexpr int TC_M = 128, TC_N = 64, TC_K = 64, TC_STAGES = 4;
+constexpr int TC_M = 128, TC_N = 64, TC_K = 64, TC_STAGES = 4, TC_THREADS = 256;
 constexpr int TC_A_BYTES = TC_M * TC_K * 2, TC_B_BYTES = TC_N * TC_K * 2, TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
 // 96 KB of stages: two CTAs share an SM, and their 2 x 64 accumulator columns
 // fit its 512 tensor-memory columns
@@ -132,6 +137,30 @@ __device__ __forceinline__ float silu_grad(float z)
     return s * (1.0f + z * (1.0f - s));
 }
 
+// Programmatic dependent launch: a kernel launched with launch_after may start
+// while its predecessor in the stream finishes; grid_wait returns when that
+// one has completed and its writes are visible, grid_launch_next lets the
+// successor start.  A step is a chain of kernels of a few microseconds each,
+// so the launch gaps are a good part of it.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+void launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);   // a failure shows in cudaGetLastError
+}
+
 // Copies a 16-byte segment to shared memory asynchronously; zero fill when !ok.
 __device__ __forceinline__ void cp16(uint32_t dst, const void *src, bool ok)
 {
@@ -148,9 +177,9 @@ __device__ __forceinline__ void tc_load(uint32_t sbase, const __nv_bfloat16 *__r
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int i = 0; i < ROWS / 16; ++i) {
+    for (int i = 0; i < ROWS / 4 / (TC_THREADS / 32); ++i) {
         // unit u: rows 8 (u >> 1) .. + 7, segments 4 (u & 1) .. + 3
-        const int u = i * 4 + warp;
+        const int u = i * (TC_THREADS / 32) + warp;
         const int r = (u >> 1) * 8 + (lane & 7), kc = (u & 1) * 4 + (lane >> 3);
         const int gr = row0 + r, gk = k0 + kc * 8;
         const bool ok = gr < nrows && gk < kend;
@@ -216,7 +245,8 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
     __shared__ __align__(8) unsigned long long mbar[TC_STAGES];
     __shared__ uint32_t tmem_slot;
     __shared__ float colw[4][TC_N];
-    __shared__ double lossw[4];
+    __shared__ double lossw[TC_THREADS / 32];
+    __shared__ float bias[TC_N];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t s0 = smem_u32(tc_tiles), sbar = smem_u32(mbar);
     const int nk = kend > kbeg ? (kend - kbeg + TC_K - 1) / TC_K : 0;
@@ -228,9 +258,6 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
         }
         asm volatile("cp.async.commit_group;" ::: "memory");   // one group per round, empty past the end
     };
-#pragma unroll
-    for (int i = 0; i < TC_STAGES - 1; ++i) load(i);
-
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                      "r"(TC_TMEM_COLS)
@@ -242,6 +269,13 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
         for (int i = 0; i < TC_STAGES; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar + 8 * i) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // everything above overlaps the previous kernel's end; its results are
+    // read only from here on
+    grid_wait();
+    grid_launch_next();
+#pragma unroll
+    for (int i = 0; i < TC_STAGES - 1; ++i) load(i);
+    if (EPI != kEpiPart && EPI != kEpiBack && tid < TC_N) bias[tid] = n0 + tid < N ? e.bias[n0 + tid] : 0.0f;
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -298,10 +332,11 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
             __threadfence_system();
         }
     } else {
-        const int m = m0 + warp * 32 + lane;
+        const int quad = warp & 3, m = m0 + quad * 32 + lane;
+        const int c0 = (warp >> 2) * (TC_N / 2);
         double loss = 0.0;
 #pragma unroll 1
-        for (int c = 0; c < TC_N; c += 16) {
+        for (int c = c0; c < c0 + TC_N / 2; c += 16) {
             uint32_t v[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = 0u;
@@ -311,11 +346,11 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
                              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
                                "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
                                "=r"(v[14]), "=r"(v[15])
-                             : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
+                             : "r"(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             }
             if constexpr (EPI == kEpiPart) {
-                float4 *o = reinterpret_cast<float4 *>(part + (size_t)(warp * 32 + lane) * TC_N + c);
+                float4 *o = reinterpret_cast<float4 *>(part + (size_t)(quad * 32 + lane) * TC_N + c);
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     o[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
@@ -347,7 +382,7 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
                     for (int i = 0; i < 8; ++i) {
                         const int k = 8 * half + i;
                         float a = __uint_as_float(v[k]);
-                        if (EPI != kEpiBack && in) a += __ldg(e.bias + n + i);
+                        if (EPI != kEpiBack) a += bias[c + k];
                         if (EPI == kEpiLoss) {
                             const float r = a - t[i];
                             if (in) loss += (double)r * r * e.scale;
@@ -389,7 +424,7 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
                 }
                 if constexpr (EPI == kEpiLoss || EPI == kEpiBack) {
                     const float s = colsum16(x, lane);
-                    if (!(lane & 1)) colw[warp][c + (lane >> 1)] = s;
+                    if (!(lane & 1)) colw[quad][c + (lane >> 1)] = s;
                 }
             }
         }
@@ -403,7 +438,8 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
                 e.colpart[(size_t)(m0 / TC_M) * N + n0 + tid] =
                     (colw[0][tid] + colw[1][tid]) + (colw[2][tid] + colw[3][tid]);
             if (EPI == kEpiLoss && tid == 0)
-                e.losspart[blockIdx.y * gridDim.x + blockIdx.x] = (lossw[0] + lossw[1]) + (lossw[2] + lossw[3]);
+                e.losspart[blockIdx.y * gridDim.x + blockIdx.x] =
+                    ((lossw[0] + lossw[1]) + (lossw[2] + lossw[3])) + ((lossw[4] + lossw[5]) + (lossw[6] + lossw[7]));
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -413,7 +449,7 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
 }
 
 template <int EPI>
-__global__ void __launch_bounds__(128) gemm_tc_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
+__global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
                                                       const __nv_bfloat16 *__restrict__ B, EpiArgs e, int *err)
 {
     gemm_tile<EPI>(M, N, 0, K, A, K, B, K, blockIdx.y * TC_M, blockIdx.x * TC_N, e, nullptr, err);
@@ -432,7 +468,7 @@ struct Layers {
 // 128 x 64 tile of dW_l = H^T G over its share of the batch.  A layer alone is
 // 4 to 8 tiles of 2048 rows on a 148-SM chip; all layers' tiles times the
 // splits fill it, and the update adds the parts in a fixed order.
-__global__ void __launch_bounds__(128) gemm_dw_kernel(Layers L, int n, long long ldt, float *part, int *err)
+__global__ void __launch_bounds__(TC_THREADS) gemm_dw_kernel(Layers L, int n, long long ldt, float *part, int *err)
 {
     int l = 0;
     while (l + 1 < L.nl && (int)blockIdx.x >= L.tile0[l + 1]) ++l;
@@ -450,6 +486,7 @@ __global__ void __launch_bounds__(256) input_kernel(const float *__restrict__ X,
 {
     __shared__ __nv_bfloat16 tile[32][33];
     const int x = threadIdx.x & 31, y = threadIdx.x >> 5, c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+    grid_launch_next();
 #pragma unroll
     for (int i = y; i < 32; i += 8) {
         const int r = r0 + i, c = c0 + x;
@@ -498,6 +535,7 @@ __global__ void __launch_bounds__(256) update_kernel(Layers L, const float *__re
 {
     const int l = blockIdx.y, din = L.din[l], dout = L.dout[l];
     const int tn = (dout + TC_N - 1) / TC_N;
+    grid_wait();
     const long long nw = (long long)din * dout, n = nw + dout;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         float g = 0.0f;
@@ -553,6 +591,7 @@ struct HostSlot {
 
 struct pfk_mlp {
     int device = 0, nl = 0, max_batch = 0;
+    unsigned char *arena = nullptr;           // the device memory behind every pointer below
     std::vector<int> dims;
     std::vector<long long> w_off, b_off;      // offsets in the parameter vector
     long long nparam = 0;
@@ -638,7 +677,7 @@ void gemm(pfk_mlp *m, int M, int N, int K, const __nv_bfloat16 *A, const __nv_bf
           cudaStream_t st)
 {
     dim3 grid((N + TC_N - 1) / TC_N, row_tiles(M));
-    gemm_tc_kernel<EPI><<<grid, 128, TC_SMEM, st>>>(M, N, K, A, B, e, &m->d_slot->tc_err);
+    launch_after(gemm_tc_kernel<EPI>, grid, TC_THREADS, TC_SMEM, st, M, N, K, A, B, e, &m->d_slot->tc_err);
 }
 
 // Forward pass of n rows of X: to Y, or, with T, to dZ of the last layer and the loss.
@@ -691,7 +730,8 @@ void backward(pfk_mlp *m, int n, const Layers &L, cudaStream_t st)
         e.colpart = m->colpart + L.col_off[l - 1];
         gemm<kEpiBack>(m, n, m->dims[l], m->dims[l + 1], m->G[l], m->wb + m->w_off[l], e, st);
     }
-    gemm_dw_kernel<<<dim3(L.tiles, L.splits), 128, TC_SMEM, st>>>(L, n, m->ldt, m->part, &m->d_slot->tc_err);
+    launch_after(gemm_dw_kernel, dim3(L.tiles, L.splits), TC_THREADS, TC_SMEM, st, L, n, m->ldt, m->part,
+                 &m->d_slot->tc_err);
 }
 
 template <bool UPDATE>
@@ -700,9 +740,8 @@ void finish(pfk_mlp *m, int n, const Layers &L, const AdamArgs &a, cudaStream_t 
     long long most = 0;
     for (int l = 0; l < m->nl; ++l) most = std::max(most, (long long)L.din[l] * L.dout[l] + L.dout[l]);
     const int nloss = row_tiles(n) * ((m->dims[m->nl] + TC_N - 1) / TC_N);
-    update_kernel<UPDATE><<<dim3(blocks_for(most), m->nl), 256, 0, st>>>(
-        L, m->part, m->colpart, row_tiles(n), m->losspart, nloss, &m->d_slot->loss, m->grad, m->p, m->m, m->v, m->wb,
-        m->wt, a);
+    launch_after(update_kernel<UPDATE>, dim3(blocks_for(most), m->nl), 256, 0, st, L, m->part, m->colpart,
+                 row_tiles(n), m->losspart, nloss, &m->d_slot->loss, m->grad, m->p, m->m, m->v, m->wb, m->wt, a);
 }
 
 // After a synchronised call: PFK_ERR_CUDA if a GEMM's tensor-core wait ran out.
@@ -760,19 +799,35 @@ pfk_status pfk_mlp_create(int nlayers, const int *dims, int max_batch, int devic
     long long cols = 0;
     for (int l = 0; l < nlayers; ++l) cols += (long long)row_tiles(max_batch) * dims[l + 1];
     const size_t nloss = (size_t)row_tiles(max_batch) * ((dims[nlayers] + TC_N - 1) / TC_N);
-    auto get = [](auto **q, size_t count) { return cudaMalloc(reinterpret_cast<void **>(q), sizeof(**q) * count) == cudaSuccess; };
-    bool ok = get(&m->p, m->nparam) && get(&m->grad, m->nparam) && get(&m->m, m->nparam) && get(&m->v, m->nparam) &&
-              get(&m->wb, m->nparam) && get(&m->wt, m->nparam) &&
-              get(&m->part, (size_t)tiles * split_cap(tiles) * TC_M * TC_N) && get(&m->colpart, cols) &&
-              get(&m->losspart, nloss) &&
-              cudaHostAlloc(reinterpret_cast<void **>(&m->slot), sizeof(HostSlot), cudaHostAllocMapped) == cudaSuccess &&
-              cudaHostGetDevicePointer(reinterpret_cast<void **>(&m->d_slot), m->slot, 0) == cudaSuccess;
     for (auto *b : {&m->H, &m->HT, &m->G, &m->GT}) b->assign(nlayers, nullptr);
     m->Z.assign(nlayers, nullptr);
-    for (int l = 0; ok && l < nlayers; ++l)
-        ok = get(&m->H[l], rows * dims[l]) && get(&m->HT[l], (size_t)m->ldt * dims[l]) &&
-             get(&m->G[l], rows * dims[l + 1]) && get(&m->GT[l], (size_t)m->ldt * dims[l + 1]) &&
-             (l + 1 == nlayers || get(&m->Z[l], rows * dims[l + 1]));
+    // one allocation, carved in 256-byte steps: the first pass sizes it
+    size_t total = 0;
+    auto carve = [&]() {
+        size_t at = 0;
+        auto take = [&](auto *&q, size_t count) {
+            if (m->arena) q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(m->arena + at);
+            at += (sizeof(*q) * count + 255) & ~size_t(255);
+        };
+        for (float **q : {&m->p, &m->m, &m->v, &m->grad}) take(*q, m->nparam);
+        for (__nv_bfloat16 **q : {&m->wb, &m->wt}) take(*q, m->nparam);
+        take(m->part, (size_t)tiles * split_cap(tiles) * TC_M * TC_N);
+        take(m->colpart, cols);
+        take(m->losspart, nloss);
+        for (int l = 0; l < nlayers; ++l) {
+            take(m->H[l], rows * dims[l]);
+            take(m->HT[l], (size_t)m->ldt * dims[l]);
+            take(m->G[l], rows * dims[l + 1]);
+            take(m->GT[l], (size_t)m->ldt * dims[l + 1]);
+            if (l + 1 < nlayers) take(m->Z[l], rows * dims[l + 1]);
+        }
+        total = at;
+    };
+    carve();
+    bool ok = cudaMalloc(&m->arena, total) == cudaSuccess &&
+              cudaHostAlloc(reinterpret_cast<void **>(&m->slot), sizeof(HostSlot), cudaHostAllocMapped) == cudaSuccess &&
+              cudaHostGetDevicePointer(reinterpret_cast<void **>(&m->d_slot), m->slot, 0) == cudaSuccess;
+    if (ok) carve();
     if (!ok) return bail(mlp_fail(m, "pfk_mlp_create: device allocation failed", PFK_ERR_NOMEM));
     // the product kernels' shared-memory limits on this device
     for (const void *k : {(const void *)gemm_tc_kernel<kEpiHidden>, (const void *)gemm_tc_kernel<kEpiOut>,
@@ -782,11 +837,7 @@ pfk_status pfk_mlp_create(int nlayers, const int *dims, int max_batch, int devic
             return bail(mlp_fail(m, "pfk_mlp_create: kernel configuration failed", PFK_ERR_CUDA));
     m->slot->loss = 0.0;
     m->slot->tc_err = 0;
-    cudaMemset(m->p, 0, sizeof(float) * m->nparam);
-    cudaMemset(m->m, 0, sizeof(float) * m->nparam);
-    cudaMemset(m->v, 0, sizeof(float) * m->nparam);
-    cudaMemset(m->wb, 0, sizeof(__nv_bfloat16) * m->nparam);
-    cudaMemset(m->wt, 0, sizeof(__nv_bfloat16) * m->nparam);
+    cudaMemset(m->arena, 0, reinterpret_cast<unsigned char *>(m->part) - m->arena);   // parameters, moments, weights
     cudaStreamSynchronize(nullptr);
     *out = m;
     return PFK_OK;
@@ -797,14 +848,7 @@ pfk_status pfk_mlp_destroy(pfk_mlp *m)
     if (!m) return PFK_OK;
     cudaSetDevice(m->device);
     cudaDeviceSynchronize();
-    for (void *x : {(void *)m->p, (void *)m->grad, (void *)m->m, (void *)m->v, (void *)m->wb, (void *)m->wt,
-                    (void *)m->part, (void *)m->colpart, (void *)m->losspart})
-        if (x) cudaFree(x);
-    for (float *z : m->Z)
-        if (z) cudaFree(z);
-    for (auto *b : {&m->H, &m->HT, &m->G, &m->GT})
-        for (__nv_bfloat16 *h : *b)
-            if (h) cudaFree(h);
+    if (m->arena) cudaFree(m->arena);
     if (m->slot) cudaFreeHost(m->slot);
     delete m;
     return PFK_OK;
