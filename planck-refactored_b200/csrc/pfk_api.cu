@@ -108,6 +108,9 @@ struct pfk_ctx {
     DevBuf<uint2> d_quart;
     long long q_off[kQuartetClasses] = {}, q_cnt[kQuartetClasses] = {};
     long long q32_off[kQuartetClasses] = {}, q32_cnt[kQuartetClasses] = {};
+    // first entry of every loop-length bucket of each class's FP64 list and of
+    // its FP32 list (-1: empty bucket), longest first in the lists
+    std::vector<long long> bucket0;
     ClassLauncher launch[kQuartetClasses] = {};
     float class_ms[kQuartetClasses] = {};
     // engine auto: launch flags per class (kLaunchOS / kLaunchDense or 0 for
@@ -399,16 +402,25 @@ pfk_status build_lists(pfk_ctx *ctx)
         PFK_CK(sort_quartets(ctx->d_quart.p, maxseg, ctx->d_pairs.p, ka.p, kb.p, vb.p, nullptr, sort_bytes, ctx->stream));
         DevBuf<char> st;
         PFK_CK(st.alloc(sort_bytes + 16));
+        DevBuf<long long> starts;
+        PFK_CK(starts.alloc(2 * kQuartetClasses * kLengthBuckets));
+        PFK_CK(cudaMemsetAsync(starts.p, 0xff, sizeof(long long) * starts.n, ctx->stream));   // -1
         for (int c = 0; c < kQuartetClasses; ++c) {
             size_t b1 = sort_bytes, b2 = sort_bytes;
             PFK_CK(sort_quartets(ctx->d_quart.p + ctx->q_off[c], ctx->q_cnt[c], ctx->d_pairs.p, ka.p, kb.p, vb.p, st.p,
                                  b1, ctx->stream));
             PFK_CK(sort_quartets(ctx->d_quart.p + ctx->q32_off[c], ctx->q32_cnt[c], ctx->d_pairs.p, ka.p, kb.p, vb.p,
                                  st.p, b2, ctx->stream));
+            PFK_CK(bucket_starts(ctx->d_quart.p + ctx->q_off[c], ctx->q_cnt[c], ctx->d_pairs.p,
+                                 starts.p + (size_t)(2 * c) * kLengthBuckets, ctx->stream));
+            PFK_CK(bucket_starts(ctx->d_quart.p + ctx->q32_off[c], ctx->q32_cnt[c], ctx->d_pairs.p,
+                                 starts.p + (size_t)(2 * c + 1) * kLengthBuckets, ctx->stream));
         }
+        ctx->bucket0.resize(starts.n);
+        PFK_CK(cudaMemcpyAsync(ctx->bucket0.data(), starts.p, sizeof(long long) * starts.n, cudaMemcpyDeviceToHost,
+                               ctx->stream));
         PFK_CK(cudaStreamSynchronize(ctx->stream));
     }
-    PFK_CK(cudaStreamSynchronize(ctx->stream));
     drop_graphs(ctx);   // captured builds refer to the old lists
     return PFK_OK;
 }
@@ -493,6 +505,46 @@ static int class_components(int c)
     return ncart(pc_la(x)) * ncart(pc_lb(x)) * ncart(pc_la(y)) * ncart(pc_lb(y));
 }
 
+// Segments of a sorted list (Segments) for this context's shard.  A bucket
+// of n quartets of 2^(b-1) < K <= 2^b primitive quartets gets enough lanes per
+// quartet to put kSplitLanes threads on the chip, but leaves every lane at
+// least kSplitPrims primitive quartets (the lanes' sums cost five shuffles
+// per contracted value).
+constexpr long long kSplitLanes = 1 << 17;
+constexpr int kSplitPrims = 8;
+void list_segments(const pfk_ctx *ctx, const long long *bucket0, long long n, Segments &sg)
+{
+    sg = Segments{};
+    long long end = n;
+    int glogs[kLengthBuckets], nb = 0;
+    long long begin[kLengthBuckets];
+    // shortest bucket first: the end of the list
+    for (int b = 0; b < kLengthBuckets; ++b) {
+        if (bucket0[b] < 0) continue;
+        const long long cnt = end - bucket0[b];
+        int g = 0;
+        while (g < 5 && b > 0 && cnt << (g + 1) <= kSplitLanes && (1LL << (b - 1)) >= (long long)kSplitPrims << (g + 1)) ++g;
+        begin[nb] = bucket0[b];
+        glogs[nb++] = g;
+        end = bucket0[b];
+    }
+    auto local = [&](long long m) -> long long {
+        return m > ctx->shard_rank ? (m - ctx->shard_rank + ctx->shard_n - 1) / ctx->shard_n : 0;
+    };
+    for (int k = nb - 1; k >= 0; --k) {   // the list's order: longest first
+        const long long b0 = local(begin[k]), b1 = local(k > 0 ? begin[k - 1] : n);
+        if (b1 == b0) continue;
+        if (sg.n > 0 && (sg.glog[sg.n - 1] == glogs[k] || sg.n == kMaxSegments)) {
+            sg.count[sg.n - 1] += b1 - b0;
+            sg.glog[sg.n - 1] = std::min(sg.glog[sg.n - 1], glogs[k]);
+            continue;
+        }
+        sg.first[sg.n] = b0;
+        sg.count[sg.n] = b1 - b0;
+        sg.glog[sg.n++] = glogs[k];
+    }
+}
+
 // Launch every class kernel over the screened lists.  Jacc/K accumulators are
 // zeroed first.  eri_out selects the dense-tensor mode.
 pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const double *Pk1, int nk, FxWord *Jacc,
@@ -565,8 +617,14 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
         for (int i = 1; i < nlanes; ++i)
             if (load[i] < load[ln]) ln = i;
         load[ln] += cost[c];
-        if (nh) ctx->launch[c](ctx->d_quart.p + ctx->q_off[c], nh, a, nk, os, lane_st[ln]);
-        if (nl) ctx->launch[c](ctx->d_quart.p + ctx->q32_off[c], nl, a, nk, os | fp32, lane_st[ln]);
+        if (nh) {
+            list_segments(ctx, ctx->bucket0.data() + (size_t)(2 * c) * kLengthBuckets, ctx->q_cnt[c], a.seg);
+            ctx->launch[c](ctx->d_quart.p + ctx->q_off[c], nh, a, nk, os, lane_st[ln]);
+        }
+        if (nl) {
+            list_segments(ctx, ctx->bucket0.data() + (size_t)(2 * c + 1) * kLengthBuckets, ctx->q32_cnt[c], a.seg);
+            ctx->launch[c](ctx->d_quart.p + ctx->q32_off[c], nl, a, nk, os | fp32, lane_st[ln]);
+        }
         PFK_CK(cudaGetLastError());
         if (timed) {
             PFK_CK(cudaEventRecord(ev[1], st));

@@ -14,6 +14,46 @@ namespace {
 
 constexpr int kRegMaxComponents = 81;   // register path up to (pp|pp)-sized blocks
 
+constexpr long long kJoinQuartets = 1 << 15;
+
+// The segments of a that give a quartet several lanes in one launch of the
+// SPLIT build, the runs of the others (all n quartets when a has no segments)
+// in launches of the one-lane build.
+template <typename SplitLaunch, typename PlainLaunch>
+void launch_segments(const uint2 *q, long long n, const JKArgs &a, SplitLaunch &&split, PlainLaunch &&plain)
+{
+    if (a.seg.n == 0) {
+        plain(q, n, (unsigned)((n + 127) / 128));
+        return;
+    }
+    // few one-lane quartets go along in the SPLIT launch: a launch less
+    long long single = 0;
+    for (int s = 0; s < a.seg.n; ++s)
+        if (a.seg.glog[s] == 0) single += a.seg.count[s];
+    const bool all = single < n && single <= kJoinQuartets;
+    JKArgs b = a;
+    b.seg.n = 0;
+    unsigned blocks = 0;
+    for (int s = 0; s < a.seg.n; ++s) {
+        if (a.seg.glog[s] == 0 && !all) continue;
+        const int k = b.seg.n++;
+        b.seg.glog[k] = a.seg.glog[s];
+        b.seg.first[k] = a.seg.first[s];
+        b.seg.count[k] = a.seg.count[s];
+        b.seg.block0[k] = blocks;
+        blocks += (unsigned)(((a.seg.count[s] << a.seg.glog[s]) + 127) / 128);
+    }
+    if (blocks) split(b, blocks);
+    if (all) return;
+    for (int s = 0; s < a.seg.n; ++s) {
+        if (a.seg.glog[s] != 0) continue;
+        const long long first = a.seg.first[s];
+        long long cnt = a.seg.count[s];
+        while (s + 1 < a.seg.n && a.seg.glog[s + 1] == 0) cnt += a.seg.count[++s];
+        plain(q + first * a.qstride, cnt, (unsigned)((cnt + 127) / 128));
+    }
+}
+
 template <int LA, int LB, int LC, int LD>
 void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flags, cudaStream_t st)
 {
@@ -24,7 +64,6 @@ void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flag
     if constexpr (LA + LB + LC + LD <= kOSMaxL) {
         if (flags & kLaunchOS) {
             if (n <= 0) return;
-            const long long grid = (n + 127) / 128;
             const bool dense = flags & kLaunchDense;
             // the denser build: blocks per SM its register cap must allow.  Up
             // to L = 2 the kernels need at most 104 registers, so 4 blocks would
@@ -33,11 +72,20 @@ void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flag
             // whichever build is faster on the molecule's lists.
             constexpr int L = LA + LB + LC + LD;
             constexpr int MB = L <= 1 ? 8 : L == 2 ? 6 : 4;
-            if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
-            else if (fp32 && dense) eri_os_kernel<LA, LB, LC, LD, 1, float, MB><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
-            else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
-            else if (dense) eri_os_kernel<LA, LB, LC, LD, 1, double, MB><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
-            else eri_os_kernel<LA, LB, LC, LD, 1><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
+            launch_segments(
+                q, n, a,
+                [&](const JKArgs &b, unsigned grid) {
+                    if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2, double, 1, true><<<grid, 128, 0, st>>>(q, n, b);
+                    else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float, 1, true><<<grid, 128, 0, st>>>(q, n, b);
+                    else eri_os_kernel<LA, LB, LC, LD, 1, double, 1, true><<<grid, 128, 0, st>>>(q, n, b);
+                },
+                [&](const uint2 *r, long long m, unsigned grid) {
+                    if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2><<<grid, 128, 0, st>>>(r, m, a);
+                    else if (fp32 && dense) eri_os_kernel<LA, LB, LC, LD, 1, float, MB><<<grid, 128, 0, st>>>(r, m, a);
+                    else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float><<<grid, 128, 0, st>>>(r, m, a);
+                    else if (dense) eri_os_kernel<LA, LB, LC, LD, 1, double, MB><<<grid, 128, 0, st>>>(r, m, a);
+                    else eri_os_kernel<LA, LB, LC, LD, 1><<<grid, 128, 0, st>>>(r, m, a);
+                });
             return;
         }
     }

@@ -97,6 +97,22 @@ struct __align__(16) PairInfo {
 constexpr double kPrimPairFloor = 1e-21;
 constexpr double kPrimQuartetTol = 1e-16;
 
+// Lanes per quartet.  The one-thread-per-quartet kernels run a quartet's
+// primitive quartets in a serial loop, up to 6561 of them (81 x 81) at about
+// 0.45 us each: 3 ms on a thread, however few quartets the list holds.  A
+// list is therefore launched in segments of similar loop length (the lists
+// are ordered by it), and a segment may give each quartet 2^glog lanes of a
+// warp that share its primitive loops and add up their sums by shuffles.
+// Entries [first, first + count) of the list belong to the segment, its
+// blocks start at block0.  n = 0: one lane per quartet throughout.
+constexpr int kMaxSegments = 8;
+struct Segments {
+    int n;
+    int glog[kMaxSegments];
+    unsigned block0[kMaxSegments];
+    long long first[kMaxSegments], count[kMaxSegments];
+};
+
 struct JKArgs {
     const PairInfo *__restrict__ pairs;
     const PrimPair *__restrict__ prims;
@@ -126,6 +142,7 @@ struct JKArgs {
     double dtol;
     // primitive quartets with qp_ab qp_cd < ptol are skipped (0: none)
     double ptol;
+    Segments seg;
 };
 
 // ---------------------------------------------------------------------------

@@ -42,6 +42,7 @@ __host__ __device__ constexpr int cart_step(int L, int i, int axis, int delta)
                       cart_lz(L, i) + (axis == 2 ? delta : 0));
 }
 
+
 // Taylor coefficient (-1)^k / (k! (2M + 2k + 1)) of F_M(T).
 __host__ __device__ constexpr double boys_series_coef(int M, int k)
 {
@@ -335,26 +336,86 @@ __device__ __forceinline__ void os_hrr(const R *__restrict__ acc, const R AB[3],
     });
 }
 
-// One thread per shell quartet of an L <= 4 class, Obara-Saika integrals.
+// This thread's place in a segmented launch of 128-thread blocks (Segments):
+// list entry t (valid when in_list; the list's last entry otherwise, so that
+// every lane has a quartet to read) and lane sub of the entry's 2^glog lanes,
+// which are neighbours in a warp.
+struct LaneWork {
+    long long t;
+    int sub, glog;
+    bool in_list;
+};
+__device__ __forceinline__ LaneWork lane_work(const Segments &sg)
+{
+    LaneWork w{};
+    int s = 0;
+    while (s + 1 < sg.n && blockIdx.x >= sg.block0[s + 1]) ++s;
+    w.glog = sg.glog[s];
+    const long long u = (long long)(blockIdx.x - sg.block0[s]) * 128 + threadIdx.x;
+    const long long i = u >> w.glog;
+    w.sub = (int)(u & ((1 << w.glog) - 1));
+    w.in_list = i < sg.count[s];
+    w.t = sg.first[s] + (w.in_list ? i : sg.count[s] - 1);
+    return w;
+}
+
+// How a quartet's lanes share its loops: ket primitives j0, j0 + js, ..., and
+// for each of them bra primitives i0, i0 + is, ... (js is = 2^glog).  The ket
+// side takes as many lanes as it has primitives for: lanes of one ket
+// primitive and several bra ones would load the ket primitive once each.
+struct PrimSplit {
+    int j0, js, i0, is;
+};
+__device__ __forceinline__ PrimSplit prim_split(const LaneWork &w, int nket)
+{
+    const int gj = min(w.glog, 31 - __clz(max(nket, 1)));
+    return {w.sub & ((1 << gj) - 1), 1 << gj, w.sub >> gj, 1 << (w.glog - gj)};
+}
+
+// Sum of every lane's block over the 2^glog lanes of its quartet, left on the
+// first of them; the others hold zeros (no contribution to the digestion).
+template <int N, typename R>
+__device__ __forceinline__ void lanes_sum(R *acc, const LaneWork &w)
+{
+    if (w.glog == 0) return;   // uniform over the block
+    for (int o = 1 << (w.glog - 1); o; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < N; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if (w.sub)
+#pragma unroll
+        for (int c = 0; c < N; ++c) acc[c] = R(0);
+}
+
+// One thread (or 2^glog lanes, Segments) per shell quartet of an L <= 4 class, Obara-Saika integrals.
 // R as in eri_reg_kernel: double, or float for the FP32 list (the Boys
 // values and the per-primitive scalars stay FP64).  MINB: blocks of 128 per
 // SM the register allocation must allow (1: the compiler's choice; the
 // denser build of each class asks for 8, 6 or 4, at most 64, 80 or 128
 // registers, for the autotuner to weigh occupancy against spills).
-template <int LA, int LB, int LC, int LD, int NK, typename R = double, int MINB = 1>
+//
+// SPLIT: the launch covers args.seg, whose segments give each quartet 2^glog
+// lanes (Segments); otherwise one lane per quartet over nq entries.  Two
+// builds because the split bookkeeping costs the other one 4 to 8 registers
+// ((ss|ss) 62 -> 68: 7 blocks per SM instead of 8).
+template <int LA, int LB, int LC, int LD, int NK, typename R = double, int MINB = 1, bool SPLIT = false>
 __global__ void __launch_bounds__(128, MINB) eri_os_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
 {
     using O = OSShape<LA, LB, LC, LD>;
     constexpr int L = O::L;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    LaneWork lw{};
+    if constexpr (SPLIT) {
+        lw = lane_work(args.seg);
+    } else {
+        lw.t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        lw.in_list = lw.t < nq;
+    }
     // lanes without a quartet stay with an empty primitive loop and a zero
     // block (finish_block needs the whole warp); a warp with none leaves
-    const bool in_list = t < nq;
-    if (!__any_sync(0xffffffffu, in_list)) return;
-    const uint2 qd = quartets[(in_list ? t : nq - 1) * args.qstride + args.qoffset];
+    if (!__any_sync(0xffffffffu, lw.in_list)) return;
+    const uint2 qd = quartets[(SPLIT || lw.in_list ? lw.t : nq - 1) * args.qstride + args.qoffset];
     const PairInfo pb = args.pairs[qd.x];
     const PairInfo pk = args.pairs[qd.y];
-    const bool live = in_list && !density_negligible(pb, pk, args);
+    const bool live = lw.in_list && !density_negligible(pb, pk, args);
 
     R acc[O::NACC];
 #pragma unroll
@@ -365,10 +426,12 @@ __global__ void __launch_bounds__(128, MINB) eri_os_kernel(const uint2 *__restri
     // occupancy than the latency it hides.
     const double qb0 = pb.nprim ? __ldg(&args.prims[pb.prim_off].qp) : 0.0;   // largest bra qp
     const int nket = live ? pk.nprim : 0;
-    for (int jp = 0; jp < nket; ++jp) {
+    PrimSplit ps{0, 1, 0, 1};
+    if constexpr (SPLIT) ps = prim_split(lw, nket);
+    for (int jp = ps.j0; jp < nket; jp += ps.js) {
         const PrimPair q = load_prim(args.prims, pk.prim_off + jp);
         if (q.qp * qb0 < args.ptol) break;   // kets sorted by qp
-        for (int ip = 0; ip < pb.nprim; ++ip) {
+        for (int ip = ps.i0; ip < pb.nprim; ip += ps.is) {
             const PrimPair p = load_prim(args.prims, pb.prim_off + ip);
             if (p.qp * q.qp < args.ptol) break;   // bras sorted by qp
             const QuartetScalars s = quartet_scalars(p, q);
@@ -379,12 +442,13 @@ __global__ void __launch_bounds__(128, MINB) eri_os_kernel(const uint2 *__restri
             os_vrr<LA, LB, LC, LD, R>(Fm, p, q, s, acc);
         }
     }
+    if constexpr (SPLIT) lanes_sum<O::NACC>(acc, lw);
     constexpr int N = ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD);
     R blk[N];
     const R AB[3] = {R(pb.ABx), R(pb.ABy), R(pb.ABz)};
     const R CD[3] = {R(pk.ABx), R(pk.ABy), R(pk.ABz)};
     os_hrr<LA, LB, LC, LD, R>(acc, AB, CD, blk);
-    finish_block<LA, LB, LC, LD, NK, R>(blk, qd, pb, pk, args, live, t);
+    finish_block<LA, LB, LC, LD, NK, R>(blk, qd, pb, pk, args, live && lw.sub == 0, lw.t);
 }
 
 }  // namespace pfk

@@ -375,15 +375,46 @@ cudaError_t measure_fma_peak(int device, double *fp64, double *fp32)
 
 namespace pfk {
 
-// Sort key of a shell quartet: (evaluated bra primitives, evaluated ket
-// primitives), so that a warp's lanes run the same primitive loop lengths.
+// Loop-length bucket of a shell quartet: ceil(log2) of its primitive quartets.
+__device__ __forceinline__ int length_bucket(const PairInfo &b, const PairInfo &k)
+{
+    const unsigned n = (unsigned)b.nprim * (unsigned)k.nprim;
+    return n <= 1 ? 0 : 32 - __clz(n - 1);
+}
+
+// Sort key of a shell quartet: longest loops first (their threads finish last
+// otherwise), then (evaluated bra primitives, evaluated ket primitives), so
+// that a warp's lanes run the same primitive loop lengths.
 __global__ void quartet_key_kernel(const uint2 *__restrict__ q, long long n, const PairInfo *__restrict__ pairs,
                                    unsigned *keys)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const uint2 v = q[t];
-    keys[t] = (unsigned)pairs[v.x].nprim * 4096u + (unsigned)pairs[v.y].nprim;
+    const PairInfo b = pairs[v.x], k = pairs[v.y];
+    // nprim <= 4096 needs 13 bits, the bucket (0..24) 5
+    keys[t] = (unsigned)(31 - length_bucket(b, k)) << 26 | (unsigned)b.nprim << 13 | (unsigned)k.nprim;
+}
+
+// First entry of every length bucket of a sorted list (untouched when empty).
+__global__ void bucket_start_kernel(const uint2 *__restrict__ q, long long n, const PairInfo *__restrict__ pairs,
+                                    long long *start)
+{
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const uint2 v = q[t];
+    const int b = length_bucket(pairs[v.x], pairs[v.y]);
+    if (t > 0) {
+        const uint2 w = q[t - 1];
+        if (length_bucket(pairs[w.x], pairs[w.y]) == b) return;
+    }
+    start[b] = t;
+}
+
+cudaError_t bucket_starts(const uint2 *q, long long n, const PairInfo *pairs, long long *start, cudaStream_t st)
+{
+    if (n > 0) bucket_start_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(q, n, pairs, start);
+    return cudaGetLastError();
 }
 
 // Stable sort of one list segment by its key; tmp buffers sized by the caller
@@ -394,13 +425,13 @@ cudaError_t sort_quartets(uint2 *q, long long n, const PairInfo *pairs, unsigned
     if (!temp) {
         return cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys_a, keys_b,
                                                reinterpret_cast<unsigned long long *>(q),
-                                               reinterpret_cast<unsigned long long *>(vals_b), n, 0, 24, st);
+                                               reinterpret_cast<unsigned long long *>(vals_b), n, 0, 31, st);
     }
     if (n <= 1) return cudaSuccess;
     quartet_key_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(q, n, pairs, keys_a);
     cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys_a, keys_b,
                                                     reinterpret_cast<unsigned long long *>(q),
-                                                    reinterpret_cast<unsigned long long *>(vals_b), n, 0, 24, st);
+                                                    reinterpret_cast<unsigned long long *>(vals_b), n, 0, 31, st);
     if (e != cudaSuccess) return e;
     return cudaMemcpyAsync(q, vals_b, sizeof(uint2) * n, cudaMemcpyDeviceToDevice, st);
 }

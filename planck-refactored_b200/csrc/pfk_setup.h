@@ -30,6 +30,11 @@ cudaError_t measure_fma_peak(int device, double *fp64, double *fp32);
 // every non-null density P0..P2 (rounded up to FP32), for density screening.
 cudaError_t shell_block_max(int nshell, const int *bf_off, const int *nbf, const double *P0, const double *P1,
                             const double *P2, int nb, float *D, cudaStream_t st);
+// start[b] = first entry of the sorted list whose loop length is in bucket b
+// (kLengthBuckets of them, ceil(log2) of the primitive quartets); entries of
+// empty buckets stay as they are.
+constexpr int kLengthBuckets = 25;
+cudaError_t bucket_starts(const uint2 *q, long long n, const PairInfo *pairs, long long *start, cudaStream_t st);
 cudaError_t sort_quartets(uint2 *q, long long n, const PairInfo *pairs, unsigned *keys_a, unsigned *keys_b,
                           uint2 *vals_b, void *temp, size_t &temp_bytes, cudaStream_t st);
 
