@@ -26,10 +26,10 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + CSRC,
 
 DEVICE_DEPS = ["pfk_device.cuh", "pfk_internal.h", "rys_table_data.inc", "../../include/planck_fock.h"]
 DEPS = {
-    "pfk_classes.cu": DEVICE_DEPS + ["pfk_kernels.cuh", "pfk_os.cuh"],
+    "pfk_classes.cu": DEVICE_DEPS + ["pfk_kernels.cuh", "pfk_os.cuh", "boys_table_data.inc"],
     "pfk_setup.cu": DEVICE_DEPS + ["pfk_kernels.cuh", "pfk_setup.h"],
     "pfk_api.cu": DEVICE_DEPS + ["pfk_setup.h", "../../include/planck_fock.h"],
-    "pfk_onee.cu": DEVICE_DEPS + ["pfk_kernels.cuh", "pfk_os.cuh"],
+    "pfk_onee.cu": DEVICE_DEPS + ["pfk_kernels.cuh", "pfk_os.cuh", "boys_table_data.inc"],
     "pfk_mlp.cu": ["../../include/planck_fock.h"],
     "pfk_checkpoint.cu": ["../../include/planck_fock.h"],
     "pfk_scf.cu": ["../../include/planck_fock.h", "pfk_internal.h", "pfk_device.cuh"],

@@ -72,6 +72,10 @@ void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flag
             // whichever build is faster on the molecule's lists.
             constexpr int L = LA + LB + LC + LD;
             constexpr int MB = L <= 1 ? 8 : L == 2 ? 6 : 4;
+            // the plain build: left alone the compiler takes 94 registers at
+            // L = 1 and 190 at L = 3 to have more of the Boys polynomials in
+            // flight, at 5 and 2 blocks per SM
+            constexpr int PB = L == 0 ? 8 : L == 1 ? 6 : L == 2 ? 5 : L == 3 ? 3 : 1;
             launch_segments(
                 q, n, a,
                 [&](const JKArgs &b, unsigned grid) {
@@ -80,11 +84,11 @@ void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flag
                     else eri_os_kernel<LA, LB, LC, LD, 1, double, 1, true><<<grid, 128, 0, st>>>(q, n, b);
                 },
                 [&](const uint2 *r, long long m, unsigned grid) {
-                    if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2><<<grid, 128, 0, st>>>(r, m, a);
+                    if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2, double, PB><<<grid, 128, 0, st>>>(r, m, a);
                     else if (fp32 && dense) eri_os_kernel<LA, LB, LC, LD, 1, float, MB><<<grid, 128, 0, st>>>(r, m, a);
-                    else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float><<<grid, 128, 0, st>>>(r, m, a);
+                    else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float, PB><<<grid, 128, 0, st>>>(r, m, a);
                     else if (dense) eri_os_kernel<LA, LB, LC, LD, 1, double, MB><<<grid, 128, 0, st>>>(r, m, a);
-                    else eri_os_kernel<LA, LB, LC, LD, 1><<<grid, 128, 0, st>>>(r, m, a);
+                    else eri_os_kernel<LA, LB, LC, LD, 1, double, PB><<<grid, 128, 0, st>>>(r, m, a);
                 });
             return;
         }

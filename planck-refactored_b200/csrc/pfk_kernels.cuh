@@ -680,6 +680,11 @@ struct SplitShape {
     static constexpr bool TEAMRED =
         LEVEL == 1 && TEAM <= 32 && (REDV1 + 2 * REDVK) * GROUP * 8 <= TABLE * (int)sizeof(R);
     static constexpr bool OK = TEAM <= 128 && M <= 64;
+    // blocks of 128 per SM the register allocation must allow: the kernels
+    // wait on loads more than on arithmetic, so four where the accumulators
+    // leave room: (H2O)32 (dd|ps) 1.57 -> 1.43 ms, (dd|dp) 1.19 -> 1.01 (both
+    // M = 18); at M = 27 the spills cost more ((dp|pp) 3.42 -> 3.70)
+    static constexpr int MINB = M <= 18 ? 4 : 3;
 };
 
 template <int TEAM>
@@ -716,7 +721,7 @@ __device__ __forceinline__ int cart_l_axis(int i, int axis)
 // Schwarz bound is below the FP32 threshold); roots, weights and the
 // per-primitive scalars stay FP64, and so does the digestion.
 template <int LA, int LB, int LC, int LD, int NK, typename R = double>
-__global__ void __launch_bounds__(128, 3) eri_split_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
+__global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) eri_split_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
 {
     using S = ClassShape<LA, LB, LC, LD>;
     using SS = SplitShape<LA, LB, LC, LD, R>;

@@ -4,9 +4,9 @@
 // The reference runs the vertical recurrence once per Cartesian component
 // quartet and primitive, then a horizontal recurrence.  Here one thread owns
 // a whole shell quartet of class (LA LB | LC LD), L = LA+LB+LC+LD <= 4:
-//   * Boys values F_0..F_L (boys_fm) in registers, from a Taylor series for
-//     small T and from erf/exp with upward recursion otherwise -- no table
-//     reads, so these kernels do not compete for L1 with the Rys tables;
+//   * Boys values F_0..F_L (boys_fm) in registers, from polynomials with
+//     constant-bank coefficients -- no table reads, so these kernels do not
+//     compete for L1 with the Rys tables;
 //   * the vertical recurrence (Obara-Saika / Head-Gordon-Pople form) builds
 //     [e0|f0] for e in [LA, LA+LB], f in [LC, LC+LD] per primitive quartet
 //     and accumulates them contracted;
@@ -19,6 +19,8 @@
 #include "pfk_kernels.cuh"
 
 namespace pfk {
+
+#include "boys_table_data.inc"
 
 // Cartesian component index of exponents (x, y, z), the inverse of
 // cart_lx/ly/lz (lx descending, then ly descending).
@@ -43,75 +45,106 @@ __host__ __device__ constexpr int cart_step(int L, int i, int axis, int delta)
 }
 
 
-// Taylor coefficient (-1)^k / (k! (2M + 2k + 1)) of F_M(T).
-__host__ __device__ constexpr double boys_series_coef(int M, int k)
+// sum_k c[k] x^k, k = 0 .. N, as even and odd halves in x^2: two chains of
+// N / 2 dependent steps.  The coefficients are __constant__ (and not const, so
+// that they stay there): the FMAs read them as constant-bank operands, where
+// 64-bit literals would take two moves each.
+template <int N>
+__device__ __forceinline__ double poly_even_odd(const double *c, double x)
 {
-    double f = 1.0;
-    for (int j = 2; j <= k; ++j) f *= j;
-    return (k % 2 ? -1.0 : 1.0) / (f * (2 * M + 2 * k + 1));
+    constexpr int E = N & ~1, O = (N - 1) | 1;   // highest even and odd degree
+    const double x2 = x * x;
+    double e = c[E], o = c[O];
+#pragma unroll
+    for (int k = E - 2; k >= 0; k -= 2) e = fma(e, x2, c[k]);
+#pragma unroll
+    for (int k = O - 2; k >= 1; k -= 2) o = fma(o, x2, c[k]);
+    return fma(o, x, e);
+}
+template <int N>
+__device__ __forceinline__ double poly_horner(const double *c, double x)
+{
+    double s = c[N];
+#pragma unroll
+    for (int k = N - 1; k >= 0; --k) s = fma(s, x, c[k]);
+    return s;
 }
 
-// The series coefficients as a constant-memory table: the FMAs of the series
-// then read them as constant-bank operands instead of materialising each
-// 64-bit literal in registers.
-struct BoysSeriesTable {
-    double c[7][32];
-};
-__host__ __device__ constexpr BoysSeriesTable make_boys_series_table()
+// e^-T, 0 <= T < 700: T = -(n ln 2 + r) with n = rint(-T log2 e) (Cody and
+// Waite's two-part ln 2), e^r by interpolation (kBoysExp), n into the
+// exponent.  n is read from the low bits of 1.5 2^52 + n.
+__device__ __forceinline__ double boys_exp(double T)
 {
-    BoysSeriesTable t{};
-    for (int M = 0; M < 7; ++M)
-        for (int k = 0; k < 32; ++k) t.c[M][k] = boys_series_coef(M, k);
-    return t;
+    constexpr double kLog2e = 1.4426950408889634074, kMagic = 6755399441055744.0;
+    constexpr double kLn2Hi = 0.693147180559890330187045037746429443359375;   // ln 2 in 42 bits
+    constexpr double kLn2Lo = 5.497923018708371174712471e-14;                 // ln 2 - kLn2Hi
+    const double t = fma(T, -kLog2e, kMagic);
+    const double n = t - kMagic;
+    const double r = fma(n, -kLn2Lo, fma(n, -kLn2Hi, -T));
+    const double p = poly_even_odd<kBoysExpDeg>(kBoysExp, r);
+    return __hiloint2double(__double2hiint(p) + (__double2loint(t) << 20), __double2loint(p));
 }
-static __constant__ const BoysSeriesTable kBoysSeries = make_boys_series_table();
 
-// Boys function F_m(T), m = 0..M (M <= 6).  T below TS: the Taylor series of
-// F_M and downward recursion F_m = (2T F_{m+1} + e^-T) / (2m+1), which is
-// stable.  T >= TS: F_0 = sqrt(pi)/2 erf(sqrt T)/sqrt T (with erf(sqrt T) =
-// 1 - e^-T erfcx(sqrt T), so one exponential serves all m) and the upward
-// recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T); its error growth stays
-// below ~10x for m <= 4 at T >= 2 (~2x for m <= 1 at T >= 1; TS = 3 for
-// m = 5, 6).  T >= TA: the large-T limit F_0 = sqrt(pi / 4T), F_{m+1} =
-// (2m+1) F_m / (2T), with no erf or exp; TA = 34, 38, 42, 44, 46 for
-// M = 0..4 is where the limit's relative error (the dropped e^-T terms)
-// falls to its own rounding level against 40-digit values, 60 above M = 4.
-// Measured against 40-digit values: max relative error 1e-15 (M <= 1),
-// 8e-15 (M = 4), 2e-14 (M = 6).
+// Boys function F_m(T), m = 0..M (M <= 6).
+//
+// T < TA, M = 0: F_0 = P(y) / sqrt(T + 16), y linear in T / (T + 16)
+// (kBoysMid; gen_boys_table.py).  One polynomial covers the whole range, so
+// the lanes of a warp, whose T are unrelated, run one path of about 40
+// instructions.  M >= 1: the same for T >= TS, then the upward recursion
+// F_{m+1} = ((2m+1) F_m - e^-T) / (2T), whose error growth stays below ~10x
+// for m <= 4 at T >= 2 (TS = 1 for M = 1, 2 up to M = 4, 3 above); for T < TS
+// F_M by interpolation in T (kBoysSmall) and the stable downward recursion
+// F_m = (2T F_{m+1} + e^-T) / (2m+1).  One rsqrt gives both 1/sqrt(T + 16)
+// and 1/T: r = 1 / (T sqrt(T + 16)).
+// T >= TA: the large-T limit F_0 = sqrt(pi / 4T), F_{m+1} = (2m+1) F_m /
+// (2T); TA = 34, 38, 42, 44, 46 for M = 0..4 is where the limit's relative
+// error (the dropped e^-T terms) falls to its own rounding level, 60 above.
+//
+// Largest relative error against 40-digit values: 4e-16 (M = 0), 7e-16 (1),
+// 1e-15 (2), 3e-15 (3), 5e-15 (4), 1e-14 (6); with the Taylor series below TS
+// and 1 - e^-T erfcx above, which this replaces, 1e-15 (M <= 1), 8e-15 (4),
+// 2e-14 (6).  The library's exp and erfcx keep their coefficients as
+// literals, and a warp paid for both branches: with them
+// (ss|ss) issued 160 instructions per primitive quartet, 26% of them FP64.
+// (H2O)32 / 6-31G**: (ss|ss) 3.16 -> 2.17 ms, (ps|ss) 5.56 -> 4.96; C40H82 /
+// cc-pVDZ build 289 -> 245 ms.
 template <int M>
 __device__ __forceinline__ void boys_fm(double T, double *F)
 {
-    constexpr double TS = M <= 1 ? 1.0 : M <= 4 ? 2.0 : 3.0;
-    constexpr int NT = M <= 1 ? 18 : M <= 4 ? 25 : 32;   // terms: last term < 1e-17 at T = TS
-    constexpr double TA = M == 0 ? 34.0 : M == 1 ? 38.0 : M == 2 ? 42.0 : M == 3 ? 44.0 : M == 4 ? 46.0 : 60.0;
-    if (T < TS) {
-        double s = kBoysSeries.c[M][NT - 1];
-#pragma unroll
-        for (int k = NT - 2; k >= 0; --k) s = fma(s, T, kBoysSeries.c[M][k]);
-        F[M] = s;
-        if constexpr (M > 0) {
-            const double e = exp(-T);
-#pragma unroll
-            for (int m = M - 1; m >= 0; --m) F[m] = fma(2.0 * T, F[m + 1], e) * (1.0 / (2 * m + 1));
-        }
-    } else if (T < TA) {
-        // erf(sqrt T) = 1 - e^-T erfcx(sqrt T): one exponential serves both
-        // F_0 and the recursion (erfc(sqrt T) <= erfc(1) = 0.16, no cancellation)
-        const double ist = rsqrt(T);
-        const double e = exp(-T);
-        F[0] = 0.88622692545275801365 * fma(-e, erfcx(T * ist), 1.0) * ist;   // sqrt(pi)/2
-        if constexpr (M > 0) {
-            const double h = 0.5 * ist * ist;                     // 1/(2T)
-#pragma unroll
-            for (int m = 0; m < M; ++m) F[m + 1] = fma(double(2 * m + 1), F[m], -e) * h;
-        }
+    constexpr double TS = kBoysTS[M], TA = kBoysTA[M], kScale = kBoysMidScale[M];
+    constexpr double kHalfSqrtPi = 0.88622692545275801365;
+    const bool near = T < TA;
+    const double s = T + kBoysShift;
+    if constexpr (M == 0) {
+        const double rs = rsqrt(near ? s : T);
+        double f = kHalfSqrtPi;
+        if (near) f = poly_even_odd<kBoysMidDeg[M]>(kBoysMid[M], fma(T * (rs * rs), kScale, -1.0));
+        F[0] = f * rs;
     } else {
-        // erfc(sqrt T) and e^-T are below 1e-17 of every (2m+1) F_m here
-        const double ist = rsqrt(T);
-        F[0] = 0.88622692545275801365 * ist;
-        const double h = 0.5 * ist * ist;
+        const double r = rsqrt(near ? T * T * s : T);
+        if (near) {
+            const double e = boys_exp(T);
+            if (T < TS) {
+                F[M] = poly_even_odd<kBoysSmallDeg[M]>(kBoysSmall[M], T);
 #pragma unroll
-        for (int m = 0; m < M; ++m) F[m + 1] = double(2 * m + 1) * h * F[m];
+                for (int m = M - 1; m >= 0; --m) F[m] = fma(2.0 * T, F[m + 1], e) * (1.0 / (2 * m + 1));
+            } else {
+                const double rs = r * T;             // 1 / sqrt(T + 16)
+                const double h = 0.5 * r * (s * rs);   // 1 / (2T)
+                const double y = fma(T * (rs * rs), kScale, -1.0);
+                // the two halves of the longest polynomials cancel more than a digit
+                F[0] = rs * (M <= 4 ? poly_even_odd<kBoysMidDeg[M]>(kBoysMid[M], y)
+                                    : poly_horner<kBoysMidDeg[M]>(kBoysMid[M], y));
+#pragma unroll
+                for (int m = 0; m < M; ++m) F[m + 1] = fma(double(2 * m + 1), F[m], -e) * h;
+            }
+        } else {
+            // erfc(sqrt T) and e^-T are below 1e-17 of every (2m+1) F_m here
+            F[0] = kHalfSqrtPi * r;
+            const double h = 0.5 * r * r;
+#pragma unroll
+            for (int m = 0; m < M; ++m) F[m + 1] = double(2 * m + 1) * h * F[m];
+        }
     }
 }
 

@@ -1,0 +1,119 @@
+"""The Boys evaluation of the Obara-Saika and nuclear-attraction kernels
+(boys_fm in csrc/pfk_os.cuh) restated with the tables the kernels include
+(csrc/boys_table_data.inc) and checked against 40-digit values (CPU test).
+
+Bounds: a fused multiply-add chain whose terms add up to about the result
+leaves 1 to 2 units of 2^-53 relative, the reciprocal square root and the
+factors around it another 2: 5e-16 for F_0.  Each upward step multiplies the
+error by up to (2m+1) F_m / (2T F_{m+1}), at T = TS: 2.2 from F_0 to F_1 at
+TS = 1, at most 2.4 a step at TS = 2 (M <= 4) and 2.0 at TS = 3 (M = 6)."""
+import importlib
+import math
+import os
+import re
+
+import numpy as np
+import pytest
+
+mpmath = pytest.importorskip("mpmath")
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "planck-refactored_b200", "csrc")
+
+
+def _tables():
+    text = open(os.path.join(CSRC, "boys_table_data.inc")).read()
+    out = {}
+    for name, body in re.findall(r"(\w+)\[[^=;]*\] = (\{.*?\});", text, re.S):
+        rows = re.findall(r"\{([^{}]*)\}", body)
+        vals = [[float(v) for v in r.split(",") if v.strip()] for r in rows]
+        out[name] = vals if len(vals) > 1 else vals[0]
+    return out
+
+
+T_ = _tables()
+SHIFT = 16.0
+
+
+def _fma(a, b, c):
+    return float(np.float64(np.longdouble(a) * np.longdouble(b) + np.longdouble(c)))
+
+
+def _horner(c, x):
+    s = c[-1]
+    for v in c[-2::-1]:
+        s = _fma(s, x, v)
+    return s
+
+
+def _even_odd(c, x):
+    return _fma(_horner(c[1::2], x * x), x, _horner(c[0::2], x * x))
+
+
+def _rsqrt(v):
+    return float(1 / mpmath.sqrt(mpmath.mpf(v)))
+
+
+def _exp(t):
+    n = float(np.rint(-t * 1.4426950408889634074))
+    r = _fma(n, -5.497923018708371174712471e-14, _fma(n, -0.693147180559890330187045037746429443359375, -t))
+    return math.ldexp(_even_odd(T_["kBoysExp"], r), int(n))
+
+
+def boys(M, T):
+    ts, ta, scale = T_["kBoysTS"][M], T_["kBoysTA"][M], T_["kBoysMidScale"][M]
+    mid = T_["kBoysMid"][M][:int(T_["kBoysMidDeg"][M]) + 1]
+    small = T_["kBoysSmall"][M][:int(T_["kBoysSmallDeg"][M]) + 1]
+    near, s = T < ta, T + SHIFT
+    if M == 0:
+        rs = _rsqrt(s if near else T)
+        return [(_even_odd(mid, _fma(T * (rs * rs), scale, -1.0)) if near else 0.88622692545275801365) * rs]
+    F = [0.0] * (M + 1)
+    if near and T < ts:
+        e = _exp(T)
+        F[M] = _even_odd(small, T)
+        for m in range(M - 1, -1, -1):
+            F[m] = _fma(2.0 * T, F[m + 1], e) * (1.0 / (2 * m + 1))
+        return F
+    r = _rsqrt(T * T * s if near else T)
+    if near:
+        e, rs = _exp(T), r * T
+        h = 0.5 * r * (s * rs)
+        F[0] = rs * (_even_odd if M <= 4 else _horner)(mid, _fma(T * (rs * rs), scale, -1.0))
+        for m in range(M):
+            F[m + 1] = _fma(2 * m + 1.0, F[m], -e) * h
+    else:
+        F[0] = 0.88622692545275801365 * r
+        for m in range(M):
+            F[m + 1] = (2 * m + 1) * (0.5 * r * r) * F[m]
+    return F
+
+
+@pytest.mark.parametrize("M,bound", [(0, 5e-16), (1, 1e-15), (2, 2e-15), (3, 4e-15), (4, 8e-15), (5, 1e-14),
+                                     (6, 2e-14)])
+def test_relative_error(M, bound):
+    rng = np.random.default_rng(50 + M)
+    ts, ta = T_["kBoysTS"][M], T_["kBoysTA"][M]
+    Ts = np.concatenate([rng.uniform(0, 3, 100), rng.uniform(0, 80, 150), rng.uniform(ta - 3, ta + 3, 40),
+                         np.logspace(-300, 3, 30),
+                         [0.0, ts * (1 - 1e-15), ts, ts * (1 + 1e-15), ta * (1 - 1e-15), ta]])
+    worst = 0.0
+    with mpmath.workdps(40):
+        for T in Ts:
+            F, t = boys(M, float(T)), mpmath.mpf(float(T))
+            for m in range(M + 1):
+                a = m + mpmath.mpf(1) / 2
+                ref = 1 / (2 * a) if t < 1e-30 else mpmath.gammainc(a, 0, t) / (2 * t ** a)
+                worst = max(worst, float(abs((F[m] - ref) / ref)))
+    assert worst < bound, worst
+
+
+def test_tables_are_the_generators():
+    """The committed table is what gen_boys_table.py writes."""
+    g = importlib.import_module("planck-refactored_b200.gen_boys_table")
+    t = g.tables()
+    for M in range(7):
+        assert T_["kBoysMid"][M][:g.MID_DEG[M] + 1] == t["mid"][M]
+        assert T_["kBoysSmall"][M][:g.SMALL_DEG[M] + 1] == t["small"][M]
+    assert T_["kBoysExp"] == t["exp"] and T_["kBoysMidScale"] == t["mid_scale"]
+    assert [int(v) for v in T_["kBoysTA"]] == g.TA and [int(v) for v in T_["kBoysTS"]] == g.TS
