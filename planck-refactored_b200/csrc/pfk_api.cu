@@ -58,7 +58,15 @@ struct GraphEntry {
 
 }  // namespace
 
-constexpr int kMaxLanes = 4;
+// Launch streams of a build: pfk_set_lanes takes 1 to kMaxLanes; by default
+// kMaxLanes, or kSmallLanes for lists of at most kSmallQuartets shell
+// quartets.  There a class kernel is a few blocks and lasts as long as one
+// quartet's chain of loads, recurrences and adds (20 to 60 us), so what counts
+// is how many run at once: one water / 6-31G** 272 -> 149 us a build with
+// 12 instead of 4; more than 4 were slower for (H2O)32 (49.8 ms with 4, 50.4
+// with 6, 50.6 with 8).
+constexpr int kMaxLanes = 4, kSmallLanes = 12;
+constexpr long long kSmallQuartets = 4 << 20;
 
 struct pfk_ctx {
     int device = 0;
@@ -66,9 +74,11 @@ struct pfk_ctx {
     std::string err;
     // concurrent class launches: lanes - 1 side streams forked from the
     // build's stream (fork_ev) and joined back (join_ev) around the classes
-    int lanes = kMaxLanes;
-    cudaStream_t side[kMaxLanes - 1] = {};
-    cudaEvent_t fork_ev = nullptr, join_ev[kMaxLanes - 1] = {};
+    int lanes = 0;                    // 0: by the size of the lists (auto_lanes)
+    int auto_lanes = kMaxLanes;       // set by build_lists
+    int nside = 0;                    // side streams created so far
+    cudaStream_t side[kSmallLanes - 1] = {};
+    cudaEvent_t fork_ev = nullptr, join_ev[kSmallLanes - 1] = {};
     cublasHandle_t blas = nullptr;   // created by the first pfk_mo_transform
     double mo_ms[3] = {0.0, 0.0, 0.0};   // last pfk_mo_transform: AO tensor, GEMMs, copy out
     // two pinned staging chunks for copying MO blocks into pageable host memory
@@ -306,6 +316,17 @@ void drop_graphs(pfk_ctx *ctx)
     ctx->graphs.clear();
 }
 
+// Creates the context's side streams up to n of them.
+cudaError_t side_streams(pfk_ctx *ctx, int n)
+{
+    for (; ctx->nside < n; ++ctx->nside) {
+        cudaError_t e = cudaStreamCreateWithFlags(&ctx->side[ctx->nside], cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->join_ev[ctx->nside], cudaEventDisableTiming);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 // Pair classes from fs on hold an f shell.  Quartet classes with one keep
 // their whole list in FP64: on the ERI class microbenchmark's random shells
 // the FP32 variants of those classes lose up to 1e-5 (fd|fd) and more
@@ -361,6 +382,8 @@ pfk_status build_lists(pfk_ctx *ctx)
         ctx->q32_off[c] = pos;
         pos += ctx->q32_cnt[c];
     }
+    ctx->auto_lanes = total <= kSmallQuartets ? kSmallLanes : kMaxLanes;
+    PFK_CK(side_streams(ctx, ctx->auto_lanes - 1));
     PFK_CK(ctx->d_quart.alloc((size_t)std::max(total, 1LL)));
     // pass 2: fill
     for (int x = 0; x < kPairClasses; ++x)
@@ -588,8 +611,8 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
     }
     // lanes: the classes go, largest estimated cost first, to the lane with
     // the least work so far; a per-class timed pass stays on one stream
-    const int nlanes = timed ? 1 : ctx->lanes;
-    cudaStream_t lane_st[kMaxLanes] = {st};
+    const int nlanes = timed ? 1 : ctx->lanes ? ctx->lanes : ctx->auto_lanes;
+    cudaStream_t lane_st[kSmallLanes] = {st};
     if (nlanes > 1) {
         PFK_CK(cudaEventRecord(ctx->fork_ev, st));
         for (int i = 1; i < nlanes; ++i) {
@@ -605,7 +628,7 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
     }
     if (nlanes > 1)
         std::stable_sort(order, order + kQuartetClasses, [&](int x, int y) { return cost[x] > cost[y]; });
-    double load[kMaxLanes] = {};
+    double load[kSmallLanes] = {};
     for (int oc = 0; oc < kQuartetClasses; ++oc) {
         const int c = order[oc];
         const long long nh = local(ctx->q_cnt[c]), nl = local(ctx->q32_cnt[c]);
@@ -729,12 +752,8 @@ pfk_status pfk_create(const pfk_basis_desc *basis, int device, pfk_ctx **out)
         if (e != cudaSuccess) return bail(ctx->cuda_fail("cudaStreamCreate", e));
         e = cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming);
         if (e != cudaSuccess) return bail(ctx->cuda_fail("cudaEventCreate", e));
-        for (int i = 0; i < kMaxLanes - 1; ++i) {
-            e = cudaStreamCreateWithFlags(&ctx->side[i], cudaStreamNonBlocking);
-            if (e != cudaSuccess) return bail(ctx->cuda_fail("cudaStreamCreate", e));
-            e = cudaEventCreateWithFlags(&ctx->join_ev[i], cudaEventDisableTiming);
-            if (e != cudaSuccess) return bail(ctx->cuda_fail("cudaEventCreate", e));
-        }
+        e = side_streams(ctx, kMaxLanes - 1);
+        if (e != cudaSuccess) return bail(ctx->cuda_fail("side streams", e));
         ctx->nshell = basis->nshell;
         ctx->L.assign(basis->L, basis->L + basis->nshell);
         ctx->bf_off.resize(basis->nshell);
@@ -817,7 +836,7 @@ pfk_status pfk_destroy(pfk_ctx *ctx)
     ctx->d_Dsh.release();
     for (DevBuf<double> *b : {&ctx->d_P, &ctx->d_Pb, &ctx->d_Pt, &ctx->d_G, &ctx->d_Gb}) b->release();
     for (DevBuf<FxWord> *b : {&ctx->d_J, &ctx->d_K0, &ctx->d_K1}) b->release();
-    for (int i = 0; i < kMaxLanes - 1; ++i) {
+    for (int i = 0; i < kSmallLanes - 1; ++i) {
         if (ctx->side[i]) cudaStreamDestroy(ctx->side[i]);
         if (ctx->join_ev[i]) cudaEventDestroy(ctx->join_ev[i]);
     }

@@ -2,11 +2,14 @@
 (boys_fm in csrc/pfk_os.cuh) restated with the tables the kernels include
 (csrc/boys_table_data.inc) and checked against 40-digit values (CPU test).
 
-Bounds: a fused multiply-add chain whose terms add up to about the result
+Bound: a fused multiply-add chain whose terms add up to about the result
 leaves 1 to 2 units of 2^-53 relative, the reciprocal square root and the
-factors around it another 2: 5e-16 for F_0.  Each upward step multiplies the
-error by up to (2m+1) F_m / (2T F_{m+1}), at T = TS: 2.2 from F_0 to F_1 at
-TS = 1, at most 2.4 a step at TS = 2 (M <= 4) and 2.0 at TS = 3 (M = 6)."""
+factors around it another 2: 5e-16 for F_0.  An upward step multiplies the
+relative error by (2m+1) F_m / (2T F_{m+1}), largest at T = TS, adds that of
+e^-T (3e-16) times e^-T / (2T F_{m+1}), and that of h = 1/(2T) = 0.5 r (s r T):
+r enters twice (its argument's two roundings halved and its own: 2.2e-16
+each time) and four roundings follow, the product's included: 6e-16.  The next
+steps multiply all of it in turn."""
 import importlib
 import math
 import os
@@ -89,9 +92,21 @@ def boys(M, T):
     return F
 
 
-@pytest.mark.parametrize("M,bound", [(0, 5e-16), (1, 1e-15), (2, 2e-15), (3, 4e-15), (4, 8e-15), (5, 1e-14),
-                                     (6, 2e-14)])
-def test_relative_error(M, bound):
+def _exact(m, t):
+    a = m + mpmath.mpf(1) / 2
+    return 1 / (2 * a) if t < 1e-30 else mpmath.gammainc(a, 0, t) / (2 * t ** a)
+
+
+def _bound(M):
+    err, t = 5e-16, mpmath.mpf(T_["kBoysTS"][M])
+    for m in range(M):
+        up = float((2 * m + 1) * _exact(m, t) / (2 * t * _exact(m + 1, t)))
+        err = err * up + 3e-16 * (up - 1) + 6e-16     # e^-T = (up - 1) 2T F_{m+1}
+    return err
+
+
+@pytest.mark.parametrize("M", range(7))
+def test_relative_error(M):
     rng = np.random.default_rng(50 + M)
     ts, ta = T_["kBoysTS"][M], T_["kBoysTA"][M]
     Ts = np.concatenate([rng.uniform(0, 3, 100), rng.uniform(0, 80, 150), rng.uniform(ta - 3, ta + 3, 40),
@@ -102,10 +117,9 @@ def test_relative_error(M, bound):
         for T in Ts:
             F, t = boys(M, float(T)), mpmath.mpf(float(T))
             for m in range(M + 1):
-                a = m + mpmath.mpf(1) / 2
-                ref = 1 / (2 * a) if t < 1e-30 else mpmath.gammainc(a, 0, t) / (2 * t ** a)
+                ref = _exact(m, t)
                 worst = max(worst, float(abs((F[m] - ref) / ref)))
-    assert worst < bound, worst
+    assert worst < _bound(M), (worst, _bound(M))
 
 
 def test_tables_are_the_generators():
