@@ -33,12 +33,16 @@ struct DevBuf {
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
     ~DevBuf() { release(); }   // the temporaries of list building are freed on every path
+    // at least `count` elements, keeping what is there if it is enough
+    cudaError_t reserve(size_t count) { return count <= n ? cudaSuccess : alloc(count); }
     cudaError_t alloc(size_t count)
     {
         release();
-        n = count;
         if (count == 0) return cudaSuccess;
-        return cudaMalloc(reinterpret_cast<void **>(&p), sizeof(T) * count);
+        const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&p), sizeof(T) * count);
+        if (e == cudaSuccess) n = count;
+        else p = nullptr;
+        return e;
     }
     void release()
     {
@@ -81,6 +85,9 @@ struct pfk_ctx {
     cudaEvent_t fork_ev = nullptr, join_ev[kSmallLanes - 1] = {};
     cublasHandle_t blas = nullptr;   // created by the first pfk_mo_transform
     double mo_ms[3] = {0.0, 0.0, 0.0};   // last pfk_mo_transform: AO tensor, GEMMs, copy out
+    // buffers of the MO transform (mo_run), kept for the next call while they
+    // are within kMoKeepBytes together
+    DevBuf<double> mo_E, mo_T1, mo_T2, mo_C, mo_red;
     // two pinned staging chunks for copying MO blocks into pageable host memory
     void *pin[2] = {nullptr, nullptr};
     cudaEvent_t pin_ev[2] = {nullptr, nullptr};
@@ -834,6 +841,7 @@ pfk_status pfk_destroy(pfk_ctx *ctx)
     ctx->d_shell_bf.release();
     ctx->d_shell_nbf.release();
     ctx->d_Dsh.release();
+    for (DevBuf<double> *b : {&ctx->mo_E, &ctx->mo_T1, &ctx->mo_T2, &ctx->mo_C, &ctx->mo_red}) b->release();
     for (DevBuf<double> *b : {&ctx->d_P, &ctx->d_Pb, &ctx->d_Pt, &ctx->d_G, &ctx->d_Gb}) b->release();
     for (DevBuf<FxWord> *b : {&ctx->d_J, &ctx->d_K0, &ctx->d_K1}) b->release();
     for (int i = 0; i < kSmallLanes - 1; ++i) {
@@ -1104,14 +1112,32 @@ __global__ void __launch_bounds__(256) mp2_sum_kernel(const double *__restrict__
 // result goes to the host buffer `out`, or, with eps1 set (blocks occ, vir,
 // occ, vir; eps1 and eps2 the nbasis orbital energies of the first and the
 // second pair's spin), into the MP2 sum of `mode` in *e_corr without leaving
-// the device.  shared_E: an AO tensor (nbasis^4) kept across calls -- built
-// by the first call that gets it empty, then reused and left intact (the
-// second quarter's result then gets its own buffer instead of overwriting
-// the tensor); null: a tensor of this call only.
+// the device.  share: 0 for a tensor of this call only (the second quarter's
+// result overwrites it), 1 to build it and leave it intact for a next call
+// with 2, which uses it as it is (the second quarter's result then has its own
+// buffer).
+//
+// The buffers belong to the context: a call that allocated and freed its
+// 2 GB tensor (125 functions) spent about 3 of its 8 ms on that.  Above kMoKeepBytes
+// together they are given back when the call ends (mo_release).
+constexpr size_t kMoKeepBytes = size_t(4) << 30;
+static void mo_release(pfk_ctx *ctx)
+{
+    DevBuf<double> *all[] = {&ctx->mo_E, &ctx->mo_T1, &ctx->mo_T2, &ctx->mo_C, &ctx->mo_red};
+    size_t bytes = 0;
+    for (auto *b : all) bytes += sizeof(double) * b->n;
+    if (bytes > kMoKeepBytes)
+        for (auto *b : all) b->release();
+}
 static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C2, int n2, const double *C3, int n3,
                          const double *C4, int n4, double *out, const double *eps1, const double *eps2, int mode,
-                         double *e_corr, DevBuf<double> *shared_E = nullptr)
+                         double *e_corr, int share = 0)
 {
+    struct Release {
+        pfk_ctx *c;
+        bool on;
+        ~Release() { if (on) mo_release(c); }
+    } release{ctx, share == 0};
     const int nb = ctx->nb;
     if (n1 < 1 || n2 < 1 || n3 < 1 || n4 < 1 || n1 > nb || n2 > nb || n3 > nb || n4 > nb)
         return ctx->fail(PFK_ERR_INVALID, "need 1 <= n_k <= nbasis");
@@ -1127,14 +1153,22 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
     // (n1 n2 nb^2 <= nb^4) then reuses E (or, with a shared tensor, a buffer
     // of its own), T3 (n1 n2 n3 nb <= n1 nb^3) reuses T1, and the result
     // (n1 n2 n3 n4 <= n1 n2 nb^2) reuses T2's buffer
-    DevBuf<double> own_E, T1, T2buf, dC[4];
-    DevBuf<double> &E = shared_E ? *shared_E : own_E;
-    const bool build_E = E.p == nullptr;
+    DevBuf<double> &E = ctx->mo_E, &T1 = ctx->mo_T1, &T2buf = ctx->mo_T2;
+    const bool build_E = share != 2;
     const double *hC[4] = {C1, C2, C3, C4};
     const int nk[4] = {n1, n2, n3, n4};
+    PFK_CK(ctx->mo_C.reserve(b * ((size_t)n1 + n2 + n3 + n4)));
+    double *dC[4];
+    size_t c_at = 0;
     for (int k = 0; k < 4; ++k) {
-        PFK_CK(dC[k].alloc(b * nk[k]));
-        PFK_CK(cudaMemcpyAsync(dC[k].p, hC[k], sizeof(double) * b * nk[k], cudaMemcpyHostToDevice, st));
+        // the bra's and the ket's blocks are often the same ones
+        if (k >= 2 && hC[k] == hC[k - 2] && nk[k] == nk[k - 2]) {
+            dC[k] = dC[k - 2];
+            continue;
+        }
+        dC[k] = ctx->mo_C.p + c_at;
+        c_at += b * nk[k];
+        PFK_CK(cudaMemcpyAsync(dC[k], hC[k], sizeof(double) * b * nk[k], cudaMemcpyHostToDevice, st));
     }
     cudaEvent_t ev[4] = {};
     struct EvFree {
@@ -1142,9 +1176,9 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
         ~EvFree() { for (int k = 0; k < 4; ++k) if (e[k]) cudaEventDestroy(e[k]); }
     } ev_free{ev};
     for (auto &x : ev) PFK_CK(cudaEventCreate(&x));
-    if (build_E) PFK_CK(E.alloc(b2 * b2));
-    PFK_CK(T1.alloc(b3 * n1));
-    if (shared_E) PFK_CK(T2buf.alloc(b2 * (size_t)n1 * n2));
+    PFK_CK(E.reserve(b2 * b2));
+    PFK_CK(T1.reserve(b3 * n1));
+    if (share) PFK_CK(T2buf.reserve(b2 * (size_t)n1 * n2));
     PFK_CK(cudaEventRecord(ev[0], st));
     pfk_status s = PFK_OK;
     if (build_E) {
@@ -1157,21 +1191,21 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
     auto ck = [&](cublasStatus_t r, const char *what) {
         return r == CUBLAS_STATUS_SUCCESS ? PFK_OK : ctx->fail(PFK_ERR_CUDA, std::string(what) + " failed");
     };
-    double *T2 = shared_E ? T2buf.p : E.p, *T3 = T1.p, *O = T2;
-    s = ck(cublasDgemm(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)b3, n1, nb, &one, E.p, (int)b3, dC[0].p, nb, &zero,
+    double *T2 = share ? T2buf.p : E.p, *T3 = T1.p, *O = T2;
+    s = ck(cublasDgemm(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)b3, n1, nb, &one, E.p, (int)b3, dC[0], nb, &zero,
                        T1.p, (int)b3),
            "quarter transform 1 (cublasDgemm)");
     if (s != PFK_OK) return s;
     s = ck(cublasDgemmStridedBatched(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)b2, n2, nb, &one, T1.p, (int)b2,
-                                     (long long)b3, dC[1].p, nb, 0, &zero, T2, (int)b2, (long long)b2 * n2, n1),
+                                     (long long)b3, dC[1], nb, 0, &zero, T2, (int)b2, (long long)b2 * n2, n1),
            "quarter transform 2 (cublasDgemmStridedBatched)");
     if (s != PFK_OK) return s;
     s = ck(cublasDgemmStridedBatched(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, nb, n3, nb, &one, T2, nb, (long long)b2,
-                                     dC[2].p, nb, 0, &zero, T3, nb, (long long)b * n3, n1 * n2),
+                                     dC[2], nb, 0, &zero, T3, nb, (long long)b * n3, n1 * n2),
            "quarter transform 3 (cublasDgemmStridedBatched)");
     if (s != PFK_OK) return s;
     const size_t no = (size_t)n1 * n2 * n3 * n4;
-    s = ck(cublasDgemm(ctx->blas, CUBLAS_OP_T, CUBLAS_OP_N, n4, n1 * n2 * n3, nb, &one, dC[3].p, nb, T3, nb, &zero,
+    s = ck(cublasDgemm(ctx->blas, CUBLAS_OP_T, CUBLAS_OP_N, n4, n1 * n2 * n3, nb, &one, dC[3], nb, T3, nb, &zero,
                        O, n4),
            "quarter transform 4 (cublasDgemm)");
     if (s != PFK_OK) return s;
@@ -1180,15 +1214,14 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
         int nsm = 0;
         PFK_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
         const int grid = 8 * std::max(nsm, 1);   // 8 blocks of 256 per SM
-        DevBuf<double> d_eps, d_sum;
-        PFK_CK(d_eps.alloc(2 * b));
-        PFK_CK(d_sum.alloc(grid));
-        PFK_CK(cudaMemcpyAsync(d_eps.p, eps1, sizeof(double) * nb, cudaMemcpyHostToDevice, st));
-        PFK_CK(cudaMemcpyAsync(d_eps.p + nb, eps2, sizeof(double) * nb, cudaMemcpyHostToDevice, st));
-        mp2_sum_kernel<<<grid, 256, 0, st>>>(O, d_eps.p, d_eps.p + nb, n1, n2, n3, n4, mode, d_sum.p);
+        PFK_CK(ctx->mo_red.reserve(2 * b + grid));
+        double *d_eps = ctx->mo_red.p, *d_sum = d_eps + 2 * b;
+        PFK_CK(cudaMemcpyAsync(d_eps, eps1, sizeof(double) * nb, cudaMemcpyHostToDevice, st));
+        PFK_CK(cudaMemcpyAsync(d_eps + nb, eps2, sizeof(double) * nb, cudaMemcpyHostToDevice, st));
+        mp2_sum_kernel<<<grid, 256, 0, st>>>(O, d_eps, d_eps + nb, n1, n2, n3, n4, mode, d_sum);
         PFK_CK(cudaGetLastError());
         std::vector<double> part(grid);
-        PFK_CK(cudaMemcpyAsync(part.data(), d_sum.p, sizeof(double) * grid, cudaMemcpyDeviceToHost, st));
+        PFK_CK(cudaMemcpyAsync(part.data(), d_sum, sizeof(double) * grid, cudaMemcpyDeviceToHost, st));
         PFK_CK(cudaEventRecord(ev[3], st));
         PFK_CK(cudaStreamSynchronize(st));
         double tot = 0.0;
@@ -1263,13 +1296,13 @@ pfk_status pfk_ump2_energy(pfk_ctx *ctx, const double *Ca, const double *eps_a, 
         return ctx->fail(PFK_ERR_INVALID, "no occupied or virtual orbitals in a spin channel");
     const double *Cav = Ca + (size_t)nb * n_alpha, *Cbv = Cb + (size_t)nb * n_beta;
     double e_aa = 0.0, e_bb = 0.0, e_ab = 0.0;
-    DevBuf<double> E;   // the AO tensor, built by the first transform and shared by all three
-    pfk_status s =
-        mo_run(ctx, Ca, n_alpha, Cav, nva, Ca, n_alpha, Cav, nva, nullptr, eps_a, eps_a, kMp2Same, &e_aa, &E);
+    // the first transform builds the AO tensor, all three use it
+    pfk_status s = mo_run(ctx, Ca, n_alpha, Cav, nva, Ca, n_alpha, Cav, nva, nullptr, eps_a, eps_a, kMp2Same, &e_aa, 1);
     if (s == PFK_OK)
-        s = mo_run(ctx, Cb, n_beta, Cbv, nvb, Cb, n_beta, Cbv, nvb, nullptr, eps_b, eps_b, kMp2Same, &e_bb, &E);
+        s = mo_run(ctx, Cb, n_beta, Cbv, nvb, Cb, n_beta, Cbv, nvb, nullptr, eps_b, eps_b, kMp2Same, &e_bb, 2);
     if (s == PFK_OK)
-        s = mo_run(ctx, Ca, n_alpha, Cav, nva, Cb, n_beta, Cbv, nvb, nullptr, eps_a, eps_b, kMp2Opp, &e_ab, &E);
+        s = mo_run(ctx, Ca, n_alpha, Cav, nva, Cb, n_beta, Cbv, nvb, nullptr, eps_a, eps_b, kMp2Opp, &e_ab, 2);
+    mo_release(ctx);
     if (s == PFK_OK) *e_corr = e_aa + e_bb + e_ab;
     return s;
 }

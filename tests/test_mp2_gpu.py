@@ -114,3 +114,25 @@ def test_uhf_and_ump2_of_the_water_cation():
     assert abs(e_dev - e_corr) < 1e-12
     assert abs(r["energy"] - c["energy"]) < 1e-8
     assert abs(r["energy"] + e_corr - c["mp2_energy"]) < 1e-6
+
+
+def test_kept_buffers_do_not_leak_between_calls():
+    """The transform's buffers stay with the context.  Calls of growing and
+    shrinking blocks, UMP2 (whose tensor outlives a transform) and RMP2 in
+    turn give the bits of a fresh engine's first call."""
+    P = pfk()
+    mol, shells = P.shells_for(WATER, "6-31g**", basis_library())
+    nb = P.FockEngine(shells).nbasis
+    rng = np.random.default_rng(3)
+    C, C2 = (np.linalg.qr(rng.normal(size=(nb, nb)))[0] for _ in range(2))
+    eps = np.concatenate([-1.0 - rng.uniform(size=5), 0.5 + rng.uniform(size=nb - 5)])
+    calls = [lambda e: e.rmp2_energy(C, eps, 5), lambda e: e.mo_transform(C[:, :2], C, C2[:, :3], C2),
+             lambda e: e.ump2_energy(C, eps, C2, eps, 5, 4), lambda e: e.mo_transform(C, C, C, C),
+             lambda e: e.mo_transform(C[:, :1], C2[:, :1], C[:, :1], C[:, 3:4]),
+             lambda e: e.ump2_energy(C2, eps, C, eps, 3, 5), lambda e: e.rmp2_energy(C2, eps, 5)]
+    kept = P.FockEngine(shells)
+    for call in calls + calls[::-1]:
+        fresh = P.FockEngine(shells)
+        assert np.array_equal(call(kept), call(fresh))
+        fresh.close()
+    kept.close()
