@@ -13,16 +13,18 @@
 //   db_l = column sums of dZ_l;  dH_{l-1} = bf16(dZ_l) W_l^T;
 //   dZ_{l-1} = dH_{l-1} * SiLU'(Z_{l-1}).
 //
-// A training step is 2L + 2 launches for L layers: the input conversion, L
+// Networks up to 256 wide run a training step in three launches: everything
+// up to dZ_1 (fused_kernel), the weight gradients of every layer, and the
+// update.  Wider ones take 2L + 2 for L layers: the input conversion, L
 // forward products (the last one also forms dZ_L and the loss), L - 1
-// products for dH (their epilogue applies SiLU' and leaves dZ), one launch
-// for the weight gradients of every layer, and the update.  Each product
+// products for dH (their epilogue applies SiLU' and leaves dZ), and the same
+// last two.  Each product
 // leaves its result in both orders (rows of the batch, and transposed), so
 // every product reads both operands as rows of K by 16-byte copies.  On the
-// 112-256-256-232 network (one B200): 2048 rows, a step 98 us against 1675 us
+// 112-256-256-232 network (one B200): 2048 rows, a step 89 us against 1675 us
 // before (products staged by 2-byte gathers, bias sums by one thread per
 // column, weight gradients on 8 CTAs, two host synchronisations); forward of
-// 8192 rows 54 us against 250 us (both with the host call).
+// 8192 rows 47 us against 250 us (both with the host call).
 // The reference has no counterpart: it is the learned part of the guess
 // hook (scf.cpp:206-240 selects the guess; a learned density enters the SCF
 // as a ReadDensity guess does, scf.cpp:213-216).
@@ -46,7 +48,7 @@ thread_local std::string g_mlp_error;
 // row start 16-byte aligned), FP32 accumulation in tensor memory, and one of
 // the epilogues below.
 //
-// One CTA of 256 threads per 128 x 64 tile.  K goes in rounds of 64 through a
+// One CTA of 512 threads per 128 x 64 tile.  K goes in rounds of 64 through a
 // ring of TC_STAGES shared-memory stages: cp.async copies 16-byte segments of
 // later rounds while the tensor cores work on the current one (the products
 // here are 2 to 64 rounds deep, so a tile's time is the latency of its loads;
@@ -57,22 +59,22 @@ thread_local std::string g_mlp_error;
 // contiguous bytes in shared memory.  One thread issues four tcgen05.mma
 // (M 128, N 64, K 16) per round and commits them to the stage's mbarrier,
 // which every thread waits on before it refills the stage.  The epilogue reads
-// the accumulator back with tcgen05.ld, warps w and w + 4 taking rows 32w ..
-// 32w+31 (the tensor-memory lanes a warp may access) and 32 columns each: a
-// tile's time is mostly this epilogue (64 values a thread on four warps took
-// 17 us of kernel time for 8192 x 256; with eight warps and overlapped
-// launches the three layers' forward pass went from 73 to 54 us, a training
-// step of 2048 rows from 135 to 98 us).  Waits are bounded (2 s of
-// %globaltimer); a wait that runs out sets *err, the CTA stops issuing, waits
+// the accumulator back with tcgen05.ld, warps w, w + 4, w + 8 and w + 12 taking
+// rows 32w .. 32w+31 (the tensor-memory lanes a warp may access) and 16 columns
+// each: a tile's time is mostly this epilogue, a latency-bound chain per
+// thread, so it is spread over 16 warps (with 4 warps the three layers'
+// forward pass of 8192 rows took 73 us, with 8 and overlapped launches 54).
+// Waits are bounded (2 s of
+// SM cycles); a wait that runs out sets *err, the CTA stops issuing, waits
 // (bounded again) for what is in flight and frees its columns.
 // ---------------------------------------------------------------------------
-constexpr int TC_M = 128, TC_N = 64, TC_K = 64, TC_STAGES = 4, TC_THREADS = 256;
+constexpr int TC_M = 128, TC_N = 64, TC_K = 64, TC_STAGES = 4, TC_THREADS = 512;
 constexpr int TC_A_BYTES = TC_M * TC_K * 2, TC_B_BYTES = TC_N * TC_K * 2, TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
 // 96 KB of stages: two CTAs share an SM, and their 2 x 64 accumulator columns
 // fit its 512 tensor-memory columns
 constexpr int TC_SMEM = TC_STAGES * TC_STAGE_BYTES;
 constexpr uint32_t TC_TMEM_COLS = 64;
-constexpr unsigned long long TC_WAIT_NS = 2000000000ull;
+constexpr long long TC_WAIT_CYCLES = 4000000000ll;   // 2 s at 1.965 GHz
 // instruction descriptor (kind::f16): D F32 (bits 4-5 = 1), A and B BF16
 // (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits
 // 17-22, M >> 4 at bits 24-28
@@ -100,18 +102,11 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr)
            ((uint64_t)((TC_K / 8 * 128u) >> 4) << 32) | (1ull << 46);
 }
 
-__device__ __forceinline__ unsigned long long global_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // Waits until phase `parity` of the mbarrier at bar completes; false after
-// TC_WAIT_NS without completion.
+// TC_WAIT_CYCLES SM cycles without completion.
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
 {
-    const unsigned long long t0 = global_ns();
+    const long long t0 = clock64();
     while (true) {
         uint32_t done;
         asm volatile("{\n\t.reg .pred p;\n\t"
@@ -121,7 +116,7 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity)
                      : "r"(bar), "r"(parity)
                      : "memory");
         if (done) return true;
-        if (global_ns() - t0 > TC_WAIT_NS) return false;
+        if (clock64() - t0 > TC_WAIT_CYCLES) return false;
     }
 }
 
@@ -202,7 +197,7 @@ struct EpiArgs {
     __nv_bfloat16 *R, *RT;    // result rows (stride N; null: not wanted) and transposed (row stride ldt; null: not wanted)
     long long ldt;
     float *colpart;           // column sums per row tile: [row tile][N]
-    double *losspart;         // per CTA
+    double *losspart;         // per tile
     float scale;
     bool vec;                 // T or Y is 16-byte aligned
 };
@@ -235,6 +230,129 @@ __device__ __forceinline__ float colsum16(const float (&v)[16], int lane)
     return d + __shfl_xor_sync(0xffffffffu, d, 1);
 }
 
+// The epilogue of the tile at (m0, n0) of an M x N result, from the
+// accumulator at tmem (zero when !have).  bias: the tile's columns; colw and
+// lossw: shared scratch; part: the tile's FP32 destination (kEpiPart).
+template <int EPI>
+__device__ __forceinline__ void tile_epilogue(uint32_t tmem, bool have, int M, int N, int m0, int n0, const EpiArgs &e,
+                                              const float *bias, float (*colw)[TC_N], double *lossw, float *part)
+{
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int quad = warp & 3, m = m0 + quad * 32 + lane;
+    constexpr int kCols = TC_N / (TC_THREADS / 128);   // per warp
+    static_assert(kCols % 16 == 0, "a warp reads 16 columns at a time");
+    const int c0 = (warp >> 2) * kCols;
+    double loss = 0.0;
+#pragma unroll 1
+    for (int c = c0; c < c0 + kCols; c += 16) {
+        uint32_t v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0u;
+        if (have) {
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+                         "%11, %12, %13, %14, %15}, [%16];"
+                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                           "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                           "=r"(v[14]), "=r"(v[15])
+                         : "r"(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        }
+        if constexpr (EPI == kEpiPart) {
+            float4 *o = reinterpret_cast<float4 *>(part + (size_t)(quad * 32 + lane) * TC_N + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                o[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                   __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+        } else {
+            // widths are multiples of 8: each half of the 16 columns is inside or outside
+            float x[16];
+            __nv_bfloat16 h[16];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int n = n0 + c + 8 * half;
+                const bool in = m < M && n < N;
+                const size_t at = (size_t)m * N + n;
+                float t[8] = {};
+                if (EPI == kEpiLoss && in) {
+                    if (e.vec) {
+                        *reinterpret_cast<float4 *>(t) = __ldg(reinterpret_cast<const float4 *>(e.T + at));
+                        *reinterpret_cast<float4 *>(t + 4) = __ldg(reinterpret_cast<const float4 *>(e.T + at + 4));
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) t[i] = __ldg(e.T + at + i);
+                    }
+                }
+                if (EPI == kEpiBack && in) {
+                    *reinterpret_cast<float4 *>(t) = *reinterpret_cast<const float4 *>(e.Z + at);
+                    *reinterpret_cast<float4 *>(t + 4) = *reinterpret_cast<const float4 *>(e.Z + at + 4);
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int k = 8 * half + i;
+                    float a = __uint_as_float(v[k]);
+                    if (EPI != kEpiBack) a += bias[c + k];
+                    if (EPI == kEpiLoss) {
+                        const float r = a - t[i];
+                        if (in) loss += (double)r * r * e.scale;
+                        a = 2.0f * r * e.scale;
+                    }
+                    if (EPI == kEpiBack) a *= silu_grad(t[i]);
+                    x[k] = in ? a : 0.0f;
+                    if (EPI == kEpiHidden) h[k] = in ? __float2bfloat16(silu(a)) : __float2bfloat16(0.0f);
+                    if (EPI == kEpiLoss || EPI == kEpiBack) h[k] = __float2bfloat16(x[k]);
+                }
+                if ((EPI == kEpiHidden && e.Z) || EPI == kEpiOut) {
+                    float *o = EPI == kEpiOut ? e.Y : e.Z;
+                    if (in) {
+                        if (EPI == kEpiHidden || e.vec) {
+                            *reinterpret_cast<float4 *>(o + at) = *reinterpret_cast<const float4 *>(x + 8 * half);
+                            *reinterpret_cast<float4 *>(o + at + 4) = *reinterpret_cast<const float4 *>(x + 8 * half + 4);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) o[at + i] = x[8 * half + i];
+                        }
+                    }
+                }
+                if (EPI != kEpiOut) {
+                    if (e.R && in) {
+                        uint4 w;
+                        w.x = pack2(h[8 * half], h[8 * half + 1]);
+                        w.y = pack2(h[8 * half + 2], h[8 * half + 3]);
+                        w.z = pack2(h[8 * half + 4], h[8 * half + 5]);
+                        w.w = pack2(h[8 * half + 6], h[8 * half + 7]);
+                        *reinterpret_cast<uint4 *>(e.R + at) = w;
+                    }
+                    // transposed, zero up to the next multiple of 8 rows: the
+                    // weight-gradient products read whole 16-byte segments
+                    if (e.RT && n < N && m < ((M + 7) & ~7)) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) e.RT[(size_t)(n + i) * e.ldt + m] = h[8 * half + i];
+                    }
+                }
+            }
+            if constexpr (EPI == kEpiLoss || EPI == kEpiBack) {
+                const float s = colsum16(x, lane);
+                if (!(lane & 1)) colw[quad][c + (lane >> 1)] = s;
+            }
+        }
+    }
+    if constexpr (EPI == kEpiLoss || EPI == kEpiBack) {
+        if (EPI == kEpiLoss) {
+            for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+            if (lane == 0) lossw[warp] = loss;
+        }
+        __syncthreads();
+        if (tid < TC_N && n0 + tid < N)
+            e.colpart[(size_t)(m0 / TC_M) * N + n0 + tid] =
+                (colw[0][tid] + colw[1][tid]) + (colw[2][tid] + colw[3][tid]);
+        if (EPI == kEpiLoss && tid == 0) {
+            double sum = 0.0;
+            for (int w = 0; w < TC_THREADS / 32; ++w) sum += lossw[w];
+            e.losspart[m0 / TC_M * ((N + TC_N - 1) / TC_N) + n0 / TC_N] = sum;
+        }
+    }
+}
+
 // The whole tile: K loop and epilogue.  part: the tile's FP32 destination (kEpiPart).
 template <int EPI>
 __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, const __nv_bfloat16 *__restrict__ A,
@@ -247,7 +365,7 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
     __shared__ float colw[4][TC_N];
     __shared__ double lossw[TC_THREADS / 32];
     __shared__ float bias[TC_N];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t s0 = smem_u32(tc_tiles), sbar = smem_u32(mbar);
     const int nk = kend > kbeg ? (kend - kbeg + TC_K - 1) / TC_K : 0;
     auto load = [&](int kt) {
@@ -332,115 +450,7 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
             __threadfence_system();
         }
     } else {
-        const int quad = warp & 3, m = m0 + quad * 32 + lane;
-        const int c0 = (warp >> 2) * (TC_N / 2);
-        double loss = 0.0;
-#pragma unroll 1
-        for (int c = c0; c < c0 + TC_N / 2; c += 16) {
-            uint32_t v[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0u;
-            if (nk > 0) {
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
-                             "%11, %12, %13, %14, %15}, [%16];"
-                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                               "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                               "=r"(v[14]), "=r"(v[15])
-                             : "r"(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            }
-            if constexpr (EPI == kEpiPart) {
-                float4 *o = reinterpret_cast<float4 *>(part + (size_t)(quad * 32 + lane) * TC_N + c);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    o[i] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                       __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-            } else {
-                // widths are multiples of 8: each half of the 16 columns is inside or outside
-                float x[16];
-                __nv_bfloat16 h[16];
-    #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int n = n0 + c + 8 * half;
-                    const bool in = m < M && n < N;
-                    const size_t at = (size_t)m * N + n;
-                    float t[8] = {};
-                    if (EPI == kEpiLoss && in) {
-                        if (e.vec) {
-                            *reinterpret_cast<float4 *>(t) = __ldg(reinterpret_cast<const float4 *>(e.T + at));
-                            *reinterpret_cast<float4 *>(t + 4) = __ldg(reinterpret_cast<const float4 *>(e.T + at + 4));
-                        } else {
-    #pragma unroll
-                            for (int i = 0; i < 8; ++i) t[i] = __ldg(e.T + at + i);
-                        }
-                    }
-                    if (EPI == kEpiBack && in) {
-                        *reinterpret_cast<float4 *>(t) = *reinterpret_cast<const float4 *>(e.Z + at);
-                        *reinterpret_cast<float4 *>(t + 4) = *reinterpret_cast<const float4 *>(e.Z + at + 4);
-                    }
-    #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int k = 8 * half + i;
-                        float a = __uint_as_float(v[k]);
-                        if (EPI != kEpiBack) a += bias[c + k];
-                        if (EPI == kEpiLoss) {
-                            const float r = a - t[i];
-                            if (in) loss += (double)r * r * e.scale;
-                            a = 2.0f * r * e.scale;
-                        }
-                        if (EPI == kEpiBack) a *= silu_grad(t[i]);
-                        x[k] = in ? a : 0.0f;
-                        if (EPI == kEpiHidden) h[k] = in ? __float2bfloat16(silu(a)) : __float2bfloat16(0.0f);
-                        if (EPI == kEpiLoss || EPI == kEpiBack) h[k] = __float2bfloat16(x[k]);
-                    }
-                    if ((EPI == kEpiHidden && e.Z) || EPI == kEpiOut) {
-                        float *o = EPI == kEpiOut ? e.Y : e.Z;
-                        if (in) {
-                            if (EPI == kEpiHidden || e.vec) {
-                                *reinterpret_cast<float4 *>(o + at) = *reinterpret_cast<const float4 *>(x + 8 * half);
-                                *reinterpret_cast<float4 *>(o + at + 4) = *reinterpret_cast<const float4 *>(x + 8 * half + 4);
-                            } else {
-    #pragma unroll
-                                for (int i = 0; i < 8; ++i) o[at + i] = x[8 * half + i];
-                            }
-                        }
-                    }
-                    if (EPI != kEpiOut) {
-                        if (e.R && in) {
-                            uint4 w;
-                            w.x = pack2(h[8 * half], h[8 * half + 1]);
-                            w.y = pack2(h[8 * half + 2], h[8 * half + 3]);
-                            w.z = pack2(h[8 * half + 4], h[8 * half + 5]);
-                            w.w = pack2(h[8 * half + 6], h[8 * half + 7]);
-                            *reinterpret_cast<uint4 *>(e.R + at) = w;
-                        }
-                        // transposed, zero up to the next multiple of 8 rows: the
-                        // weight-gradient products read whole 16-byte segments
-                        if (e.RT && n < N && m < ((M + 7) & ~7)) {
-    #pragma unroll
-                            for (int i = 0; i < 8; ++i) e.RT[(size_t)(n + i) * e.ldt + m] = h[8 * half + i];
-                        }
-                    }
-                }
-                if constexpr (EPI == kEpiLoss || EPI == kEpiBack) {
-                    const float s = colsum16(x, lane);
-                    if (!(lane & 1)) colw[quad][c + (lane >> 1)] = s;
-                }
-            }
-        }
-        if constexpr (EPI == kEpiLoss || EPI == kEpiBack) {
-            if (EPI == kEpiLoss) {
-                for (int o = 16; o; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-                if (lane == 0) lossw[warp] = loss;
-            }
-            __syncthreads();
-            if (tid < TC_N && n0 + tid < N)
-                e.colpart[(size_t)(m0 / TC_M) * N + n0 + tid] =
-                    (colw[0][tid] + colw[1][tid]) + (colw[2][tid] + colw[3][tid]);
-            if (EPI == kEpiLoss && tid == 0)
-                e.losspart[blockIdx.y * gridDim.x + blockIdx.x] =
-                    ((lossw[0] + lossw[1]) + (lossw[2] + lossw[3])) + ((lossw[4] + lossw[5]) + (lossw[6] + lossw[7]));
-        }
+        tile_epilogue<EPI>(tmem, nk > 0, M, N, m0, n0, e, bias, colw, lossw, part);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -449,7 +459,7 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int kbeg, int kend, cons
 }
 
 template <int EPI>
-__global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
+__global__ void __launch_bounds__(TC_THREADS, 2) gemm_tc_kernel(int M, int N, int K, const __nv_bfloat16 *__restrict__ A,
                                                       const __nv_bfloat16 *__restrict__ B, EpiArgs e, int *err)
 {
     gemm_tile<EPI>(M, N, 0, K, A, K, B, K, blockIdx.y * TC_M, blockIdx.x * TC_N, e, nullptr, err);
@@ -468,7 +478,7 @@ struct Layers {
 // 128 x 64 tile of dW_l = H^T G over its share of the batch.  A layer alone is
 // 4 to 8 tiles of 2048 rows on a 148-SM chip; all layers' tiles times the
 // splits fill it, and the update adds the parts in a fixed order.
-__global__ void __launch_bounds__(TC_THREADS) gemm_dw_kernel(Layers L, int n, long long ldt, float *part, int *err)
+__global__ void __launch_bounds__(TC_THREADS, 2) gemm_dw_kernel(Layers L, int n, long long ldt, float *part, int *err)
 {
     int l = 0;
     while (l + 1 < L.nl && (int)blockIdx.x >= L.tile0[l + 1]) ++l;
@@ -545,8 +555,10 @@ __global__ void __launch_bounds__(256) update_kernel(Layers L, const float *__re
             c = (int)(i % dout);
             const float *q = part + (size_t)(L.tile0[l] + (r / TC_M) * tn + c / TC_N) * (TC_M * TC_N) +
                              (r % TC_M) * TC_N + c % TC_N;
+#pragma unroll 8
             for (int s = 0; s < L.splits; ++s) g += q[(size_t)s * L.tiles * (TC_M * TC_N)];
         } else {
+#pragma unroll 8
             for (int t = 0; t < row_tiles; ++t) g += colpart[L.col_off[l] + (size_t)t * dout + (i - nw)];
         }
         const long long at = i < nw ? L.w_off[l] + i : L.b_off[l] + (i - nw);
@@ -579,6 +591,201 @@ __global__ void __launch_bounds__(256) update_kernel(Layers L, const float *__re
 }
 
 unsigned blocks_for(long long n) { return (unsigned)std::min<long long>((n + 255) / 256, 148 * 16); }
+
+// All layers of a network whose widths are at most kFuseWidth in one kernel: a
+// cluster of four CTAs takes 128 rows of the batch through the forward pass
+// (with TRAIN also the loss and the backward pass to dZ_1), CTA c computing
+// columns 64c .. 64c + 63 of every layer.  A layer of 128 rows is a microsecond
+// of loads and products and two of epilogue; as a launch of its own it took 8
+// to 10.  Between layers the CTAs exchange their columns through global
+// memory (L2) and a cluster barrier; the next layer's weights are fetched
+// while the epilogue runs.  The layer's whole K (at most four rounds) sits in
+// the four stages.  Every CTA passes every barrier, also one whose wait ran out.
+// 112-256-256-232, 2048 rows: a step 98 -> 89 us, forward of 8192 rows 54 ->
+// 47 us (with 16-warp epilogues and waits that poll the SM clock instead of
+// the global timer).
+constexpr int kFuseWidth = 256, kFuseCtas = 4;
+static_assert(kFuseWidth <= TC_STAGES * TC_K && kFuseWidth <= kFuseCtas * TC_N, "a layer must fit the stages and the cluster");
+
+struct FusedArgs {
+    int n, nl;
+    int dims[kMaxLayers + 1];
+    const float *X, *T;
+    float *Y;
+    const __nv_bfloat16 *wt[kMaxLayers], *wb[kMaxLayers];
+    const float *bias[kMaxLayers];
+    float *Z[kMaxLayers];
+    __nv_bfloat16 *H[kMaxLayers], *HT[kMaxLayers], *G[kMaxLayers], *GT[kMaxLayers];
+    float *colpart[kMaxLayers];
+    double *losspart;
+    long long ldt;
+    float scale;
+    bool xvec, ovec;          // X, and T or Y, are 16-byte aligned
+};
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(TC_THREADS, TRAIN ? 1 : 2) __cluster_dims__(kFuseCtas, 1, 1) fused_kernel(FusedArgs a, int *err)
+{
+    extern __shared__ __align__(128) unsigned char tc_tiles[];
+    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ float colw[4][TC_N];
+    __shared__ double lossw[TC_THREADS / 32];
+    __shared__ float bias[TC_N];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t s0 = smem_u32(tc_tiles), sbar = smem_u32(&mbar);
+    const int m0 = blockIdx.y * TC_M, n0 = blockIdx.x * TC_N, L = a.nl;
+    const int steps = TRAIN ? 2 * L - 1 : L;   // L forward layers, then dH of layers L - 1 .. 1
+
+    // step i: forward of layer i, or (i >= L) dH of layer 2 L - 1 - i
+    auto layer = [&](int i) { return i < L ? i : 2 * L - 1 - i; };
+    auto width = [&](int i) { return i < L ? a.dims[i + 1] : a.dims[layer(i)]; };
+    auto depth = [&](int i) { return i < L ? a.dims[i] : a.dims[layer(i) + 1]; };
+    auto load_b = [&](int i) {
+        const int K = depth(i), N = width(i);
+        if (n0 >= N) return;
+        const __nv_bfloat16 *B = i < L ? a.wt[i] : a.wb[layer(i)];
+        for (int k = 0; k < K; k += TC_K)
+            tc_load<TC_N>(s0 + k / TC_K * TC_STAGE_BYTES + TC_A_BYTES, B, K, n0, N, k, K);
+    };
+    load_b(0);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(TC_TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    grid_launch_next();
+    // the network's input, rounded to BF16 in place; CTA c also leaves every
+    // fourth group of 8 columns transposed for the weight gradients
+    {
+        const int d0 = a.dims[0], rounds = (d0 + TC_K - 1) / TC_K;
+        for (int u = warp; u < rounds * (TC_M / 4); u += TC_THREADS / 32) {
+            const int kt = u / (TC_M / 4), v = u % (TC_M / 4);
+            const int r = (v >> 1) * 8 + (lane & 7), kc = (v & 1) * 4 + (lane >> 3);
+            const int gr = m0 + r, gk = kt * TC_K + kc * 8;
+            const bool ok = gr < a.n && gk < d0;
+            float x[8] = {};
+            if (ok) {
+                const float *src = a.X + (size_t)gr * d0 + gk;
+                if (a.xvec) {
+                    *reinterpret_cast<float4 *>(x) = __ldg(reinterpret_cast<const float4 *>(src));
+                    *reinterpret_cast<float4 *>(x + 4) = __ldg(reinterpret_cast<const float4 *>(src) + 1);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) x[i] = __ldg(src + i);
+                }
+            }
+            __nv_bfloat16 h[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) h[i] = __float2bfloat16(x[i]);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(s0 + kt * TC_STAGE_BYTES + tc_off(r, kc)),
+                         "r"(pack2(h[0], h[1])), "r"(pack2(h[2], h[3])), "r"(pack2(h[4], h[5])), "r"(pack2(h[6], h[7]))
+                         : "memory");
+            if (TRAIN && (gk >> 3) % kFuseCtas == (int)blockIdx.x && gk < d0 && gr < ((a.n + 7) & ~7)) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) a.HT[0][(size_t)(gk + i) * a.ldt + gr] = h[i];
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+
+    bool failed = false;
+    uint32_t parity = 0;
+    for (int i = 0; i < steps; ++i) {
+        const int l = layer(i), K = depth(i), N = width(i);
+        const bool mine = n0 < N && !failed;   // uniform over the CTA
+        const __nv_bfloat16 *A = i < L ? a.H[l] : a.G[l];
+        if (mine) {
+            if (i > 0)
+                for (int k = 0; k < K; k += TC_K)
+                    tc_load<TC_M>(s0 + k / TC_K * TC_STAGE_BYTES, A, K, m0, a.n, k, K);
+            if (i < L && tid < TC_N) bias[tid] = n0 + tid < N ? a.bias[l][n0 + tid] : 0.0f;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // staged tiles visible to the tensor cores
+        __syncthreads();
+        if (mine) {
+            if (tid == 0) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int k = 0; k < K; k += 16) {
+                    const uint32_t st = s0 + k / TC_K * TC_STAGE_BYTES + k % TC_K / 16 * 256;
+                    const uint64_t da = tc_desc(st), db = tc_desc(st + TC_A_BYTES);
+                    const uint32_t accumulate = k > 0 ? 1u : 0u;
+                    asm volatile("{\n\t.reg .pred p;\n\t"
+                                 "setp.ne.b32 p, %4, 0;\n\t"
+                                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+                                 "l"(da), "l"(db), "r"(TC_IDESC), "r"(accumulate)
+                                 : "memory");
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sbar)
+                             : "memory");
+            }
+            const bool ok = tc_wait(sbar, parity);
+            if (__syncthreads_or(!ok)) {
+                failed = true;
+                tc_wait(sbar, parity);   // once more (bounded) before the tiles and columns are used again
+                if (tid == 0) {
+                    *(volatile int *)err = 1;
+                    __threadfence_system();
+                }
+            }
+            parity ^= 1u;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        if (i + 1 < steps && !failed) load_b(i + 1);   // this layer's weights are used up
+        if (mine && !failed) {
+            EpiArgs e{};
+            e.ldt = a.ldt;
+            if (i + 1 < L) {
+                e.Z = TRAIN ? a.Z[l] : nullptr;
+                e.R = a.H[l + 1];
+                e.RT = TRAIN ? a.HT[l + 1] : nullptr;
+                tile_epilogue<kEpiHidden>(tmem, true, a.n, N, m0, n0, e, bias, colw, lossw, nullptr);
+            } else if (i + 1 == L) {
+                if constexpr (TRAIN) {
+                    e.T = a.T;
+                    e.vec = a.ovec;
+                    e.R = L > 1 ? a.G[l] : nullptr;
+                    e.RT = a.GT[l];
+                    e.colpart = a.colpart[l];
+                    e.losspart = a.losspart;
+                    e.scale = a.scale;
+                    tile_epilogue<kEpiLoss>(tmem, true, a.n, N, m0, n0, e, bias, colw, lossw, nullptr);
+                } else {
+                    e.Y = a.Y;
+                    e.vec = a.ovec;
+                    tile_epilogue<kEpiOut>(tmem, true, a.n, N, m0, n0, e, bias, colw, lossw, nullptr);
+                }
+            } else if constexpr (TRAIN) {
+                e.Z = a.Z[l - 1];
+                e.R = l > 1 ? a.G[l - 1] : nullptr;
+                e.RT = a.GT[l - 1];
+                e.colpart = a.colpart[l - 1];
+                tile_epilogue<kEpiBack>(tmem, true, a.n, N, m0, n0, e, bias, colw, lossw, nullptr);
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (i + 1 < steps) cluster_barrier();   // the layer's columns of all four CTAs are in memory
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS) : "memory");
+}
 
 // What the kernels leave for the host, in page-locked memory mapped into the
 // device's address space: read after the stream is synchronised, no copy.
@@ -680,9 +887,51 @@ void gemm(pfk_mlp *m, int M, int N, int K, const __nv_bfloat16 *A, const __nv_bf
     launch_after(gemm_tc_kernel<EPI>, grid, TC_THREADS, TC_SMEM, st, M, N, K, A, B, e, &m->d_slot->tc_err);
 }
 
+bool fusable(const pfk_mlp *m)
+{
+    for (int d : m->dims)
+        if (d > kFuseWidth) return false;
+    return true;
+}
+
+// The fused kernel over n rows: forward to Y, or, with T, everything up to the
+// weight gradients.
+void fused(pfk_mlp *m, int n, const float *X, float *Y, const float *T, cudaStream_t st)
+{
+    FusedArgs a{};
+    a.n = n;
+    a.nl = m->nl;
+    a.X = X;
+    a.T = T;
+    a.Y = Y;
+    long long col = 0;
+    for (int l = 0; l < m->nl; ++l) {
+        a.wt[l] = m->wt + m->w_off[l];
+        a.wb[l] = m->wb + m->w_off[l];
+        a.bias[l] = m->p + m->b_off[l];
+        a.Z[l] = m->Z[l];
+        a.H[l] = m->H[l];
+        a.HT[l] = m->HT[l];
+        a.G[l] = m->G[l];
+        a.GT[l] = m->GT[l];
+        a.colpart[l] = m->colpart + col;
+        col += (long long)row_tiles(m->max_batch) * m->dims[l + 1];
+    }
+    for (int l = 0; l <= m->nl; ++l) a.dims[l] = m->dims[l];
+    a.losspart = m->losspart;
+    a.ldt = m->ldt;
+    a.scale = 1.0f / (float)((long long)n * m->dims[m->nl]);
+    a.xvec = aligned16(X);
+    a.ovec = aligned16(T ? (const void *)T : (const void *)Y);
+    const dim3 grid(kFuseCtas, row_tiles(n));
+    if (T) fused_kernel<true><<<grid, TC_THREADS, TC_SMEM, st>>>(a, &m->d_slot->tc_err);
+    else fused_kernel<false><<<grid, TC_THREADS, TC_SMEM, st>>>(a, &m->d_slot->tc_err);
+}
+
 // Forward pass of n rows of X: to Y, or, with T, to dZ of the last layer and the loss.
 void forward(pfk_mlp *m, int n, const float *X, float *Y, const float *T, cudaStream_t st)
 {
+    if (fusable(m)) return fused(m, n, X, Y, T, st);
     const bool train = T != nullptr;
     const int d0 = m->dims[0];
     dim3 gi((d0 + 31) / 32, (n + 31) / 32);
@@ -720,7 +969,7 @@ void forward(pfk_mlp *m, int n, const float *X, float *Y, const float *T, cudaSt
 // Gradient parts of the mean squared error after forward(..., T).
 void backward(pfk_mlp *m, int n, const Layers &L, cudaStream_t st)
 {
-    for (int l = m->nl - 1; l > 0; --l) {
+    for (int l = fusable(m) ? 0 : m->nl - 1; l > 0; --l) {
         // dH_{l-1} = G W_l^T (n x din); dZ_{l-1} = dH * SiLU'(Z_{l-1})
         EpiArgs e{};
         e.ldt = m->ldt;
@@ -832,7 +1081,8 @@ pfk_status pfk_mlp_create(int nlayers, const int *dims, int max_batch, int devic
     // the product kernels' shared-memory limits on this device
     for (const void *k : {(const void *)gemm_tc_kernel<kEpiHidden>, (const void *)gemm_tc_kernel<kEpiOut>,
                           (const void *)gemm_tc_kernel<kEpiLoss>, (const void *)gemm_tc_kernel<kEpiBack>,
-                          (const void *)gemm_dw_kernel})
+                          (const void *)gemm_dw_kernel, (const void *)fused_kernel<true>,
+                          (const void *)fused_kernel<false>})
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) != cudaSuccess)
             return bail(mlp_fail(m, "pfk_mlp_create: kernel configuration failed", PFK_ERR_CUDA));
     m->slot->loss = 0.0;
