@@ -13,24 +13,29 @@ namespace pfk {
 namespace {
 
 constexpr int kRegMaxComponents = 81;   // register path up to (pp|pp)-sized blocks
+// The split kernels' SPLIT build exists for the s..d classes, whose basis sets
+// have contracted shells in molecules small enough to need it.
+template <int LA>
+constexpr bool kSplitTeams = LA <= 2;
 
-constexpr long long kJoinQuartets = 1 << 15;
+constexpr long long kJoinLanes = 1 << 15;
 
 // The segments of a that give a quartet several lanes in one launch of the
 // SPLIT build, the runs of the others (all n quartets when a has no segments)
 // in launches of the one-lane build.
+// per: lanes (or teams) per block, of 128 / per threads each.
 template <typename SplitLaunch, typename PlainLaunch>
-void launch_segments(const uint2 *q, long long n, const JKArgs &a, SplitLaunch &&split, PlainLaunch &&plain)
+void launch_segments(const uint2 *q, long long n, const JKArgs &a, int per, SplitLaunch &&split, PlainLaunch &&plain)
 {
     if (a.seg.n == 0) {
-        plain(q, n, (unsigned)((n + 127) / 128));
+        plain(q, n, (unsigned)((n + per - 1) / per));
         return;
     }
     // few one-lane quartets go along in the SPLIT launch: a launch less
     long long single = 0;
     for (int s = 0; s < a.seg.n; ++s)
         if (a.seg.glog[s] == 0) single += a.seg.count[s];
-    const bool all = single < n && single <= kJoinQuartets;
+    const bool all = single < n && single * (128 / per) <= kJoinLanes;
     JKArgs b = a;
     b.seg.n = 0;
     unsigned blocks = 0;
@@ -41,7 +46,7 @@ void launch_segments(const uint2 *q, long long n, const JKArgs &a, SplitLaunch &
         b.seg.first[k] = a.seg.first[s];
         b.seg.count[k] = a.seg.count[s];
         b.seg.block0[k] = blocks;
-        blocks += (unsigned)(((a.seg.count[s] << a.seg.glog[s]) + 127) / 128);
+        blocks += (unsigned)(((a.seg.count[s] << a.seg.glog[s]) + per - 1) / per);
     }
     if (blocks) split(b, blocks);
     if (all) return;
@@ -50,17 +55,20 @@ void launch_segments(const uint2 *q, long long n, const JKArgs &a, SplitLaunch &
         const long long first = a.seg.first[s];
         long long cnt = a.seg.count[s];
         while (s + 1 < a.seg.n && a.seg.glog[s + 1] == 0) cnt += a.seg.count[++s];
-        plain(q + first * a.qstride, cnt, (unsigned)((cnt + 127) / 128));
+        plain(q + first * a.qstride, cnt, (unsigned)((cnt + per - 1) / per));
     }
 }
 
 template <int LA, int LB, int LC, int LD>
-void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flags, cudaStream_t st)
+void launch_class(const uint2 *q, long long n, const JKArgs &args, int nk, int flags, cudaStream_t st)
 {
     using S = ClassShape<LA, LB, LC, LD>;
     using SS = SplitShape<LA, LB, LC, LD>;
     using TS = TeamShape<LA, LB, LC, LD>;
     const int fp32 = flags & kLaunchFP32;
+    const bool out = args.blk_out || args.eri_out;   // tensor and block modes: the OUT builds, one density
+    JKArgs a = args;
+    if (out && fp32) a.seg.n = 0;                    // their FP32 builds have no SPLIT form
     if constexpr (LA + LB + LC + LD <= kOSMaxL) {
         if (flags & kLaunchOS) {
             if (n <= 0) return;
@@ -77,14 +85,17 @@ void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flag
             // flight, at 5 and 2 blocks per SM
             constexpr int PB = L == 0 ? 8 : L == 1 ? 6 : L == 2 ? 5 : L == 3 ? 3 : 1;
             launch_segments(
-                q, n, a,
+                q, n, a, 128,
                 [&](const JKArgs &b, unsigned grid) {
-                    if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2, double, 1, true><<<grid, 128, 0, st>>>(q, n, b);
+                    if (out) eri_os_kernel<LA, LB, LC, LD, 1, double, 1, true, true><<<grid, 128, 0, st>>>(q, n, b);
+                    else if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2, double, 1, true><<<grid, 128, 0, st>>>(q, n, b);
                     else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float, 1, true><<<grid, 128, 0, st>>>(q, n, b);
                     else eri_os_kernel<LA, LB, LC, LD, 1, double, 1, true><<<grid, 128, 0, st>>>(q, n, b);
                 },
                 [&](const uint2 *r, long long m, unsigned grid) {
-                    if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2, double, PB><<<grid, 128, 0, st>>>(r, m, a);
+                    if (out && fp32) eri_os_kernel<LA, LB, LC, LD, 1, float, PB, false, true><<<grid, 128, 0, st>>>(r, m, a);
+                    else if (out) eri_os_kernel<LA, LB, LC, LD, 1, double, PB, false, true><<<grid, 128, 0, st>>>(r, m, a);
+                    else if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2, double, PB><<<grid, 128, 0, st>>>(r, m, a);
                     else if (fp32 && dense) eri_os_kernel<LA, LB, LC, LD, 1, float, MB><<<grid, 128, 0, st>>>(r, m, a);
                     else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float, PB><<<grid, 128, 0, st>>>(r, m, a);
                     else if (dense) eri_os_kernel<LA, LB, LC, LD, 1, double, MB><<<grid, 128, 0, st>>>(r, m, a);
@@ -96,7 +107,9 @@ void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flag
     if constexpr (S::N <= kRegMaxComponents) {
         if (n <= 0) return;
         const long long grid = (n + 127) / 128;
-        if (nk == 2) eri_reg_kernel<LA, LB, LC, LD, 2><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
+        if (out && fp32) eri_reg_kernel<LA, LB, LC, LD, 1, float, true><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
+        else if (out) eri_reg_kernel<LA, LB, LC, LD, 1, double, true><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
+        else if (nk == 2) eri_reg_kernel<LA, LB, LC, LD, 2><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
         else if (fp32) eri_reg_kernel<LA, LB, LC, LD, 1, float><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
         else eri_reg_kernel<LA, LB, LC, LD, 1><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
     } else if constexpr (SS::OK) {
@@ -106,13 +119,44 @@ void launch_class(const uint2 *q, long long n, const JKArgs &a, int nk, int flag
             cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS::SMEM);
             cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)SF::SMEM);
+            cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, double, false, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS::SMEM);
+            cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, float, false, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SF::SMEM);
+            if constexpr (kSplitTeams<LA>) {
+                cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, double, true, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS::SMEM_SPLIT);
+                cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, double, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS::SMEM_SPLIT);
+                cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 2, double, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS::SMEM_SPLIT);
+                cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, float, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SF::SMEM_SPLIT);
+            }
             return;
         }
         if (n == 0) return;
-        const long long grid = (n + SS::TEAMS - 1) / SS::TEAMS;
-        if (nk == 2) eri_split_kernel<LA, LB, LC, LD, 2><<<(unsigned)grid, 128, SS::SMEM, st>>>(q, n, a);
-        else if (fp32) eri_split_kernel<LA, LB, LC, LD, 1, float><<<(unsigned)grid, 128, SF::SMEM, st>>>(q, n, a);
-        else eri_split_kernel<LA, LB, LC, LD, 1><<<(unsigned)grid, 128, SS::SMEM, st>>>(q, n, a);
+        const auto plain = [&](const uint2 *r, long long m, unsigned grid) {
+            if (out && fp32)
+                eri_split_kernel<LA, LB, LC, LD, 1, float, false, true><<<grid, 128, SF::SMEM, st>>>(r, m, a);
+            else if (out) eri_split_kernel<LA, LB, LC, LD, 1, double, false, true><<<grid, 128, SS::SMEM, st>>>(r, m, a);
+            else if (nk == 2) eri_split_kernel<LA, LB, LC, LD, 2><<<grid, 128, SS::SMEM, st>>>(r, m, a);
+            else if (fp32) eri_split_kernel<LA, LB, LC, LD, 1, float><<<grid, 128, SF::SMEM, st>>>(r, m, a);
+            else eri_split_kernel<LA, LB, LC, LD, 1><<<grid, 128, SS::SMEM, st>>>(r, m, a);
+        };
+        if constexpr (kSplitTeams<LA>)
+            launch_segments(
+                q, n, a, SS::TEAMS,
+                [&](const JKArgs &b, unsigned grid) {
+                    if (out)
+                        eri_split_kernel<LA, LB, LC, LD, 1, double, true, true><<<grid, 128, SS::SMEM_SPLIT, st>>>(q, n, b);
+                    else if (nk == 2) eri_split_kernel<LA, LB, LC, LD, 2, double, true><<<grid, 128, SS::SMEM_SPLIT, st>>>(q, n, b);
+                    else if (fp32) eri_split_kernel<LA, LB, LC, LD, 1, float, true><<<grid, 128, SF::SMEM_SPLIT, st>>>(q, n, b);
+                    else eri_split_kernel<LA, LB, LC, LD, 1, double, true><<<grid, 128, SS::SMEM_SPLIT, st>>>(q, n, b);
+                },
+                plain);
+        else
+            plain(q, n, (unsigned)((n + SS::TEAMS - 1) / SS::TEAMS));
     } else {
         using TF = TeamShape<LA, LB, LC, LD, float>;
         if (n < 0) {

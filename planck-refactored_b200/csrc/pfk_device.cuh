@@ -104,7 +104,8 @@ constexpr double kPrimQuartetTol = 1e-16;
 // are ordered by it), and a segment may give each quartet 2^glog lanes of a
 // warp that share its primitive loops and add up their sums by shuffles.
 // Entries [first, first + count) of the list belong to the segment, its
-// blocks start at block0.  n = 0: one lane per quartet throughout.
+// blocks start at block0.  n = 0: one lane per quartet throughout.  In the
+// split kernels the same counts whole teams of lanes.
 constexpr int kMaxSegments = 8;
 struct Segments {
     int n;
@@ -125,10 +126,16 @@ struct JKArgs {
     unsigned long long *Jacc;
     unsigned long long *Kacc0;
     unsigned long long *Kacc1;
-    double *eri_out;                    // dense tensor mode (nb^4) when non-null
+    // dense tensor mode when non-null: nb^4 values, or with eri_packed
+    // [i][j][k (k + 1) / 2 + l], k >= l, for every i and j
+    double *eri_out;
+    int eri_packed;
     // block mode when non-null: list entry t writes its normalised Cartesian
     // block, unscreened, to blk_out[t * N ...] (no digestion, no tensor)
     double *blk_out;
+    // block mode, optional: list entry t writes to blk_out[(blk_pos[t] - blk_first) * N ...]
+    const int *blk_pos;
+    long long blk_first;
     double tol;
     int nb;
     // this launch evaluates quartets[t * qstride + qoffset], t < nq (one
@@ -370,6 +377,25 @@ __host__ __device__ __forceinline__ double fx_value(long long hi, long long lo)
 // writes into its tensor (os.cpp:137-163) and then contracts
 // (os.cpp:1514-1520), with s = 1/|stabiliser| removing the duplicates.
 
+// Block mode: where list entry t's block goes, in blocks.
+__device__ __forceinline__ size_t block_pos(const JKArgs &a, long long t)
+{
+    return (size_t)(a.blk_pos ? a.blk_pos[t] - a.blk_first : t);
+}
+
+// Scatter of one AO quartet into the packed tensor: the members of its 8-fold
+// orbit with k >= l.
+__device__ __forceinline__ void scatter_packed(double *eri, int nb, int i, int j, int k, int l, double v)
+{
+    const size_t n = nb, np = n * (n + 1) / 2;
+    const size_t ij = i >= j ? (size_t)i * (i + 1) / 2 + j : (size_t)j * (j + 1) / 2 + i;
+    const size_t kl = k >= l ? (size_t)k * (k + 1) / 2 + l : (size_t)l * (l + 1) / 2 + k;
+    eri[(i * n + j) * np + kl] = v;
+    eri[(j * n + i) * np + kl] = v;
+    eri[(k * n + l) * np + ij] = v;
+    eri[(l * n + k) * np + ij] = v;
+}
+
 // 8-fold scatter of one AO quartet into a dense tensor (os.cpp:137-163).
 __device__ __forceinline__ void scatter8(double *eri, int nb, int i, int j, int k, int l, double v)
 {
@@ -382,6 +408,12 @@ __device__ __forceinline__ void scatter8(double *eri, int nb, int i, int j, int 
     eri[l * n3 + k * n2 + i * n + j] = v;
     eri[k * n3 + l * n2 + j * n + i] = v;
     eri[l * n3 + k * n2 + j * n + i] = v;
+}
+
+__device__ __forceinline__ void scatter(const JKArgs &a, int i, int j, int k, int l, double v)
+{
+    if (a.eri_packed) scatter_packed(a.eri_out, a.nb, i, j, k, l, v);
+    else scatter8(a.eri_out, a.nb, i, j, k, l, v);
 }
 
 }  // namespace pfk

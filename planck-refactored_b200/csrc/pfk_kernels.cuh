@@ -254,34 +254,39 @@ __device__ __forceinline__ int warp_bra_lead(bool live, unsigned bra)
 // scattered instead, in block mode written out.  Every lane of the warp calls
 // it; lanes with live = false hold a zero block (their digestion adds
 // nothing) and write nothing in the tensor and block modes.
-template <int LA, int LB, int LC, int LD, int NK, typename R>
+//
+// OUT: the build for the tensor and block modes; the others digest.  Builds
+// of their own because the unrolled scatter of every component cost the Fock
+// builds registers and schedule: (H2O)32 mixed 48.8 -> 46.5 ms a build (with
+// the split kernels' two blocks per SM at 54 accumulators).
+template <int LA, int LB, int LC, int LD, int NK, typename R, bool OUT>
 __device__ __forceinline__ void finish_block(R *acc, const uint2 qd, const PairInfo &pb, const PairInfo &pk,
                                              const JKArgs &args, bool live, long long t)
 {
     using S = ClassShape<LA, LB, LC, LD>;
     constexpr int NA = S::NA, NB = S::NB, NC = S::NC, ND = S::ND;
-    if (args.blk_out) {
-        if (!live) return;
-        double *o = args.blk_out + (size_t)t * S::N;
-#pragma unroll
-        for (int ia = 0; ia < NA; ++ia)
-#pragma unroll
-            for (int ib = 0; ib < NB; ++ib)
-#pragma unroll
-                for (int ic = 0; ic < NC; ++ic)
-#pragma unroll
-                    for (int id = 0; id < ND; ++id) {
-                        const int c = ((ia * NB + ib) * NC + ic) * ND + id;
-                        o[c] = double(acc[c]) * S::norm(ia, ib, ic, id);
-                    }
-        return;
-    }
     const int nb = args.nb;
     const int i0 = pb.bf_a, j0 = pb.bf_b, k0 = pk.bf_a, l0 = pk.bf_b;
     const bool same_ab = (i0 == j0), same_cd = (k0 == l0), same_bk = (qd.x == qd.y);
     const bool check = pb.qmin * pk.qmin < args.tol;
 
-    if (args.eri_out) {
+    if constexpr (OUT) {
+        if (args.blk_out) {
+            if (!live) return;
+            double *o = args.blk_out + block_pos(args, t) * S::N;
+#pragma unroll
+            for (int ia = 0; ia < NA; ++ia)
+#pragma unroll
+                for (int ib = 0; ib < NB; ++ib)
+#pragma unroll
+                    for (int ic = 0; ic < NC; ++ic)
+#pragma unroll
+                        for (int id = 0; id < ND; ++id) {
+                            const int c = ((ia * NB + ib) * NC + ic) * ND + id;
+                            o[c] = double(acc[c]) * S::norm(ia, ib, ic, id);
+                        }
+            return;
+        }
         if (!live) return;
 #pragma unroll
         for (int ia = 0; ia < NA; ++ia)
@@ -295,7 +300,7 @@ __device__ __forceinline__ void finish_block(R *acc, const uint2 qd, const PairI
                         const double sw = quartet_weight(same_ab, same_cd, same_bk, ia, ib, ic, id, NB, ND, check,
                                                          args.Qao, nb, i0 + ia, j0 + ib, k0 + ic, l0 + id, args.tol);
                         if (sw != 0.0)
-                            scatter8(args.eri_out, nb, i0 + ia, j0 + ib, k0 + ic, l0 + id,
+                            scatter(args, i0 + ia, j0 + ib, k0 + ic, l0 + id,
                                      double(acc[c]) * S::norm(ia, ib, ic, id));
                     }
         return;
@@ -320,6 +325,42 @@ __device__ __forceinline__ void finish_block(R *acc, const uint2 qd, const PairI
     digest_blocks<NA, NB, NC, ND, NK>(acc, i0, j0, k0, l0, args, lead);
 }
 
+// A lane's (or team's) place in a segmented launch with `per` of them per
+// block (Segments): list entry t (valid when in_list; the segment's last entry
+// otherwise, so that every lane has a quartet to read) and number sub of the
+// entry's 2^glog lanes, which are neighbours.  per >= 2^glog, a power of two.
+struct LaneWork {
+    long long t;
+    int sub, glog;
+    bool in_list;
+};
+__device__ __forceinline__ LaneWork lane_work(const Segments &sg, int per, int lane)
+{
+    LaneWork w{};
+    int s = 0;
+    while (s + 1 < sg.n && blockIdx.x >= sg.block0[s + 1]) ++s;
+    w.glog = sg.glog[s];
+    const long long u = (long long)(blockIdx.x - sg.block0[s]) * per + lane;
+    const long long i = u >> w.glog;
+    w.sub = (int)(u & ((1 << w.glog) - 1));
+    w.in_list = i < sg.count[s];
+    w.t = sg.first[s] + (w.in_list ? i : sg.count[s] - 1);
+    return w;
+}
+
+// How a quartet's lanes share its loops: ket primitives j0, j0 + js, ..., and
+// for each of them bra primitives i0, i0 + is, ... (js is = 2^glog).  The ket
+// side takes as many lanes as it has primitives for: lanes of one ket
+// primitive and several bra ones would load the ket primitive once each.
+struct PrimSplit {
+    int j0, js, i0, is;
+};
+__device__ __forceinline__ PrimSplit prim_split(const LaneWork &w, int nket)
+{
+    const int gj = min(w.glog, 31 - __clz(max(nket, 1)));
+    return {w.sub & ((1 << gj) - 1), 1 << gj, w.sub >> gj, 1 << (w.glog - gj)};
+}
+
 // ---------------------------------------------------------------------------
 // Register path
 // ---------------------------------------------------------------------------
@@ -328,7 +369,7 @@ __device__ __forceinline__ void finish_block(R *acc, const uint2 qd, const PairI
 // of quartets whose Schwarz bound is below the FP32 threshold.  Roots,
 // weights and the per-primitive-quartet scalars stay FP64 in both, and so
 // does the J/K digestion and accumulation.
-template <int LA, int LB, int LC, int LD, int NK, typename R = double>
+template <int LA, int LB, int LC, int LD, int NK, typename R = double, bool OUT = false>
 __global__ void __launch_bounds__(128) eri_reg_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
 {
     using S = ClassShape<LA, LB, LC, LD>;
@@ -390,7 +431,7 @@ __global__ void __launch_bounds__(128) eri_reg_kernel(const uint2 *__restrict__ 
         }
     }
 
-    finish_block<LA, LB, LC, LD, NK, R>(acc, qd, pb, pk, args, live, t);
+    finish_block<LA, LB, LC, LD, NK, R, OUT>(acc, qd, pb, pk, args, live, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -506,7 +547,7 @@ __global__ void __launch_bounds__(TeamShape<LA, LB, LC, LD, R>::BLOCK) eri_team_
             const int c = lane + k * TEAM;
             if (c >= S::N) continue;
             const int id = c % ND, ic = (c / ND) % NC, ib = (c / (ND * NC)) % NB, ia = c / (ND * NC * NB);
-            args.blk_out[(size_t)t * S::N + c] =
+            args.blk_out[block_pos(args, t) * S::N + c] =
                 double(acc[k]) * cart_norm(LA, ia) * cart_norm(LB, ib) * cart_norm(LC, ic) * cart_norm(LD, id);
         }
         return;
@@ -527,7 +568,7 @@ __global__ void __launch_bounds__(TeamShape<LA, LB, LC, LD, R>::BLOCK) eri_team_
         const double v =
             double(acc[k]) * sw * cart_norm(LA, ia) * cart_norm(LB, ib) * cart_norm(LC, ic) * cart_norm(LD, id);
         if (args.eri_out) {
-            scatter8(args.eri_out, nb, i, j, kk, l, v / sw);
+            scatter(args, i, j, kk, l, v / sw);
             continue;
         }
         fx_add(args.Jacc, (size_t)i * nb + j, v * __ldg(args.Pj + (size_t)kk * nb + l));
@@ -680,11 +721,16 @@ struct SplitShape {
     static constexpr bool TEAMRED =
         LEVEL == 1 && TEAM <= 32 && (REDV1 + 2 * REDVK) * GROUP * 8 <= TABLE * (int)sizeof(R);
     static constexpr bool OK = TEAM <= 128 && M <= 64;
+    // SPLIT build: the teams of a quartet add their blocks through shared memory
+    static constexpr size_t SMEM_SPLIT =
+        SMEM > sizeof(R) * TEAMS * GROUP * M ? SMEM : sizeof(R) * TEAMS * GROUP * M;
     // blocks of 128 per SM the register allocation must allow: the kernels
     // wait on loads more than on arithmetic, so four where the accumulators
     // leave room: (H2O)32 (dd|ps) 1.57 -> 1.43 ms, (dd|dp) 1.19 -> 1.01 (both
-    // M = 18); at M = 27 the spills cost more ((dp|pp) 3.42 -> 3.70)
-    static constexpr int MINB = M <= 18 ? 4 : 3;
+    // M = 18); at M = 27 the spills cost more ((dp|pp) 3.42 -> 3.70).  With 54
+    // accumulators three blocks spill 900 to 1300 bytes into the inner loop,
+    // two none: 16384 (fd|pp) blocks 4.00 -> 3.33 ms
+    static constexpr int MINB = M <= 18 ? 4 : M <= 36 ? 3 : 2;
 };
 
 template <int TEAM>
@@ -720,7 +766,13 @@ __device__ __forceinline__ int cart_l_axis(int i, int axis)
 // the contraction (double, or float for the FP32 list of quartets whose
 // Schwarz bound is below the FP32 threshold); roots, weights and the
 // per-primitive scalars stay FP64, and so does the digestion.
-template <int LA, int LB, int LC, int LD, int NK, typename R = double>
+//
+// SPLIT: the launch covers args.seg; 2^glog of the block's teams share a
+// quartet's primitive quartets (each 1 to 2 us of dependent loads, root
+// series and recurrences to a team, however idle the chip) and the first of
+// them adds up the others' blocks and digests.  One water / 6-31G** (dp|pp),
+// 27 primitive quartets: 66 -> 28 us; the build 149 -> 126 us.
+template <int LA, int LB, int LC, int LD, int NK, typename R = double, bool SPLIT = false, bool OUT = false>
 __global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) eri_split_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
 {
     using S = ClassShape<LA, LB, LC, LD>;
@@ -730,11 +782,17 @@ __global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) er
     extern __shared__ __align__(16) unsigned char pfk_dyn_smem[];
     R *smem = reinterpret_cast<R *>(pfk_dyn_smem);
     const int team = threadIdx.x / TEAM, lane = threadIdx.x % TEAM;
-    const long long t = (long long)blockIdx.x * SS::TEAMS + team;
-    // Whole teams leave together; every barrier below is per team.  No
-    // full-warp intrinsic follows: the teams of a warp run different
-    // primitive loops, each synchronising only its own lanes.
-    if (t >= nq) return;
+    LaneWork lw{};
+    if constexpr (SPLIT) {
+        lw = lane_work(args.seg, SS::TEAMS, team);
+    } else {
+        lw.t = (long long)blockIdx.x * SS::TEAMS + team;
+        // Whole teams leave together; every barrier below is per team.  No
+        // full-warp intrinsic follows: the teams of a warp run different
+        // primitive loops, each synchronising only its own lanes.
+        if (lw.t >= nq) return;
+    }
+    const long long t = lw.t;
     const unsigned mask = TEAM >= 32 ? 0xffffffffu
                                      : (((1u << TEAM) - 1u) << ((threadIdx.x & 31) / TEAM * TEAM));
     R *g = smem + team * SS::TABLE;   // g[r][axis][NIP]
@@ -742,7 +800,12 @@ __global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) er
     const uint2 qd = quartets[t * args.qstride + args.qoffset];
     const PairInfo pb = args.pairs[qd.x];
     const PairInfo pk = args.pairs[qd.y];
-    if (density_negligible(pb, pk, args)) return;   // whole quartet (team-uniform)
+    bool live = true;
+    if constexpr (SPLIT) {
+        live = lw.in_list && !density_negligible(pb, pk, args);   // every team reaches the block's barriers
+    } else {
+        if (density_negligible(pb, pk, args)) return;   // whole quartet (team-uniform)
+    }
     const bool owner = lane < SS::GROUP;
     const int gi = owner ? lane : 0;
     const int ia = LEVEL == 1 ? gi : gi / NB;
@@ -762,10 +825,13 @@ __global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) er
     // ket primitives outer: a warp's lanes usually share the bra pair, so the
     // inner loads of bra primitives are broadcasts
     const double qb0 = pb.nprim ? __ldg(&args.prims[pb.prim_off].qp) : 0.0;   // largest bra qp
-    for (int jp = 0; jp < pk.nprim; ++jp) {
+    const int nket = live ? pk.nprim : 0;
+    PrimSplit ps{0, 1, 0, 1};
+    if constexpr (SPLIT) ps = prim_split(lw, nket);
+    for (int jp = ps.j0; jp < nket; jp += ps.js) {
         const PrimPair q = load_prim(args.prims, pk.prim_off + jp);
         if (q.qp * qb0 < args.ptol) break;   // kets sorted by qp
-        for (int ip = 0; ip < pb.nprim; ++ip) {
+        for (int ip = ps.i0; ip < pb.nprim; ip += ps.is) {
             const PrimPair p = load_prim(args.prims, pb.prim_off + ip);
             if (p.qp * q.qp < args.ptol) break;   // bras sorted by qp
             const QuartetScalars s = quartet_scalars(p, q);
@@ -818,6 +884,20 @@ __global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) er
             split_sync<TEAM>(mask, team);
         }
     }
+    if constexpr (SPLIT) {
+        __syncthreads();   // every team is past its tables
+        R *red = smem;
+        if (lw.sub && owner)
+#pragma unroll
+            for (int c = 0; c < M; ++c) red[(team * M + c) * SS::GROUP + gi] = acc[c];
+        __syncthreads();
+        if (!lw.sub && owner)
+            for (int k = 1; k < 1 << lw.glog; ++k)
+#pragma unroll
+                for (int c = 0; c < M; ++c) acc[c] += red[((team + k) * M + c) * SS::GROUP + gi];
+        __syncthreads();   // the first teams stage their digestion in the same memory
+        if (lw.sub || !live) return;
+    }
     // ---- digestion of this thread's components: A index ia, B indices
     // ib0 .. ib0 + NBT - 1, all C and D.  Non-owner lanes hold a zero block
     // (ia = 0) and take part only in the team reduction. ----
@@ -827,8 +907,9 @@ __global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) er
     const bool check = pb.qmin * pk.qmin < args.tol;
     const int i = i0 + ia;
 
-    if (args.blk_out) {
+    if (OUT && args.blk_out) {
         if (!owner) return;
+        const size_t at = block_pos(args, t);
 #pragma unroll
         for (int bl = 0; bl < NBT; ++bl)
 #pragma unroll
@@ -837,12 +918,12 @@ __global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) er
                 for (int id = 0; id < ND; ++id) {
                     const int ib = ib0 + bl;
                     const double nrm = cart_norm_rt<LA>(ia) * cart_norm_rt<LB>(ib) * cart_norm(LC, ic) * cart_norm(LD, id);
-                    args.blk_out[(size_t)t * S::N + ((ia * NB + ib) * NC + ic) * ND + id] =
+                    args.blk_out[at * S::N + ((ia * NB + ib) * NC + ic) * ND + id] =
                         double(acc[(bl * NC + ic) * ND + id]) * nrm;
                 }
         return;
     }
-    if (args.eri_out) {
+    if constexpr (OUT) {
         if (!owner) return;
 #pragma unroll
         for (int bl = 0; bl < NBT; ++bl)
@@ -855,7 +936,7 @@ __global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) er
                                                      nb, i, j0 + ib, k0 + ic, l0 + id, args.tol);
                     if (sw != 0.0) {
                         const double nrm = cart_norm_rt<LA>(ia) * cart_norm_rt<LB>(ib) * cart_norm(LC, ic) * cart_norm(LD, id);
-                        scatter8(args.eri_out, nb, i, j0 + ib, k0 + ic, l0 + id, double(acc[(bl * NC + ic) * ND + id]) * nrm);
+                        scatter(args, i, j0 + ib, k0 + ic, l0 + id, double(acc[(bl * NC + ic) * ND + id]) * nrm);
                     }
                 }
         return;

@@ -369,42 +369,6 @@ __device__ __forceinline__ void os_hrr(const R *__restrict__ acc, const R AB[3],
     });
 }
 
-// This thread's place in a segmented launch of 128-thread blocks (Segments):
-// list entry t (valid when in_list; the list's last entry otherwise, so that
-// every lane has a quartet to read) and lane sub of the entry's 2^glog lanes,
-// which are neighbours in a warp.
-struct LaneWork {
-    long long t;
-    int sub, glog;
-    bool in_list;
-};
-__device__ __forceinline__ LaneWork lane_work(const Segments &sg)
-{
-    LaneWork w{};
-    int s = 0;
-    while (s + 1 < sg.n && blockIdx.x >= sg.block0[s + 1]) ++s;
-    w.glog = sg.glog[s];
-    const long long u = (long long)(blockIdx.x - sg.block0[s]) * 128 + threadIdx.x;
-    const long long i = u >> w.glog;
-    w.sub = (int)(u & ((1 << w.glog) - 1));
-    w.in_list = i < sg.count[s];
-    w.t = sg.first[s] + (w.in_list ? i : sg.count[s] - 1);
-    return w;
-}
-
-// How a quartet's lanes share its loops: ket primitives j0, j0 + js, ..., and
-// for each of them bra primitives i0, i0 + is, ... (js is = 2^glog).  The ket
-// side takes as many lanes as it has primitives for: lanes of one ket
-// primitive and several bra ones would load the ket primitive once each.
-struct PrimSplit {
-    int j0, js, i0, is;
-};
-__device__ __forceinline__ PrimSplit prim_split(const LaneWork &w, int nket)
-{
-    const int gj = min(w.glog, 31 - __clz(max(nket, 1)));
-    return {w.sub & ((1 << gj) - 1), 1 << gj, w.sub >> gj, 1 << (w.glog - gj)};
-}
-
 // Sum of every lane's block over the 2^glog lanes of its quartet, left on the
 // first of them; the others hold zeros (no contribution to the digestion).
 template <int N, typename R>
@@ -430,14 +394,14 @@ __device__ __forceinline__ void lanes_sum(R *acc, const LaneWork &w)
 // lanes (Segments); otherwise one lane per quartet over nq entries.  Two
 // builds because the split bookkeeping costs the other one 4 to 8 registers
 // ((ss|ss) 62 -> 68: 7 blocks per SM instead of 8).
-template <int LA, int LB, int LC, int LD, int NK, typename R = double, int MINB = 1, bool SPLIT = false>
+template <int LA, int LB, int LC, int LD, int NK, typename R = double, int MINB = 1, bool SPLIT = false, bool OUT = false>
 __global__ void __launch_bounds__(128, MINB) eri_os_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
 {
     using O = OSShape<LA, LB, LC, LD>;
     constexpr int L = O::L;
     LaneWork lw{};
     if constexpr (SPLIT) {
-        lw = lane_work(args.seg);
+        lw = lane_work(args.seg, 128, (int)threadIdx.x);
     } else {
         lw.t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
         lw.in_list = lw.t < nq;
@@ -481,7 +445,7 @@ __global__ void __launch_bounds__(128, MINB) eri_os_kernel(const uint2 *__restri
     const R AB[3] = {R(pb.ABx), R(pb.ABy), R(pb.ABz)};
     const R CD[3] = {R(pk.ABx), R(pk.ABy), R(pk.ABz)};
     os_hrr<LA, LB, LC, LD, R>(acc, AB, CD, blk);
-    finish_block<LA, LB, LC, LD, NK, R>(blk, qd, pb, pk, args, live && lw.sub == 0, lw.t);
+    finish_block<LA, LB, LC, LD, NK, R, OUT>(blk, qd, pb, pk, args, live && lw.sub == 0, lw.t);
 }
 
 }  // namespace pfk

@@ -386,14 +386,15 @@ __device__ __forceinline__ int length_bucket(const PairInfo &b, const PairInfo &
 // otherwise), then (evaluated bra primitives, evaluated ket primitives), so
 // that a warp's lanes run the same primitive loop lengths.
 __global__ void quartet_key_kernel(const uint2 *__restrict__ q, long long n, const PairInfo *__restrict__ pairs,
-                                   unsigned *keys)
+                                   int prim_bits, unsigned *keys)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const uint2 v = q[t];
     const PairInfo b = pairs[v.x], k = pairs[v.y];
-    // nprim <= 4096 needs 13 bits, the bucket (0..24) 5
-    keys[t] = (unsigned)(31 - length_bucket(b, k)) << 26 | (unsigned)b.nprim << 13 | (unsigned)k.nprim;
+    // nprim < 2^prim_bits <= 2^13, the bucket 0 .. 2 prim_bits
+    keys[t] = (unsigned)(2 * prim_bits - length_bucket(b, k)) << (2 * prim_bits) | (unsigned)b.nprim << prim_bits |
+              (unsigned)k.nprim;
 }
 
 // First entry of every length bucket of a sorted list (untouched when empty).
@@ -417,22 +418,35 @@ cudaError_t bucket_starts(const uint2 *q, long long n, const PairInfo *pairs, lo
     return cudaGetLastError();
 }
 
-// Stable sort of one list segment by its key; tmp buffers sized by the caller
-// (keys_a/keys_b: n unsigned, vals_b: n uint2, temp: temp_bytes).
-cudaError_t sort_quartets(uint2 *q, long long n, const PairInfo *pairs, unsigned *keys_a, unsigned *keys_b,
-                          uint2 *vals_b, void *temp, size_t &temp_bytes, cudaStream_t st)
+__global__ void rank_key_kernel(const uint2 *__restrict__ q, long long n, const unsigned *__restrict__ rank, int ket,
+                                unsigned *keys)
 {
-    if (!temp) {
-        return cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys_a, keys_b,
-                                               reinterpret_cast<unsigned long long *>(q),
-                                               reinterpret_cast<unsigned long long *>(vals_b), n, 0, 31, st);
-    }
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) keys[t] = rank[ket ? q[t].y : q[t].x];
+}
+
+// Orders one list: by (loop length, bra rank, ket rank), as three stable
+// radix sorts, least significant key first, over the bits that the ranks and
+// primitive counts have.  tmp buffers sized by the caller (keys_a/keys_b: n
+// unsigned, vals_b: n uint2, temp: temp_bytes).
+cudaError_t sort_quartets(uint2 *q, long long n, const PairInfo *pairs, const SortKeys &k, unsigned *keys_a,
+                          unsigned *keys_b, uint2 *vals_b, void *temp, size_t &temp_bytes, cudaStream_t st)
+{
+    auto *a = reinterpret_cast<unsigned long long *>(q), *b = reinterpret_cast<unsigned long long *>(vals_b);
+    if (!temp) return cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys_a, keys_b, a, b, n, 0, 32, st);
     if (n <= 1) return cudaSuccess;
-    quartet_key_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(q, n, pairs, keys_a);
-    cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys_a, keys_b,
-                                                    reinterpret_cast<unsigned long long *>(q),
-                                                    reinterpret_cast<unsigned long long *>(vals_b), n, 0, 31, st);
-    if (e != cudaSuccess) return e;
+    const unsigned grid = (unsigned)((n + 255) / 256);
+    int len_bits = 1;   // of a bucket number, 0 .. 2 prim_bits
+    while (1 << len_bits <= 2 * k.prim_bits) ++len_bits;
+    const int bits[3] = {k.ket_bits, k.bra_bits, 2 * k.prim_bits + len_bits};
+    for (int i = 0; i < 3; ++i) {
+        const uint2 *src = i == 1 ? vals_b : q;
+        if (i < 2) rank_key_kernel<<<grid, 256, 0, st>>>(src, n, i == 0 ? k.ket_rank : k.bra_rank, i == 0, keys_a);
+        else quartet_key_kernel<<<grid, 256, 0, st>>>(src, n, pairs, k.prim_bits, keys_a);
+        cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys_a, keys_b, i == 1 ? b : a,
+                                                        i == 1 ? a : b, n, 0, bits[i], st);
+        if (e != cudaSuccess) return e;
+    }
     return cudaMemcpyAsync(q, vals_b, sizeof(uint2) * n, cudaMemcpyDeviceToDevice, st);
 }
 

@@ -35,7 +35,13 @@ cudaError_t shell_block_max(int nshell, const int *bf_off, const int *nbf, const
 // empty buckets stay as they are.
 constexpr int kLengthBuckets = 25;
 cudaError_t bucket_starts(const uint2 *q, long long n, const PairInfo *pairs, long long *start, cudaStream_t st);
-cudaError_t sort_quartets(uint2 *q, long long n, const PairInfo *pairs, unsigned *keys_a, unsigned *keys_b,
-                          uint2 *vals_b, void *temp, size_t &temp_bytes, cudaStream_t st);
+// Sort keys of one list: ranks of the pairs as bras and as kets (by pair id)
+// and how many bits they and the primitive counts take.
+struct SortKeys {
+    const unsigned *bra_rank, *ket_rank;
+    int bra_bits, ket_bits, prim_bits;
+};
+cudaError_t sort_quartets(uint2 *q, long long n, const PairInfo *pairs, const SortKeys &k, unsigned *keys_a,
+                          unsigned *keys_b, uint2 *vals_b, void *temp, size_t &temp_bytes, cudaStream_t st);
 
 }  // namespace pfk
