@@ -81,7 +81,9 @@ pfk_status pfk_destroy(pfk_ctx *ctx);
 
 /* OptionsIntegral (types.h:408-412): tol_eri and engine.  precision and
  * fp32_bound select the mixed-precision path.  Rebuilds the quartet lists
- * when tol_eri or fp32_bound change. */
+ * when tol_eri, precision or fp32_bound change.  If that fails (no memory),
+ * the context has no lists: builds, counts and statistics return
+ * PFK_ERR_STATE until a later call succeeds. */
 pfk_status pfk_set_options(pfk_ctx *ctx, double tol_eri, int engine, int precision,
                            double fp32_bound);
 

@@ -24,6 +24,9 @@ ClassLauncher g_class_launchers[kQuartetClasses];   // constant-initialised; fil
 namespace {
 
 thread_local std::string g_last_error;   // for failures without a context
+// Countdown to a device allocation that fails (0: none); set by the tests
+// through pfk_test_fail_alloc, for this thread.
+thread_local long long g_fail_alloc = 0;
 
 template <typename T>
 struct DevBuf {
@@ -39,9 +42,14 @@ struct DevBuf {
     {
         release();
         if (count == 0) return cudaSuccess;
+        if (g_fail_alloc > 0 && --g_fail_alloc == 0) return cudaErrorMemoryAllocation;
         const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&p), sizeof(T) * count);
-        if (e == cudaSuccess) n = count;
-        else p = nullptr;
+        if (e == cudaSuccess) {
+            n = count;
+        } else {
+            p = nullptr;
+            cudaGetLastError();   // reported here, not by the next launch's check
+        }
         return e;
     }
     void release()
@@ -125,6 +133,9 @@ struct pfk_ctx {
     DevBuf<uint2> d_quart;
     long long q_off[kQuartetClasses] = {}, q_cnt[kQuartetClasses] = {};
     long long q32_off[kQuartetClasses] = {}, q32_cnt[kQuartetClasses] = {};
+    // the list members (d_quart, counts, offsets, bucket0) belong together and
+    // to the options: set by build_lists when all of them are made
+    bool lists_ok = false;
     // first entry of every loop-length bucket of each class's FP64 list and of
     // its FP32 list (-1: empty bucket), longest first in the lists
     std::vector<long long> bucket0;
@@ -312,7 +323,6 @@ pfk_status upload_pairs(pfk_ctx *ctx)
     return PFK_OK;
 }
 
-// Screened shell-quartet lists for the current tol / FP32 bound.
 // Releases the captured RHF builds; the next device call captures again.
 void drop_graphs(pfk_ctx *ctx)
 {
@@ -340,7 +350,7 @@ cudaError_t side_streams(pfk_ctx *ctx, int n)
 // (ff|ff), where the s..d classes stay within 1e-7 relative.
 constexpr int kFirstFPairClass = 6;
 
-pfk_status build_lists(pfk_ctx *ctx)
+pfk_status make_lists(pfk_ctx *ctx)
 {
     const double bound = ctx->precision == PFK_PREC_MIXED ? ctx->fp32_bound : 0.0;
     int maxn = 1;
@@ -489,8 +499,30 @@ pfk_status build_lists(pfk_ctx *ctx)
                                ctx->stream));
         PFK_CK(cudaStreamSynchronize(ctx->stream));
     }
-    drop_graphs(ctx);   // captured builds refer to the old lists
     return PFK_OK;
+}
+
+// Screened shell-quartet lists for the current tol / FP32 bound.  A failure
+// leaves the context without lists: builds are refused (need_lists) until a
+// later call has made them.
+pfk_status build_lists(pfk_ctx *ctx)
+{
+    drop_graphs(ctx);   // captured builds refer to the old lists
+    ctx->lists_ok = false;
+    pfk_status s;
+    try {
+        s = make_lists(ctx);
+    } catch (const std::bad_alloc &) {
+        s = ctx->fail(PFK_ERR_NOMEM, "host allocation failed");
+    }
+    ctx->lists_ok = s == PFK_OK;
+    return s;
+}
+
+pfk_status need_lists(pfk_ctx *ctx)
+{
+    return ctx->lists_ok ? PFK_OK
+                         : ctx->fail(PFK_ERR_STATE, "no quartet lists (their last build failed): call pfk_set_options again");
 }
 
 pfk_status schwarz_and_sort(pfk_ctx *ctx)
@@ -641,6 +673,8 @@ void list_segments(const pfk_ctx *ctx, const long long *bucket0, long long n, in
 pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const double *Pk1, int nk, FxWord *Jacc,
                        FxWord *K0, FxWord *K1, double *eri_out, cudaStream_t st, bool timed, bool eri_packed = false)
 {
+    pfk_status ls = need_lists(ctx);
+    if (ls != PFK_OK) return ls;
     const size_t nb2 = (size_t)ctx->nb * ctx->nb;
     if (!eri_out) {
         PFK_CK(cudaMemsetAsync(Jacc, 0, sizeof(FxWord) * 2 * nb2, st));
@@ -936,7 +970,7 @@ pfk_status pfk_set_options(pfk_ctx *ctx, double tol_eri, int engine, int precisi
     if (precision == PFK_PREC_MIXED && !(fp32_bound > 0.0 && std::isfinite(fp32_bound)))
         return ctx->fail(PFK_ERR_INVALID, "fp32_bound must be positive");
     cudaSetDevice(ctx->device);
-    const bool rebuild = tol_eri != ctx->tol || precision != ctx->precision ||
+    const bool rebuild = !ctx->lists_ok || tol_eri != ctx->tol || precision != ctx->precision ||
                          (precision == PFK_PREC_MIXED && fp32_bound != ctx->fp32_bound);
     if (engine != ctx->engine) drop_graphs(ctx);   // captured builds hold the old engine's kernels
     ctx->tol = tol_eri;
@@ -944,6 +978,15 @@ pfk_status pfk_set_options(pfk_ctx *ctx, double tol_eri, int engine, int precisi
     ctx->precision = precision;
     if (precision == PFK_PREC_MIXED) ctx->fp32_bound = fp32_bound;
     return rebuild ? build_lists(ctx) : PFK_OK;
+}
+
+// For the tests (not in the header): the n-th device allocation of this
+// thread from now on fails; 0 for none.  Returns what was left of the last count.
+long long pfk_test_fail_alloc(long long nth)
+{
+    const long long left = g_fail_alloc;
+    g_fail_alloc = nth;
+    return left;
 }
 
 pfk_status pfk_schwarz(pfk_ctx *ctx, double *Q)
@@ -956,6 +999,8 @@ pfk_status pfk_schwarz(pfk_ctx *ctx, double *Q)
 
 static pfk_status run_census(pfk_ctx *ctx, long long *n_ao, uint64_t *digest, long long *n_shell, int *out, long long cap)
 {
+    pfk_status ls = need_lists(ctx);
+    if (ls != PFK_OK) return ls;
     cudaSetDevice(ctx->device);
     DevBuf<unsigned long long> cnt;
     PFK_CK(cnt.alloc(3));
@@ -999,6 +1044,8 @@ pfk_status pfk_quartet_list(pfk_ctx *ctx, int *out, long long cap, long long *n)
 // Captured-graph replay of the RHF build for a (dP, dG, stream) triple.
 static pfk_status rhf_graph(pfk_ctx *ctx, const double *dP, double *dG, cudaStream_t st)
 {
+    pfk_status ls = need_lists(ctx);   // before a capture begins
+    if (ls != PFK_OK) return ls;
     GraphEntry *ge = nullptr;
     for (auto &g : ctx->graphs)
         if (g.in == dP && g.out == dG && g.stream == st) ge = &g;
@@ -1400,6 +1447,8 @@ pfk_status pfk_mo_transform_times(const pfk_ctx *ctx, double *ms3)
 pfk_status pfk_class_stats(pfk_ctx *ctx, long long *quartets55, long long *prim_quartets55, double *ms55)
 {
     if (!ctx) return PFK_ERR_STATE;
+    pfk_status ls = need_lists(ctx);
+    if (ls != PFK_OK) return ls;
     cudaSetDevice(ctx->device);
     if (ms55) {
         for (int c = 0; c < kQuartetClasses; ++c) ctx->class_ms[c] = 0.f;
@@ -1418,6 +1467,8 @@ pfk_status pfk_class_stats(pfk_ctx *ctx, long long *quartets55, long long *prim_
 pfk_status pfk_precision_stats(pfk_ctx *ctx, long long *fp32_quartets55, long long *fp32_prim_quartets55)
 {
     if (!ctx) return PFK_ERR_STATE;
+    pfk_status ls = need_lists(ctx);
+    if (ls != PFK_OK) return ls;
     for (int c = 0; c < kQuartetClasses; ++c) {
         const bool mixed = ctx->precision == PFK_PREC_MIXED;
         if (fp32_quartets55) fp32_quartets55[c] = mixed ? ctx->q32_cnt[c] : 0;
@@ -1429,8 +1480,10 @@ pfk_status pfk_precision_stats(pfk_ctx *ctx, long long *fp32_quartets55, long lo
 pfk_status pfk_autotune(pfk_ctx *ctx, int *choice55, double *ms55x3)
 {
     if (!ctx) return PFK_ERR_STATE;
+    pfk_status s = need_lists(ctx);
+    if (s != PFK_OK) return s;
     cudaSetDevice(ctx->device);
-    pfk_status s = ensure_work(ctx);
+    s = ensure_work(ctx);
     if (s != PFK_OK) return s;
     const size_t nb2 = (size_t)ctx->nb * ctx->nb;
     PFK_CK(cudaMemsetAsync(ctx->d_P.p, 0, sizeof(double) * nb2, ctx->stream));   // timing only needs a density
