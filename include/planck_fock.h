@@ -354,7 +354,7 @@ const char *pfk_mlp_last_error(const pfk_mlp *m);
 long long pfk_mlp_param_count(const pfk_mlp *m);
 pfk_status pfk_mlp_set_params(pfk_mlp *m, const float *params);   /* host; resets Adam */
 pfk_status pfk_mlp_get_params(pfk_mlp *m, float *params);         /* host */
-/* Y = network(X). */
+/* Y = network(X).  Y may overlap X. */
 pfk_status pfk_mlp_forward(pfk_mlp *m, const float *X, int n, float *Y, void *stream);
 /* Gradients (host vector in the parameter layout, may be NULL) and the loss
  * mean((Y - T)^2) of one batch, without an update. */

@@ -928,10 +928,19 @@ void fused(pfk_mlp *m, int n, const float *X, float *Y, const float *T, cudaStre
     else fused_kernel<false><<<grid, TC_THREADS, TC_SMEM, st>>>(a, &m->d_slot->tc_err);
 }
 
+// Whether the n rows of Y share memory with the n rows of X.
+bool overlaps(const pfk_mlp *m, int n, const float *X, const float *Y)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(X), y = reinterpret_cast<uintptr_t>(Y);
+    return y < x + sizeof(float) * (size_t)n * m->dims[0] && x < y + sizeof(float) * (size_t)n * m->dims[m->nl];
+}
+
 // Forward pass of n rows of X: to Y, or, with T, to dZ of the last layer and the loss.
 void forward(pfk_mlp *m, int n, const float *X, float *Y, const float *T, cudaStream_t st)
 {
-    if (fusable(m)) return fused(m, n, X, Y, T, st);
+    // the fused kernel's clusters write their rows of Y while others still
+    // read X; layer by layer, all of X is converted before Y is written
+    if (fusable(m) && (T || !overlaps(m, n, X, Y))) return fused(m, n, X, Y, T, st);
     const bool train = T != nullptr;
     const int d0 = m->dims[0];
     dim3 gi((d0 + 31) / 32, (n + 31) / 32);

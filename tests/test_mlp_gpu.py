@@ -129,3 +129,23 @@ def test_tile_edges(dims, n):
     Y1o = mlp_ref.forward(dims, p1, X)[0]
     assert np.linalg.norm(net.forward(Xd).cpu().numpy() - Y1o) < 1e-4 * np.linalg.norm(Y1o)
     net.close()
+
+
+@pytest.mark.parametrize("dims", [[64, 64], [64, 128, 64], [256, 8], [8, 256], [264, 264]])
+def test_output_over_the_input(dims):
+    """pfk_mlp_forward converts X before it writes Y, so Y may lie anywhere on
+    X: the bits of a separate output.  1000 rows are eight row tiles, whose
+    outputs land on other tiles' inputs when the widths or the starts differ."""
+    torch = pytest.importorskip("torch")
+    n = 1000
+    net = _net(dims, seed=4, max_batch=n)
+    X, _ = _data(dims, n, 6)
+    Y = net.forward(torch.from_numpy(X).cuda()).cpu().numpy()
+    nx, ny = n * dims[0], n * dims[-1]
+    for at in (0, 4, dims[0] * 129, max(nx - ny, 0)):       # Y's start, in floats after X's
+        buf = torch.zeros(max(nx, at + ny), device="cuda")
+        buf[:nx] = torch.from_numpy(X).cuda().reshape(-1)
+        torch.cuda.synchronize()
+        net._check(net.L.pfk_mlp_forward(net.h, buf.data_ptr(), n, buf.data_ptr() + 4 * at, None))
+        assert np.array_equal(buf[at:at + ny].view(n, -1).cpu().numpy(), Y), at
+    net.close()
