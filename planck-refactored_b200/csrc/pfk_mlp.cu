@@ -490,12 +490,13 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemm_dw_kernel(Layers L, int n,
 }
 
 // H = bf16(X) and, with HT, its transpose (zero up to the next multiple of 8
-// rows); 32 x 32 tiles through shared memory.
+// rows); 32 x 32 tiles through shared memory, rows of the batch along grid.x
+// (grid.y ends at 65535).
 __global__ void __launch_bounds__(256) input_kernel(const float *__restrict__ X, int n, int d, __nv_bfloat16 *H,
                                                     __nv_bfloat16 *HT, long long ldt)
 {
     __shared__ __nv_bfloat16 tile[32][33];
-    const int x = threadIdx.x & 31, y = threadIdx.x >> 5, c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5, c0 = blockIdx.y * 32, r0 = blockIdx.x * 32;
     grid_launch_next();
 #pragma unroll
     for (int i = y; i < 32; i += 8) {
@@ -943,7 +944,7 @@ void forward(pfk_mlp *m, int n, const float *X, float *Y, const float *T, cudaSt
     if (fusable(m) && (T || !overlaps(m, n, X, Y))) return fused(m, n, X, Y, T, st);
     const bool train = T != nullptr;
     const int d0 = m->dims[0];
-    dim3 gi((d0 + 31) / 32, (n + 31) / 32);
+    dim3 gi((n + 31) / 32, (d0 + 31) / 32);
     input_kernel<<<gi, 256, 0, st>>>(X, n, d0, m->H[0], train ? m->HT[0] : nullptr, m->ldt);
     long long col = 0;
     for (int l = 0; l < m->nl; ++l) {

@@ -149,3 +149,18 @@ def test_output_over_the_input(dims):
         net._check(net.L.pfk_mlp_forward(net.h, buf.data_ptr(), n, buf.data_ptr() + 4 * at, None))
         assert np.array_equal(buf[at:at + ny].view(n, -1).cpu().numpy(), Y), at
     net.close()
+
+
+def test_rows_beyond_a_grid_axis():
+    """65535 x 32 rows and a few more through the layer-by-layer path: the
+    input conversion's row tiles are not limited to one grid's y axis.  The
+    last rows' outputs are those of a small batch (a row's arithmetic does not
+    depend on its batch)."""
+    torch = pytest.importorskip("torch")
+    dims, n = [264, 8], 65535 * 32 + 70
+    net = _net(dims, seed=2, max_batch=n)
+    X = torch.randn((n, dims[0]), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    Y = net.forward(X)
+    for a, b in ((0, 100), (n - 300, n)):
+        assert bool((net.forward(X[a:b].contiguous()) == Y[a:b]).all())
+    net.close()
