@@ -164,3 +164,21 @@ def test_rows_beyond_a_grid_axis():
     for a, b in ((0, 100), (n - 300, n)):
         assert bool((net.forward(X[a:b].contiguous()) == Y[a:b]).all())
     net.close()
+
+
+@pytest.mark.parametrize("dims,n", [([24, 8], 129), ([72, 136, 8], 127), ([112, 256, 256, 232], 300), ([264, 16], 70)])
+def test_unaligned_input(dims, n):
+    """X 4 bytes past a 16-byte boundary: the bits of an aligned X."""
+    torch = pytest.importorskip("torch")
+    net = _net(dims, seed=9, max_batch=n)
+    X, T = _data(dims, n, 10)
+    Xd, Td = torch.from_numpy(X).cuda(), torch.from_numpy(T).cuda()
+    flat = torch.zeros(n * dims[0] + 1, device="cuda")
+    flat[1:] = Xd.reshape(-1)
+    Xu = flat[1:].view(n, dims[0])
+    assert Xu.data_ptr() % 16 == 4
+    assert bool((net.forward(Xu) == net.forward(Xd)).all())
+    g, loss = net.gradients(Xd, Td)
+    gu, lossu = net.gradients(Xu, Td)
+    assert np.array_equal(g, gu) and loss == lossu
+    net.close()
