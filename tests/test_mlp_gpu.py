@@ -182,3 +182,35 @@ def test_unaligned_input(dims, n):
     gu, lossu = net.gradients(Xu, Td)
     assert np.array_equal(g, gu) and loss == lossu
     net.close()
+
+
+def test_many_networks_share_the_host_slots():
+    """150 networks at a time (64 result slots per page-locked slab), made,
+    used and closed from several threads, give one network's results."""
+    import threading
+    torch = pytest.importorskip("torch")
+    dims, n = [16, 24, 8], 40
+    X, T = _data(dims, n, 3)
+    Xd, Td = torch.from_numpy(X).cuda(), torch.from_numpy(T).cuda()
+    torch.cuda.synchronize()
+    first = _net(dims, seed=1)
+    g0, loss0 = first.gradients(Xd, Td)
+    bad = []
+
+    def work(k):
+        for _ in range(2):
+            nets = [_net(dims, seed=1) for _ in range(50)]
+            for net in nets[k::3] + nets[:2]:
+                g, loss = net.gradients(Xd, Td, stream=torch.cuda.Stream())
+                if loss != loss0 or not np.array_equal(g, g0):
+                    bad.append(k)
+            for net in nets[::-1] if k == 1 else nets:
+                net.close()
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    assert first.gradients(Xd, Td)[1] == loss0
+    first.close()
