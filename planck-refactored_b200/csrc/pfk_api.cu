@@ -1,6 +1,7 @@
 // pfk_api.cu -- the C ABI (include/planck_fock.h): context, per-geometry
 // setup, and the per-iteration Fock builds.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -19,6 +20,7 @@ using namespace pfk;
 
 namespace pfk {
 ClassLauncher g_class_launchers[kQuartetClasses];   // constant-initialised; filled by the class units
+ClassResident g_class_resident[kQuartetClasses];
 }
 
 namespace {
@@ -1864,7 +1866,19 @@ extern "C" pfk_status pfk_fock_rhf_noalloc(const pfk_basis_desc *basis, const do
 // A batch's quartets come in the caller's order, with contraction depths that
 // have nothing to do with their neighbours': a warp (or a block of teams) ran
 // until its longest loop was through: 16384 (fd|pp) quartets 5.99 -> 4.00 ms
-// in windows of this many.
+// in windows of this many, longest loops first.
+//
+// A launch that the device takes in one wave lasts as long as its slowest
+// warp, and that one is slower in a window's order: its 32 quartets are all
+// of the longest, each with primitives of its own to load, to the end, where
+// in the caller's order most lanes drop out.  So up to one wave
+// (g_class_resident) runs as listed, in the builds for that (kLaunchShort),
+// and the windows begin above it.  Windowed / listed time, FP64, at n of the
+// wave w: (ss|ss) w = 151552: 2.2 (n = 8192), 1.6 (65536); (ps|ps) Rys 1.9,
+// 1.3 (w = 75776); (pp|pp) w = 37888: 1.4, 0.72; (pp|ps) w = 56832: 1.55, 0.84;
+// (dp|pp) w = 7104: 1.02 (6144), 0.92 (8192), 0.66 (16384); (fp|pp) w = 3552:
+// 1.09 (3072), 1.06 (4096), 0.62 (16384); (dd|dd) w = 888: 1.00 (512), 0.91
+// (1024), 0.58 (8192).
 constexpr long long kBatchWindow = 1 << 14;
 struct pfk_eri_batch {
     int ncomp = 0;             // components per quartet
@@ -1883,6 +1897,17 @@ struct pfk_eri_batch {
     std::vector<int> pair_nprim;
     long long nq = 0;
     int cls = -1;              // class of the listed quartets
+    // one wave of the listed class per launch flags (-1: not asked for yet)
+    std::atomic<long long> wave[16] = {};
+    long long one_wave(int flags)
+    {
+        long long w = wave[flags].load(std::memory_order_relaxed);
+        if (w < 0) {
+            w = g_class_resident[cls](flags);
+            wave[flags].store(w, std::memory_order_relaxed);
+        }
+        return w;
+    }
 
     pfk_status fail(pfk_status s, const std::string &msg)
     {
@@ -2034,19 +2059,23 @@ pfk_status pfk_eri_batch_set_quartets(pfk_eri_batch *ctx, const int *quartets, l
     PFK_CK(cudaStreamSynchronize(ctx->stream));
     ctx->d_sorted.release();
     ctx->d_pos.release();
+    for (auto &w : ctx->wave) w.store(-1, std::memory_order_relaxed);
     if (n <= INT32_MAX) {
         try {
+            // (longest first, place) as one key: at most 64^4 primitive quartets
+            std::vector<unsigned long long> key((size_t)n);
+            for (long long t = 0; t < n; ++t)
+                key[t] = (unsigned long long)(0xffffffffu - (unsigned)ctx->pair_nprim[q[t].x] *
+                                                                (unsigned)ctx->pair_nprim[q[t].y]) << 32 |
+                         (unsigned long long)t;
+            for (long long w = 0; w < n; w += kBatchWindow)
+                std::sort(key.begin() + w, key.begin() + std::min(n, w + kBatchWindow));
             std::vector<int> pos((size_t)n);
-            std::vector<unsigned> len((size_t)n);
             std::vector<uint2> sorted((size_t)n);
             for (long long t = 0; t < n; ++t) {
-                pos[t] = (int)t;
-                len[t] = (unsigned)ctx->pair_nprim[q[t].x] * (unsigned)ctx->pair_nprim[q[t].y];
+                pos[t] = (int)(key[t] & 0xffffffffu);
+                sorted[t] = q[pos[t]];
             }
-            for (long long w = 0; w < n; w += kBatchWindow)
-                std::stable_sort(pos.begin() + w, pos.begin() + std::min(n, w + kBatchWindow),
-                                 [&](int a, int b) { return len[a] > len[b]; });
-            for (long long t = 0; t < n; ++t) sorted[t] = q[pos[t]];
             PFK_CK(ctx->d_sorted.alloc((size_t)n));
             PFK_CK(ctx->d_pos.alloc((size_t)n));
             PFK_CK(cudaMemcpyAsync(ctx->d_sorted.p, sorted.data(), sizeof(uint2) * n, cudaMemcpyHostToDevice,
@@ -2092,12 +2121,15 @@ pfk_status pfk_eri_batch_run(pfk_eri_batch *ctx, long long first, long long coun
     a.nb = 0;
     a.qstride = 1;
     a.qoffset = 0;
-    const int flags = (engine == PFK_ENGINE_OS ? kLaunchOS : 0) | (precision == PFK_PREC_MIXED ? kLaunchFP32 : 0);
-    // whole windows of the range run in their sorted order, the ends as listed
+    int flags = (engine == PFK_ENGINE_OS ? kLaunchOS : 0) | (precision == PFK_PREC_MIXED ? kLaunchFP32 : 0);
+    const bool few = count <= ctx->one_wave(flags | kLaunchShort);
+    if (few) flags |= kLaunchShort;
+    // above a wave, whole windows of the range run in their sorted order, the ends as listed
+    const bool windows = !few && count > ctx->one_wave(flags) && ctx->d_sorted.p;
     const long long end = first + count;
     long long w0 = (first + kBatchWindow - 1) / kBatchWindow * kBatchWindow;
     long long w1 = end == ctx->nq ? end : end / kBatchWindow * kBatchWindow;
-    if (!ctx->d_sorted.p || w0 >= w1) w0 = w1 = end;
+    if (!windows || w0 >= w1) w0 = w1 = end;
     if (w0 > first) g_class_launchers[ctx->cls](ctx->d_quart.p + first, w0 - first, a, 1, flags, st);
     if (end > w1) {
         a.blk_out = d_out + (size_t)(w1 - first) * ctx->ncomp;

@@ -59,6 +59,69 @@ void launch_segments(const uint2 *q, long long n, const JKArgs &a, int per, Spli
     }
 }
 
+// The build that the tensor and block modes take (one-lane form).
+struct OutBuild {
+    void (*kernel)(const uint2 *, long long, JKArgs);
+    int threads;
+    size_t smem;
+    int per;   // quartets per block
+};
+// the plain Obara-Saika build: left alone the compiler takes 94 registers at
+// L = 1 and 190 at L = 3 to have more of the Boys polynomials in flight, at 5
+// and 2 blocks per SM.  In FP32 L = 3 needs 123 registers: 4 blocks.
+template <int L, typename R>
+constexpr int kOSBlocks = L == 0 ? 8 : L == 1 ? 6 : L == 2 ? 5 : L == 3 ? (sizeof(R) == 4 ? 4 : 3) : 1;
+
+template <int LA, int LB, int LC, int LD>
+OutBuild out_build(int flags)
+{
+    using S = ClassShape<LA, LB, LC, LD>;
+    using SS = SplitShape<LA, LB, LC, LD>;
+    const bool fp32 = flags & kLaunchFP32, few = flags & kLaunchShort;
+    constexpr int L = LA + LB + LC + LD;
+    if constexpr (L <= kOSMaxL) {
+        if (flags & kLaunchOS)
+            return {fp32 ? &eri_os_kernel<LA, LB, LC, LD, 1, float, kOSBlocks<L, float>, false, true>
+                         : &eri_os_kernel<LA, LB, LC, LD, 1, double, kOSBlocks<L, double>, false, true>,
+                    128, 0, 128};
+    }
+    if constexpr (S::N <= kRegMaxComponents) {
+        if (fp32)
+            return {few ? &eri_reg_kernel<LA, LB, LC, LD, 1, float, true, RegShape<LA, LB, LC, LD, float>::MINB_SHORT>
+                        : &eri_reg_kernel<LA, LB, LC, LD, 1, float, true>,
+                    128, 0, 128};
+        return {&eri_reg_kernel<LA, LB, LC, LD, 1, double, true>, 128, 0, 128};
+    } else if constexpr (SS::OK) {
+        using SF = SplitShape<LA, LB, LC, LD, float>;
+        if (fp32)
+            return {few ? &eri_split_kernel<LA, LB, LC, LD, 1, float, false, true, SF::MINB_SHORT>
+                        : &eri_split_kernel<LA, LB, LC, LD, 1, float, false, true>,
+                    128, SF::SMEM, SF::TEAMS};
+        return {few ? &eri_split_kernel<LA, LB, LC, LD, 1, double, false, true, SS::MINB_SHORT>
+                    : &eri_split_kernel<LA, LB, LC, LD, 1, double, false, true>,
+                128, SS::SMEM, SS::TEAMS};
+    } else {
+        using TS = TeamShape<LA, LB, LC, LD>;
+        using TF = TeamShape<LA, LB, LC, LD, float>;
+        if (fp32) return {&eri_team_kernel<LA, LB, LC, LD, 1, float>, TF::BLOCK, TF::SMEM, TF::TEAMS};
+        return {&eri_team_kernel<LA, LB, LC, LD, 1>, TS::BLOCK, TS::SMEM, TS::TEAMS};
+    }
+}
+
+template <int LA, int LB, int LC, int LD>
+long long resident_quartets(int flags)
+{
+    const OutBuild o = out_build<LA, LB, LC, LD>(flags);
+    int dev = 0, sms = 0, blocks = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, o.kernel, o.threads, o.smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return (long long)blocks * sms * o.per;
+}
+
 template <int LA, int LB, int LC, int LD>
 void launch_class(const uint2 *q, long long n, const JKArgs &args, int nk, int flags, cudaStream_t st)
 {
@@ -66,7 +129,7 @@ void launch_class(const uint2 *q, long long n, const JKArgs &args, int nk, int f
     using SS = SplitShape<LA, LB, LC, LD>;
     using TS = TeamShape<LA, LB, LC, LD>;
     const int fp32 = flags & kLaunchFP32;
-    const bool out = args.blk_out || args.eri_out;   // tensor and block modes: the OUT builds, one density
+    const bool out = args.blk_out || args.eri_out;   // tensor and block modes: out_build, one density
     JKArgs a = args;
     if (out && fp32) a.seg.n = 0;                    // their FP32 builds have no SPLIT form
     if constexpr (LA + LB + LC + LD <= kOSMaxL) {
@@ -80,10 +143,7 @@ void launch_class(const uint2 *q, long long n, const JKArgs &args, int nk, int f
             // whichever build is faster on the molecule's lists.
             constexpr int L = LA + LB + LC + LD;
             constexpr int MB = L <= 1 ? 8 : L == 2 ? 6 : 4;
-            // the plain build: left alone the compiler takes 94 registers at
-            // L = 1 and 190 at L = 3 to have more of the Boys polynomials in
-            // flight, at 5 and 2 blocks per SM
-            constexpr int PB = L == 0 ? 8 : L == 1 ? 6 : L == 2 ? 5 : L == 3 ? 3 : 1;
+            constexpr int PB = kOSBlocks<L, double>, PF = kOSBlocks<L, float>;
             launch_segments(
                 q, n, a, 128,
                 [&](const JKArgs &b, unsigned grid) {
@@ -93,11 +153,10 @@ void launch_class(const uint2 *q, long long n, const JKArgs &args, int nk, int f
                     else eri_os_kernel<LA, LB, LC, LD, 1, double, 1, true><<<grid, 128, 0, st>>>(q, n, b);
                 },
                 [&](const uint2 *r, long long m, unsigned grid) {
-                    if (out && fp32) eri_os_kernel<LA, LB, LC, LD, 1, float, PB, false, true><<<grid, 128, 0, st>>>(r, m, a);
-                    else if (out) eri_os_kernel<LA, LB, LC, LD, 1, double, PB, false, true><<<grid, 128, 0, st>>>(r, m, a);
+                    if (out) out_build<LA, LB, LC, LD>(flags).kernel<<<grid, 128, 0, st>>>(r, m, a);
                     else if (nk == 2) eri_os_kernel<LA, LB, LC, LD, 2, double, PB><<<grid, 128, 0, st>>>(r, m, a);
                     else if (fp32 && dense) eri_os_kernel<LA, LB, LC, LD, 1, float, MB><<<grid, 128, 0, st>>>(r, m, a);
-                    else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float, PB><<<grid, 128, 0, st>>>(r, m, a);
+                    else if (fp32) eri_os_kernel<LA, LB, LC, LD, 1, float, PF><<<grid, 128, 0, st>>>(r, m, a);
                     else if (dense) eri_os_kernel<LA, LB, LC, LD, 1, double, MB><<<grid, 128, 0, st>>>(r, m, a);
                     else eri_os_kernel<LA, LB, LC, LD, 1, double, PB><<<grid, 128, 0, st>>>(r, m, a);
                 });
@@ -107,8 +166,7 @@ void launch_class(const uint2 *q, long long n, const JKArgs &args, int nk, int f
     if constexpr (S::N <= kRegMaxComponents) {
         if (n <= 0) return;
         const long long grid = (n + 127) / 128;
-        if (out && fp32) eri_reg_kernel<LA, LB, LC, LD, 1, float, true><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
-        else if (out) eri_reg_kernel<LA, LB, LC, LD, 1, double, true><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
+        if (out) out_build<LA, LB, LC, LD>(flags).kernel<<<(unsigned)grid, 128, 0, st>>>(q, n, a);
         else if (nk == 2) eri_reg_kernel<LA, LB, LC, LD, 2><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
         else if (fp32) eri_reg_kernel<LA, LB, LC, LD, 1, float><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
         else eri_reg_kernel<LA, LB, LC, LD, 1><<<(unsigned)grid, 128, 0, st>>>(q, n, a);
@@ -119,10 +177,10 @@ void launch_class(const uint2 *q, long long n, const JKArgs &args, int nk, int f
             cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS::SMEM);
             cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)SF::SMEM);
-            cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, double, false, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS::SMEM);
-            cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, float, false, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SF::SMEM);
+            for (int f : {0, kLaunchShort, (int)kLaunchFP32, kLaunchFP32 | kLaunchShort}) {
+                const OutBuild o = out_build<LA, LB, LC, LD>(f);
+                cudaFuncSetAttribute(o.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o.smem);
+            }
             if constexpr (kSplitTeams<LA>) {
                 cudaFuncSetAttribute(eri_split_kernel<LA, LB, LC, LD, 1, double, true, true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SS::SMEM_SPLIT);
@@ -137,10 +195,10 @@ void launch_class(const uint2 *q, long long n, const JKArgs &args, int nk, int f
         }
         if (n == 0) return;
         const auto plain = [&](const uint2 *r, long long m, unsigned grid) {
-            if (out && fp32)
-                eri_split_kernel<LA, LB, LC, LD, 1, float, false, true><<<grid, 128, SF::SMEM, st>>>(r, m, a);
-            else if (out) eri_split_kernel<LA, LB, LC, LD, 1, double, false, true><<<grid, 128, SS::SMEM, st>>>(r, m, a);
-            else if (nk == 2) eri_split_kernel<LA, LB, LC, LD, 2><<<grid, 128, SS::SMEM, st>>>(r, m, a);
+            if (out) {
+                const OutBuild o = out_build<LA, LB, LC, LD>(flags);
+                o.kernel<<<grid, 128, o.smem, st>>>(r, m, a);
+            } else if (nk == 2) eri_split_kernel<LA, LB, LC, LD, 2><<<grid, 128, SS::SMEM, st>>>(r, m, a);
             else if (fp32) eri_split_kernel<LA, LB, LC, LD, 1, float><<<grid, 128, SF::SMEM, st>>>(r, m, a);
             else eri_split_kernel<LA, LB, LC, LD, 1><<<grid, 128, SS::SMEM, st>>>(r, m, a);
         };
@@ -184,16 +242,17 @@ constexpr int cls_bra(int c)
 constexpr int cls_ket(int c) { return c - cls_bra(c) * (cls_bra(c) + 1) / 2; }
 
 template <int C>
-void reg_range(ClassLauncher *table)
+void reg_range()
 {
     constexpr int X = cls_bra(C), Y = cls_ket(C);
-    table[C] = &launch_class<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
-    if constexpr (C + 1 < PFK_CLASS_END) reg_range<C + 1>(table);
+    g_class_launchers[C] = &launch_class<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
+    g_class_resident[C] = &resident_quartets<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
+    if constexpr (C + 1 < PFK_CLASS_END) reg_range<C + 1>();
 }
 
 // Runs at library load: puts this unit's launchers into the shared table.
 struct Registrar {
-    Registrar() { reg_range<PFK_CLASS_BEGIN>(g_class_launchers); }
+    Registrar() { reg_range<PFK_CLASS_BEGIN>(); }
 };
 const Registrar registrar;
 

@@ -30,8 +30,9 @@ __host__ __device__ constexpr int quartet_class_L(int c)
 // FP64).  kLaunchOS asks for the Obara-Saika kernel, which exists
 // for classes with LA+LB+LC+LD <= kOSMaxL; the other classes run Rys.
 // kLaunchDense picks the Obara-Saika kernel compiled for 4 blocks of 128
-// per SM (single exchange density only).
-constexpr int kLaunchFP32 = 1, kLaunchOS = 2, kLaunchDense = 4;
+// per SM (single exchange density only).  kLaunchShort, in block mode, picks
+// the build for launches of at most one wave (MINB_SHORT).
+constexpr int kLaunchFP32 = 1, kLaunchOS = 2, kLaunchDense = 4, kLaunchShort = 8;
 constexpr int kOSMaxL = 4;
 
 // One launcher per quartet class.  nk = number of exchange densities (1 or 2).
@@ -42,6 +43,11 @@ using ClassLauncher = void (*)(const uint2 *quartets, long long n, const JKArgs 
 // units (each compiled for a range of classes).  A launcher called with
 // n < 0 only configures the current device for its kernels.
 extern ClassLauncher g_class_launchers[kQuartetClasses];
+
+// How many quartets of each class the current device works on at once (one
+// wave) in the build that block mode takes for these flags; 0 on an error.
+using ClassResident = long long (*)(int flags);
+extern ClassResident g_class_resident[kQuartetClasses];
 
 // Context internals for the other units: its CUDA device, and recording a
 // failure message (returns s).

@@ -368,9 +368,20 @@ __device__ __forceinline__ PrimSplit prim_split(const LaneWork &w, int nket)
 // product and the contraction: double, or float for the mixed-precision list
 // of quartets whose Schwarz bound is below the FP32 threshold.  Roots,
 // weights and the per-primitive-quartet scalars stay FP64 in both, and so
-// does the J/K digestion and accumulation.
-template <int LA, int LB, int LC, int LD, int NK, typename R = double, bool OUT = false>
-__global__ void __launch_bounds__(128) eri_reg_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
+// does the J/K digestion and accumulation.  MB: blocks of 128 per SM the
+// register allocation must allow (0: the compiler's choice).
+//
+// RegShape::MINB_SHORT: the same for block-mode launches of at most one wave.
+// The FP32 builds of 30 to 36 components come out at 128 registers, which is
+// right for several waves and costs a single one (512 (dd|ss) blocks 6%, (fs|ps)
+// 8%, (fp|ss) 5% slower than at 168; 65536 of them 22 to 28% faster).
+template <int LA, int LB, int LC, int LD, typename R>
+struct RegShape {
+    static constexpr int N = ClassShape<LA, LB, LC, LD>::N;
+    static constexpr int MINB_SHORT = sizeof(R) == 4 && N >= 30 && N <= 36 ? 3 : 0;
+};
+template <int LA, int LB, int LC, int LD, int NK, typename R = double, bool OUT = false, int MB = 0>
+__global__ void __launch_bounds__(128, MB) eri_reg_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
 {
     using S = ClassShape<LA, LB, LC, LD>;
     constexpr int NA = S::NA, NB = S::NB, NC = S::NC, ND = S::ND, NR = S::NR, NI = S::NI;
@@ -728,9 +739,18 @@ struct SplitShape {
     // wait on loads more than on arithmetic, so four where the accumulators
     // leave room: (H2O)32 (dd|ps) 1.57 -> 1.43 ms, (dd|dp) 1.19 -> 1.01 (both
     // M = 18); at M = 27 the spills cost more ((dp|pp) 3.42 -> 3.70).  With 54
-    // accumulators three blocks spill 900 to 1300 bytes into the inner loop,
-    // two none: 16384 (fd|pp) blocks 4.00 -> 3.33 ms
-    static constexpr int MINB = M <= 18 ? 4 : M <= 36 ? 3 : 2;
+    // FP64 accumulators three blocks spill 900 to 1300 bytes into the inner
+    // loop, two none: 16384 (fd|pp) blocks 4.00 -> 3.33 ms.  In FP32 three
+    // spill 360 and are the faster build of long lists (16384 (dp|dp) blocks
+    // 11%, (fd|pp) 16%); short ones gain 7% from two.
+    static constexpr int MINB = M <= 18 ? 4 : M <= 36 || sizeof(R) == 4 ? 3 : 2;
+    // the SPLIT builds (lists far below one wave)
+    static constexpr int MINB_SPLIT = M <= 18 ? 4 : M <= 36 ? 3 : 2;
+    // block-mode launches of at most one wave, which lasts as long as its
+    // longest quartet: no spills count, blocks per SM do not.  512 quartets
+    // at 4 blocks per SM instead of 3: (dd|dp) 13%, (fs|dp) 8%, (dd|ps) 7%
+    // slower; 65536: 3 to 22% faster
+    static constexpr int MINB_SHORT = M <= 18 ? 3 : M <= 27 || (M <= 36 && sizeof(R) == 4) ? 3 : 2;
 };
 
 template <int TEAM>
@@ -772,8 +792,9 @@ __device__ __forceinline__ int cart_l_axis(int i, int axis)
 // series and recurrences to a team, however idle the chip) and the first of
 // them adds up the others' blocks and digests.  One water / 6-31G** (dp|pp),
 // 27 primitive quartets: 66 -> 28 us; the build 149 -> 126 us.
-template <int LA, int LB, int LC, int LD, int NK, typename R = double, bool SPLIT = false, bool OUT = false>
-__global__ void __launch_bounds__(128, (SplitShape<LA, LB, LC, LD, R>::MINB)) eri_split_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
+template <int LA, int LB, int LC, int LD, int NK, typename R = double, bool SPLIT = false, bool OUT = false,
+          int MB = SPLIT ? SplitShape<LA, LB, LC, LD, R>::MINB_SPLIT : SplitShape<LA, LB, LC, LD, R>::MINB>
+__global__ void __launch_bounds__(128, MB) eri_split_kernel(const uint2 *__restrict__ quartets, long long nq, JKArgs args)
 {
     using S = ClassShape<LA, LB, LC, LD>;
     using SS = SplitShape<LA, LB, LC, LD, R>;
