@@ -90,6 +90,7 @@ struct pfk_ctx {
     // build's stream (fork_ev) and joined back (join_ev) around the classes
     int lanes = 0;                    // 0: by the size of the lists (auto_lanes)
     int auto_lanes = kMaxLanes;       // set by build_lists
+    bool built = false;               // a build outside a capture has been launched
     int nside = 0;                    // side streams created so far
     cudaStream_t side[kSmallLanes - 1] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[kSmallLanes - 1] = {};
@@ -123,6 +124,10 @@ struct pfk_ctx {
     DevBuf<int> d_cls_ids[kPairClasses];
     DevBuf<double> d_cls_q[kPairClasses];
     DevBuf<long long> d_cls_kpref[kPairClasses];   // prefix of nprim over the sorted class list
+    // every class's pairs in ket order (tiles of basis functions), as (pair
+    // id, rank by bound); class x starts at ket_off[x]
+    DevBuf<uint2> d_kets;
+    size_t ket_off[kPairClasses] = {};
 
     long long prim_cnt[kQuartetClasses] = {};   // primitive quartets (all primitives), per class
     long long prim32_cnt[kQuartetClasses] = {}; // the part of prim_cnt on the FP32 list
@@ -340,8 +345,13 @@ cudaError_t side_streams(pfk_ctx *ctx, int n)
 {
     for (; ctx->nside < n; ++ctx->nside) {
         cudaError_t e = cudaStreamCreateWithFlags(&ctx->side[ctx->nside], cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->join_ev[ctx->nside], cudaEventDisableTiming);
         if (e != cudaSuccess) return e;
+        e = cudaEventCreateWithFlags(&ctx->join_ev[ctx->nside], cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+            cudaStreamDestroy(ctx->side[ctx->nside]);
+            ctx->side[ctx->nside] = nullptr;
+            return e;
+        }
     }
     return cudaSuccess;
 }
@@ -402,7 +412,6 @@ pfk_status make_lists(pfk_ctx *ctx)
         pos += ctx->q32_cnt[c];
     }
     ctx->auto_lanes = total <= kSmallQuartets ? kSmallLanes : kMaxLanes;
-    PFK_CK(side_streams(ctx, ctx->auto_lanes - 1));
     PFK_CK(ctx->d_quart.alloc((size_t)std::max(total, 1LL)));
     // pass 2: fill
     for (int x = 0; x < kPairClasses; ++x)
@@ -416,8 +425,8 @@ pfk_status make_lists(pfk_ctx *ctx)
             PFK_CK(exclusive_scan(cnt_hi.p, off_hi.p, nX, tmp.p, tb, ctx->stream));
             tb = tmp_bytes;
             PFK_CK(exclusive_scan(cnt_lo.p, off_lo.p, nX, tmp.p, tb, ctx->stream));
-            PFK_CK(fill_quartets(ctx->d_cls_ids[x].p, nX, ctx->d_cls_ids[y].p, x == y, off_hi.p, cnt_hi.p, off_lo.p,
-                                 cnt_lo.p, ctx->d_quart.p + ctx->q_off[cls], ctx->d_quart.p + ctx->q32_off[cls],
+            PFK_CK(fill_quartets(ctx->d_cls_ids[x].p, nX, ctx->d_kets.p + ctx->ket_off[y], nY, x == y, off_hi.p,
+                                 cnt_hi.p, off_lo.p, cnt_lo.p, ctx->d_quart.p + ctx->q_off[cls], ctx->d_quart.p + ctx->q32_off[cls],
                                  ctx->stream));
             PFK_CK(bra_work(ctx->d_cls_ids[x].p, nX, x == y, cnt_hi.p, cnt_lo.p, ctx->d_cls_kpref[y].p,
                             ctx->d_pairs.p, work_hi.p, work_lo.p, ctx->stream));
@@ -431,7 +440,7 @@ pfk_status make_lists(pfk_ctx *ctx)
             ctx->prim_cnt[cls] = w;
             ctx->prim32_cnt[cls] = w32;
         }
-    // order each list by its primitive loop lengths (stable: bra-major within a key)
+    // order each list by its primitive loop lengths (stable: the fill's order within a key)
     long long maxseg = 1;
     for (int c = 0; c < kQuartetClasses; ++c) maxseg = std::max(maxseg, std::max(ctx->q_cnt[c], ctx->q32_cnt[c]));
     {
@@ -440,62 +449,29 @@ pfk_status make_lists(pfk_ctx *ctx)
         PFK_CK(ka.alloc(maxseg));
         PFK_CK(kb.alloc(maxseg));
         PFK_CK(vb.alloc(maxseg));
-        // Each bra's kets in tiles of kKetTile x kKetTile functions (k, l): a
-        // warp's kets then share or neighbour their rows and columns, so that
-        // the density blocks it reads and the sums it adds to lie in a few
-        // cache lines, and the primitive data too.  In the order of the
-        // Schwarz bounds that the lists are made in, every lane's k and l are
-        // unrelated.  C40H82 / cc-pVDZ 242.6 -> 223.5 ms a build, (H2O)32 47.7
-        // -> 46.0; plain (k, l) order 226.0 and 46.6 (whole warps add to one
-        // K(i, k)), tiles of 8 225.2 and 46.5.  Bras stay in the order of
-        // their bounds: by pair they were slower.
-        constexpr unsigned kKetTile = 32;
-        // rank of every pair in its class, as a bra (by bound) and as a ket (by tile)
-        std::vector<unsigned> rank(2 * (size_t)ctx->npairs);
-        std::vector<std::pair<unsigned long long, int>> tiles;
-        for (const std::vector<int> &ids : ctx->cls_ids) {
-            tiles.clear();
-            for (size_t i = 0; i < ids.size(); ++i) {
-                const unsigned long long a = ctx->pairs[ids[i]].bf_a, b = ctx->pairs[ids[i]].bf_b;
-                rank[ids[i]] = (unsigned)i;
-                tiles.push_back({(a / kKetTile) << 48 | (b / kKetTile) << 32 | a << 16 | b, ids[i]});
-            }
-            std::sort(tiles.begin(), tiles.end());
-            for (size_t i = 0; i < tiles.size(); ++i) rank[(size_t)ctx->npairs + tiles[i].second] = (unsigned)i;
-        }
-        auto bits = [](size_t n) {   // of the numbers 0 .. n - 1
-            int k = 1;
-            while (k < 32 && (size_t(1) << k) < n) ++k;
-            return k;
-        };
         int most_prims = 1;
         for (const PairInfo &p : ctx->pairs) most_prims = std::max(most_prims, p.nprim);
-        DevBuf<unsigned> d_rank;
-        PFK_CK(d_rank.alloc(rank.size()));
-        PFK_CK(cudaMemcpyAsync(d_rank.p, rank.data(), sizeof(unsigned) * rank.size(), cudaMemcpyHostToDevice, ctx->stream));
-        SortKeys keys{d_rank.p, d_rank.p + ctx->npairs, 1, 1, bits((size_t)most_prims + 1)};
+        int prim_bits = 1;
+        while (1 << prim_bits <= most_prims) ++prim_bits;
         size_t sort_bytes = 0;
-        PFK_CK(sort_quartets(ctx->d_quart.p, maxseg, ctx->d_pairs.p, keys, ka.p, kb.p, vb.p, nullptr, sort_bytes, ctx->stream));
+        PFK_CK(sort_quartets(ctx->d_quart.p, maxseg, ctx->d_pairs.p, prim_bits, ka.p, kb.p, vb.p, nullptr, sort_bytes, ctx->stream));
         DevBuf<char> st;
         PFK_CK(st.alloc(sort_bytes + 16));
         DevBuf<long long> starts;
-        PFK_CK(starts.alloc(2 * kQuartetClasses * kLengthBuckets));
+        PFK_CK(starts.alloc(kLists * kLengthBuckets));
         PFK_CK(cudaMemsetAsync(starts.p, 0xff, sizeof(long long) * starts.n, ctx->stream));   // -1
+        ListStarts lists;
         for (int c = 0; c < kQuartetClasses; ++c) {
             size_t b1 = sort_bytes, b2 = sort_bytes;
-            int x = 0;
-            while ((x + 1) * (x + 2) / 2 <= c) ++x;
-            keys.bra_bits = bits(ctx->cls_ids[x].size());
-            keys.ket_bits = bits(ctx->cls_ids[c - x * (x + 1) / 2].size());
-            PFK_CK(sort_quartets(ctx->d_quart.p + ctx->q_off[c], ctx->q_cnt[c], ctx->d_pairs.p, keys, ka.p, kb.p, vb.p, st.p,
-                                 b1, ctx->stream));
-            PFK_CK(sort_quartets(ctx->d_quart.p + ctx->q32_off[c], ctx->q32_cnt[c], ctx->d_pairs.p, keys, ka.p, kb.p, vb.p,
-                                 st.p, b2, ctx->stream));
-            PFK_CK(bucket_starts(ctx->d_quart.p + ctx->q_off[c], ctx->q_cnt[c], ctx->d_pairs.p,
-                                 starts.p + (size_t)(2 * c) * kLengthBuckets, ctx->stream));
-            PFK_CK(bucket_starts(ctx->d_quart.p + ctx->q32_off[c], ctx->q32_cnt[c], ctx->d_pairs.p,
-                                 starts.p + (size_t)(2 * c + 1) * kLengthBuckets, ctx->stream));
+            PFK_CK(sort_quartets(ctx->d_quart.p + ctx->q_off[c], ctx->q_cnt[c], ctx->d_pairs.p, prim_bits, ka.p, kb.p,
+                                 vb.p, st.p, b1, ctx->stream));
+            PFK_CK(sort_quartets(ctx->d_quart.p + ctx->q32_off[c], ctx->q32_cnt[c], ctx->d_pairs.p, prim_bits, ka.p,
+                                 kb.p, vb.p, st.p, b2, ctx->stream));
+            lists.first[2 * c] = ctx->q_off[c];
+            lists.first[2 * c + 1] = ctx->q32_off[c];
         }
+        lists.first[kLists] = total;
+        PFK_CK(bucket_starts(ctx->d_quart.p, ctx->d_pairs.p, lists, starts.p, ctx->stream));
         ctx->bucket0.resize(starts.n);
         PFK_CK(cudaMemcpyAsync(ctx->bucket0.data(), starts.p, sizeof(long long) * starts.n, cudaMemcpyDeviceToHost,
                                ctx->stream));
@@ -525,6 +501,38 @@ pfk_status need_lists(pfk_ctx *ctx)
 {
     return ctx->lists_ok ? PFK_OK
                          : ctx->fail(PFK_ERR_STATE, "no quartet lists (their last build failed): call pfk_set_options again");
+}
+
+// Appends one class's pairs (ids, in the order of their bounds) to kets in ket
+// order: tiles of 32 x 32 functions (k, l), by (k, l) in a tile.  A
+// warp's kets then share or neighbour their rows and columns, so that the
+// density blocks it reads and the sums it adds to lie in a few cache lines,
+// and the primitive data too.  In the order of the Schwarz bounds every
+// lane's k and l are unrelated.  C40H82 / cc-pVDZ 242.6 -> 223.5 ms a build,
+// (H2O)32 47.7 -> 46.0; plain (k, l) order 226.0 and 46.6 (whole warps add to
+// one K(i, k)), tiles of 8 225.2 and 46.5.  Bras stay in the order of their
+// bounds: by pair they were slower.  rank: scratch of npairs.
+void append_kets(const pfk_ctx *ctx, const std::vector<int> &ids, std::vector<unsigned> &rank, std::vector<uint2> &kets)
+{
+    constexpr int kTileBits = 5;   // tiles of 32; functions are numbered in 16 bits
+    // (k tile, l tile, k, l in the tile) above the pair id
+    std::vector<unsigned long long> key(ids.size()), tmp(ids.size());
+    for (size_t i = 0; i < ids.size(); ++i) {
+        const PairInfo &p = ctx->pairs[ids[i]];
+        const unsigned a = (unsigned)p.bf_a, b = (unsigned)p.bf_b, low = (1u << kTileBits) - 1u;
+        const unsigned place = (a >> kTileBits) << (16 + kTileBits) | (b >> kTileBits) << (2 * kTileBits) |
+                               (a & low) << kTileBits | (b & low);
+        key[i] = (unsigned long long)place << 32 | (unsigned)ids[i];
+        rank[ids[i]] = (unsigned)i;
+    }
+    for (int shift = 32; shift < 64; shift += 8) {   // stable counting sorts by the key's bytes
+        size_t at[257] = {};
+        for (unsigned long long k : key) ++at[(k >> shift & 255) + 1];
+        for (int d = 0; d < 256; ++d) at[d + 1] += at[d];
+        for (unsigned long long k : key) tmp[at[k >> shift & 255]++] = k;
+        key.swap(tmp);
+    }
+    for (unsigned long long k : key) kets.push_back(make_uint2((unsigned)k, rank[(unsigned)k]));
 }
 
 pfk_status schwarz_and_sort(pfk_ctx *ctx)
@@ -565,10 +573,15 @@ pfk_status schwarz_and_sort(pfk_ctx *ctx)
     if (s != PFK_OK) return s;
     // per-class lists sorted by qmax, descending (ties by pair index)
     for (int p = 0; p < ctx->npairs; ++p) ids[ctx->pair_pc[p]].push_back(p);
+    std::vector<uint2> kets;
+    std::vector<unsigned> rank((size_t)ctx->npairs);
+    kets.reserve((size_t)ctx->npairs);
     for (int x = 0; x < kPairClasses; ++x) {
         auto &v = ids[x];
         std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return ctx->pairs[a].qmax > ctx->pairs[b].qmax; });
         ctx->cls_ids[x] = v;
+        ctx->ket_off[x] = kets.size();
+        append_kets(ctx, v, rank, kets);
         std::vector<double> q(v.size());
         for (size_t i = 0; i < v.size(); ++i) q[i] = ctx->pairs[v[i]].qmax;
         if (v.empty()) continue;
@@ -583,6 +596,9 @@ pfk_status schwarz_and_sort(pfk_ctx *ctx)
                                ctx->stream));
         PFK_CK(cudaStreamSynchronize(ctx->stream));
     }
+    PFK_CK(ctx->d_kets.alloc(kets.size()));
+    PFK_CK(cudaMemcpyAsync(ctx->d_kets.p, kets.data(), sizeof(uint2) * kets.size(), cudaMemcpyHostToDevice, ctx->stream));
+    PFK_CK(cudaStreamSynchronize(ctx->stream));
     return PFK_OK;
 }
 
@@ -670,6 +686,29 @@ void list_segments(const pfk_ctx *ctx, const long long *bucket0, long long n, in
     }
 }
 
+// The graph nodes that the next node captured on a stream would depend on.
+// What comes in order has one; only the place where a caller's capture joins
+// branches of its own would have more.
+struct LaneEnds {
+    static constexpr size_t kMost = 8;
+    cudaGraphNode_t node[kMost];
+    size_t n = 0;
+    cudaError_t read(cudaStream_t st)
+    {
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t *deps = nullptr;
+        const cudaError_t e = cudaStreamGetCaptureInfo_v2(st, &status, nullptr, nullptr, &deps, &n);
+        if (e != cudaSuccess) return e;
+        if (n > kMost) return cudaErrorNotSupported;
+        std::copy(deps, deps + n, node);
+        return cudaSuccess;
+    }
+    cudaError_t set(cudaStream_t st, unsigned how = cudaStreamSetCaptureDependencies)
+    {
+        return cudaStreamUpdateCaptureDependencies(st, node, n, how);
+    }
+};
+
 // Launch every class kernel over the screened lists.  Jacc/K accumulators are
 // zeroed first.  eri_out selects the dense-tensor mode.
 pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const double *Pk1, int nk, FxWord *Jacc,
@@ -715,10 +754,29 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
         PFK_CK(cudaEventCreate(&ev[1]));
     }
     // lanes: the classes go, largest estimated cost first, to the lane with
-    // the least work so far; a per-class timed pass stays on one stream
-    const int nlanes = timed ? 1 : ctx->lanes ? ctx->lanes : ctx->auto_lanes;
+    // the least work so far; a per-class timed pass stays on one stream.  A
+    // captured build needs no streams for them: before each class its lane's
+    // last node becomes what the next node depends on.  A build outside a
+    // capture forks to side streams; those beyond kMaxLanes cost 50 us each to
+    // create and again to destroy (0.8 ms together, the gain of a few builds),
+    // so a context's first such build does without them.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PFK_CK(cudaStreamIsCapturing(st, &capture));
+    const bool captured = capture == cudaStreamCaptureStatusActive;
+    int nlanes = timed ? 1 : ctx->lanes ? ctx->lanes : ctx->auto_lanes;
+    if (!captured && !timed) {
+        if (!ctx->built) nlanes = std::min(nlanes, kMaxLanes);
+        ctx->built = true;
+        PFK_CK(side_streams(ctx, nlanes - 1));
+    }
+    LaneEnds ends[kSmallLanes + 1];   // of a captured build: where the lanes fork, then each lane's end
+    if (captured && nlanes > 1) {
+        PFK_CK(ends[nlanes].read(st));
+        for (int i = 0; i < nlanes; ++i) ends[i] = ends[nlanes];
+    }
     cudaStream_t lane_st[kSmallLanes] = {st};
-    if (nlanes > 1) {
+    for (int i = 1; i < nlanes; ++i) lane_st[i] = st;
+    if (nlanes > 1 && !captured) {
         PFK_CK(cudaEventRecord(ctx->fork_ev, st));
         for (int i = 1; i < nlanes; ++i) {
             lane_st[i] = ctx->side[i - 1];
@@ -744,7 +802,8 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
         int ln = 0;
         for (int i = 1; i < nlanes; ++i)
             if (load[i] < load[ln]) ln = i;
-        load[ln] += cost[c];
+        load[ln] += cost[c];   // positive: every listed quartet has primitives
+        if (captured && nlanes > 1) PFK_CK(ends[ln].set(st));
         if (nh) {
             list_segments(ctx, ctx->bucket0.data() + (size_t)(2 * c) * kLengthBuckets, ctx->q_cnt[c],
                           class_team(c), a.seg);
@@ -756,6 +815,7 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
             ctx->launch[c](ctx->d_quart.p + ctx->q32_off[c], nl, a, nk, os | fp32, lane_st[ln]);
         }
         PFK_CK(cudaGetLastError());
+        if (captured && nlanes > 1) PFK_CK(ends[ln].read(st));
         if (timed) {
             PFK_CK(cudaEventRecord(ev[1], st));
             PFK_CK(cudaEventSynchronize(ev[1]));
@@ -768,6 +828,15 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
         cudaEventDestroy(ev[0]);
         cudaEventDestroy(ev[1]);
     }
+    if (captured && nlanes > 1) {   // what follows depends on the end of every lane with work
+        bool first = true;
+        for (int i = 0; i < nlanes; ++i) {
+            if (load[i] == 0.0) continue;
+            PFK_CK(ends[i].set(st, first ? cudaStreamSetCaptureDependencies : cudaStreamAddCaptureDependencies));
+            first = false;
+        }
+    }
+    if (captured) return PFK_OK;
     for (int i = 1; i < nlanes; ++i) {
         PFK_CK(cudaEventRecord(ctx->join_ev[i - 1], lane_st[i]));
         PFK_CK(cudaStreamWaitEvent(st, ctx->join_ev[i - 1], 0));
@@ -937,6 +1006,7 @@ pfk_status pfk_destroy(pfk_ctx *ctx)
         ctx->d_cls_q[x].release();
         ctx->d_cls_kpref[x].release();
     }
+    ctx->d_kets.release();
     ctx->d_quart.release();
     ctx->d_shell_bf.release();
     ctx->d_shell_nbf.release();

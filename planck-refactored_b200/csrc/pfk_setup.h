@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "pfk_device.cuh"
+#include "pfk_internal.h"
 
 namespace pfk {
 
@@ -12,7 +13,7 @@ void launch_prim_bounds(int pc, const int *ids, int n, const PairInfo *pairs, Pr
 cudaError_t count_quartets(const double *qX, int nX, const double *qY, int nY, int diag, double tol, double bound,
                            long long *cnt_hi, long long *cnt_lo, cudaStream_t st);
 cudaError_t exclusive_scan(const long long *in, long long *out, int n, void *tmp, size_t &tmp_bytes, cudaStream_t st);
-cudaError_t fill_quartets(const int *idX, int nX, const int *idY, int diag, const long long *off_hi,
+cudaError_t fill_quartets(const int *idX, int nX, const uint2 *kets, int nY, int diag, const long long *off_hi,
                           const long long *cnt_hi, const long long *off_lo, const long long *cnt_lo, uint2 *out_hi,
                           uint2 *out_lo, cudaStream_t st);
 cudaError_t census(const uint2 *q, long long nq, const PairInfo *pairs, const int *pair_la, const int *pair_lb,
@@ -30,18 +31,19 @@ cudaError_t measure_fma_peak(int device, double *fp64, double *fp32);
 // every non-null density P0..P2 (rounded up to FP32), for density screening.
 cudaError_t shell_block_max(int nshell, const int *bf_off, const int *nbf, const double *P0, const double *P1,
                             const double *P2, int nb, float *D, cudaStream_t st);
-// start[b] = first entry of the sorted list whose loop length is in bucket b
-// (kLengthBuckets of them, ceil(log2) of the primitive quartets); entries of
-// empty buckets stay as they are.
-constexpr int kLengthBuckets = 25;
-cudaError_t bucket_starts(const uint2 *q, long long n, const PairInfo *pairs, long long *start, cudaStream_t st);
-// Sort keys of one list: ranks of the pairs as bras and as kets (by pair id)
-// and how many bits they and the primitive counts take.
-struct SortKeys {
-    const unsigned *bra_rank, *ket_rank;
-    int bra_bits, ket_bits, prim_bits;
+// The quartet lists lie one after another, each class's FP64 list before its
+// FP32 list: list l is entries first[l] .. first[l + 1] - 1.
+constexpr int kLists = 2 * kQuartetClasses;
+struct ListStarts {
+    long long first[kLists + 1];
 };
-cudaError_t sort_quartets(uint2 *q, long long n, const PairInfo *pairs, const SortKeys &k, unsigned *keys_a,
+// start[l * kLengthBuckets + b] = first entry of sorted list l, from its start,
+// whose loop length is in bucket b (ceil(log2) of the primitive quartets);
+// entries of empty buckets stay as they are.
+constexpr int kLengthBuckets = 25;
+cudaError_t bucket_starts(const uint2 *q, const PairInfo *pairs, const ListStarts &lists, long long *start,
+                          cudaStream_t st);
+cudaError_t sort_quartets(uint2 *q, long long n, const PairInfo *pairs, int prim_bits, unsigned *keys_a,
                           unsigned *keys_b, uint2 *vals_b, void *temp, size_t &temp_bytes, cudaStream_t st);
 
 }  // namespace pfk

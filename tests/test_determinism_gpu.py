@@ -94,3 +94,30 @@ def test_scf_runs_repeat_exactly():
         assert r["converged"]
         runs.append((r["iterations"], r["energy"]))
     assert runs[0] == runs[1] == runs[2], runs
+
+
+def test_first_and_later_builds_take_different_streams():
+    """A context's first build outside a graph runs on four streams, later
+    ones of a short list on twelve, captured ones on branches of one stream:
+    the same bits, and those of one lane."""
+    P = pfk()
+    _, shells = P.shells_for(water_cluster(2, seed=3), "6-31g**", basis_library())
+    ref = P.FockEngine(shells)
+    ref.set_lanes(1)
+    nb = ref.nbasis
+    Pa, Pb = random_density(nb, seed=35, scale=0.1), random_density(nb, seed=36, scale=0.1)
+    U, J, G = ref.fock_uhf(Pa, Pb), ref.jk(Pa, Pb), ref.fock_rhf(Pa)
+    T = ref.eri_tensor()
+    for graph_first in (False, True):
+        eng = P.FockEngine(shells)
+        if graph_first:
+            assert np.array_equal(eng.fock_rhf(Pa), G)
+        for _ in range(3):
+            assert all(np.array_equal(a, b) for a, b in zip(eng.fock_uhf(Pa, Pb), U))
+            assert all(np.array_equal(a, b) for a, b in zip(eng.jk(Pa, Pb), J))
+            assert np.array_equal(eng.fock_rhf(Pa), G)
+            assert np.array_equal(eng.eri_tensor(), T)
+        eng.set_lanes(2)
+        assert np.array_equal(eng.fock_rhf(Pa), G) and np.array_equal(eng.fock_uhf(Pa, Pb)[0], U[0])
+        eng.close()
+    ref.close()
