@@ -154,6 +154,10 @@ struct pfk_ctx {
 
     DevBuf<double> d_P, d_Pb, d_Pt, d_G, d_Gb;
     DevBuf<FxWord> d_J, d_K0, d_K1;   // fixed-point accumulators, 2 nb^2 words each
+    // end of the last build that returned before it was done: builds share the
+    // accumulators, so the next one waits for it on whatever stream it runs
+    cudaEvent_t done_ev = nullptr;
+    bool in_flight = false;
     std::vector<GraphEntry> graphs;
 
     pfk_status fail(pfk_status s, const std::string &msg)
@@ -497,6 +501,12 @@ pfk_status build_lists(pfk_ctx *ctx)
     return s;
 }
 
+// Orders what follows on st after the context's last asynchronous build.
+cudaError_t after_build(pfk_ctx *ctx, cudaStream_t st)
+{
+    return ctx->in_flight ? cudaStreamWaitEvent(st, ctx->done_ev, 0) : cudaSuccess;
+}
+
 pfk_status need_lists(pfk_ctx *ctx)
 {
     return ctx->lists_ok ? PFK_OK
@@ -716,6 +726,10 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
 {
     pfk_status ls = need_lists(ctx);
     if (ls != PFK_OK) return ls;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PFK_CK(cudaStreamIsCapturing(st, &capture));
+    const bool captured = capture == cudaStreamCaptureStatusActive;
+    if (!captured) PFK_CK(after_build(ctx, st));
     const size_t nb2 = (size_t)ctx->nb * ctx->nb;
     if (!eri_out) {
         PFK_CK(cudaMemsetAsync(Jacc, 0, sizeof(FxWord) * 2 * nb2, st));
@@ -760,9 +774,6 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
     // capture forks to side streams; those beyond kMaxLanes cost 50 us each to
     // create and again to destroy (0.8 ms together, the gain of a few builds),
     // so a context's first such build does without them.
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    PFK_CK(cudaStreamIsCapturing(st, &capture));
-    const bool captured = capture == cudaStreamCaptureStatusActive;
     int nlanes = timed ? 1 : ctx->lanes ? ctx->lanes : ctx->auto_lanes;
     if (!captured && !timed) {
         if (!ctx->built) nlanes = std::min(nlanes, kMaxLanes);
@@ -1019,6 +1030,7 @@ pfk_status pfk_destroy(pfk_ctx *ctx)
         if (ctx->join_ev[i]) cudaEventDestroy(ctx->join_ev[i]);
     }
     if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
+    if (ctx->done_ev) cudaEventDestroy(ctx->done_ev);
     if (ctx->blas) cublasDestroy(ctx->blas);
     for (int k = 0; k < 2; ++k) {
         if (ctx->pin[k]) cudaFreeHost(ctx->pin[k]);
@@ -1153,6 +1165,7 @@ pfk_status pfk_fock_rhf(pfk_ctx *ctx, const double *P, double *G)
     if (s != PFK_OK) return s;
     cudaSetDevice(ctx->device);
     const size_t bytes = sizeof(double) * ctx->nb * ctx->nb;
+    PFK_CK(after_build(ctx, ctx->stream));
     PFK_CK(cudaMemcpyAsync(ctx->d_P.p, P, bytes, cudaMemcpyHostToDevice, ctx->stream));
     s = rhf_graph(ctx, ctx->d_P.p, ctx->d_G.p, ctx->stream);
     if (s != PFK_OK) return s;
@@ -1167,7 +1180,16 @@ pfk_status pfk_fock_rhf_device(pfk_ctx *ctx, const double *dP, double *dG, void 
     if (!dP || !dG) return ctx->fail(PFK_ERR_INVALID, "null matrix");
     cudaSetDevice(ctx->device);
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
-    return rhf_graph(ctx, dP, dG, st);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PFK_CK(cudaStreamIsCapturing(st, &capture));
+    const bool order = capture == cudaStreamCaptureStatusNone;   // a caller's graph is the caller's to order
+    if (order) PFK_CK(after_build(ctx, st));
+    pfk_status s = rhf_graph(ctx, dP, dG, st);
+    if (s != PFK_OK || !order) return s;
+    if (!ctx->done_ev) PFK_CK(cudaEventCreateWithFlags(&ctx->done_ev, cudaEventDisableTiming));
+    PFK_CK(cudaEventRecord(ctx->done_ev, st));
+    ctx->in_flight = true;
+    return PFK_OK;
 }
 
 pfk_status pfk_fock_uhf(pfk_ctx *ctx, const double *Pa, const double *Pb, double *Ga, double *Gb)

@@ -121,3 +121,36 @@ def test_first_and_later_builds_take_different_streams():
         assert np.array_equal(eng.fock_rhf(Pa), G) and np.array_equal(eng.fock_uhf(Pa, Pb)[0], U[0])
         eng.close()
     ref.close()
+
+
+def test_builds_on_several_streams_do_not_meet():
+    """Builds of one context share its accumulators; issued on different
+    streams without a synchronisation between them they run one after
+    another, device builds among themselves and before host ones."""
+    torch = pytest.importorskip("torch")
+    P = pfk()
+    _, shells = P.shells_for(water_cluster(3, seed=3), "6-31g**", basis_library())
+    eng = P.FockEngine(shells)
+    nb = eng.nbasis
+    D = [random_density(nb, seed=40 + k, scale=0.1) for k in range(3)]
+    G = [eng.fock_rhf(d) for d in D]
+    U = eng.fock_uhf(D[0], D[1])
+    streams = [torch.cuda.Stream(), torch.cuda.Stream(), None]
+    dD = [torch.tensor(d, device="cuda:0") for d in D]
+    dG = [torch.zeros_like(d) for d in dD]
+    torch.cuda.synchronize()
+    for rep in range(40):
+        for k in range(3):
+            s = streams[(k + rep) % 3]
+            eng.fock_rhf_device(dD[k].data_ptr(), dG[k].data_ptr(), s.cuda_stream if s else 0)
+        if rep % 4 == 1:
+            assert np.array_equal(eng.fock_uhf(D[0], D[1])[0], U[0])
+        if rep % 4 == 3:
+            assert np.array_equal(eng.fock_rhf(D[1]), G[1])
+        if rep % 5 == 4:
+            torch.cuda.synchronize()
+            for k in range(3):
+                assert np.array_equal(dG[k].cpu().numpy(), G[k]), (rep, k)
+                dG[k].zero_()
+            torch.cuda.synchronize()
+    eng.close()
