@@ -68,18 +68,26 @@ struct GraphEntry {
     cudaStream_t stream;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    int launches = 0;
+    bool wide = false;   // captured with kSmallLanes branches
 };
 
 }  // namespace
 
-// Launch streams of a build: pfk_set_lanes takes 1 to kMaxLanes; by default
-// kMaxLanes, or kSmallLanes for lists of at most kSmallQuartets shell
-// quartets.  There a class kernel is a few blocks and lasts as long as one
-// quartet's chain of loads, recurrences and adds (20 to 60 us), so what counts
-// is how many run at once: one water / 6-31G** 272 -> 149 us a build with
-// 12 instead of 4; more than 4 were slower for (H2O)32 (49.8 ms with 4, 50.4
-// with 6, 50.6 with 8).
-constexpr int kMaxLanes = 4, kSmallLanes = 12;
+// Launch streams of a build, or branches of a captured one: pfk_set_lanes
+// takes 1 to kMaxLanes; by default kMaxLanes, or kSmallLanes for lists of at
+// most kSmallQuartets shell quartets.  There a class kernel is a few blocks and
+// lasts as long as one quartet's chain of loads, recurrences and adds (20 to
+// 60 us), so what counts is how many run at once: one water / 6-31G** 175 us a
+// build with 4, 115 with 12; (H2O)5 464 and 447; (H2O)4 / 3-21G 104 and 88.
+// More than 4 were slower for (H2O)32 (49.8 ms with 4, 50.4 with 6, 50.6 with 8).
+//
+// But 12 branches take 0.1 (water / 3-21G) to 0.45 ms (6-31G**) longer to
+// instantiate than 4 and as much longer to destroy, and eight more streams 0.4
+// ms each way: the gain of about kWideAfter builds.  So a graph, or a context's
+// builds outside graphs, begin with 4 and widen when they have been launched so
+// often: never more than about twice the cost of either choice.
+constexpr int kMaxLanes = 4, kSmallLanes = 12, kWideAfter = 16;
 constexpr long long kSmallQuartets = 4 << 20;
 
 struct pfk_ctx {
@@ -90,7 +98,7 @@ struct pfk_ctx {
     // build's stream (fork_ev) and joined back (join_ev) around the classes
     int lanes = 0;                    // 0: by the size of the lists (auto_lanes)
     int auto_lanes = kMaxLanes;       // set by build_lists
-    bool built = false;               // a build outside a capture has been launched
+    int direct_builds = 0;            // launched outside a capture, up to kWideAfter
     int nside = 0;                    // side streams created so far
     cudaStream_t side[kSmallLanes - 1] = {};
     cudaEvent_t fork_ev = nullptr, join_ev[kSmallLanes - 1] = {};
@@ -720,9 +728,11 @@ struct LaneEnds {
 };
 
 // Launch every class kernel over the screened lists.  Jacc/K accumulators are
-// zeroed first.  eri_out selects the dense-tensor mode.
+// zeroed first.  eri_out selects the dense-tensor mode.  wide = false: at most
+// kMaxLanes lanes.
 pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const double *Pk1, int nk, FxWord *Jacc,
-                       FxWord *K0, FxWord *K1, double *eri_out, cudaStream_t st, bool timed, bool eri_packed = false)
+                       FxWord *K0, FxWord *K1, double *eri_out, cudaStream_t st, bool timed, bool eri_packed = false,
+                       bool wide = true)
 {
     pfk_status ls = need_lists(ctx);
     if (ls != PFK_OK) return ls;
@@ -771,15 +781,14 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
     // the least work so far; a per-class timed pass stays on one stream.  A
     // captured build needs no streams for them: before each class its lane's
     // last node becomes what the next node depends on.  A build outside a
-    // capture forks to side streams; those beyond kMaxLanes cost 50 us each to
-    // create and again to destroy (0.8 ms together, the gain of a few builds),
-    // so a context's first such build does without them.
+    // capture forks to side streams.
     int nlanes = timed ? 1 : ctx->lanes ? ctx->lanes : ctx->auto_lanes;
-    if (!captured && !timed) {
-        if (!ctx->built) nlanes = std::min(nlanes, kMaxLanes);
-        ctx->built = true;
-        PFK_CK(side_streams(ctx, nlanes - 1));
+    if (!captured && !timed && ctx->direct_builds < kWideAfter) {
+        ++ctx->direct_builds;
+        wide = false;
     }
+    if (!wide) nlanes = std::min(nlanes, kMaxLanes);
+    if (!captured) PFK_CK(side_streams(ctx, nlanes - 1));
     LaneEnds ends[kSmallLanes + 1];   // of a captured build: where the lanes fork, then each lane's end
     if (captured && nlanes > 1) {
         PFK_CK(ends[nlanes].read(st));
@@ -855,9 +864,9 @@ pfk_status run_classes(pfk_ctx *ctx, const double *Pj, const double *Pk0, const 
     return PFK_OK;
 }
 
-pfk_status rhf_sequence(pfk_ctx *ctx, const double *dP, double *dG, cudaStream_t st)
+pfk_status rhf_sequence(pfk_ctx *ctx, const double *dP, double *dG, cudaStream_t st, bool wide = true)
 {
-    pfk_status s = run_classes(ctx, dP, dP, nullptr, 1, ctx->d_J.p, ctx->d_K0.p, nullptr, nullptr, st, false);
+    pfk_status s = run_classes(ctx, dP, dP, nullptr, 1, ctx->d_J.p, ctx->d_K0.p, nullptr, nullptr, st, false, false, wide);
     if (s != PFK_OK) return s;
     PFK_CK(combine(ctx->d_J.p, ctx->d_K0.p, 1.0, -0.5, dG, ctx->nb, st));
     return PFK_OK;
@@ -1133,10 +1142,12 @@ static pfk_status rhf_graph(pfk_ctx *ctx, const double *dP, double *dG, cudaStre
     GraphEntry *ge = nullptr;
     for (auto &g : ctx->graphs)
         if (g.in == dP && g.out == dG && g.stream == st) ge = &g;
-    if (!ge) {
+    const bool widen = ge && !ge->wide && ge->launches >= kWideAfter && !ctx->lanes && ctx->auto_lanes > kMaxLanes;
+    if (!ge || widen) {
         GraphEntry g{dP, dG, st};
+        g.wide = widen;
         PFK_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        pfk_status s = rhf_sequence(ctx, dP, dG, st);
+        pfk_status s = rhf_sequence(ctx, dP, dG, st, widen);
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(st, &graph);
         if (s != PFK_OK) {
@@ -1150,10 +1161,17 @@ static pfk_status rhf_graph(pfk_ctx *ctx, const double *dP, double *dG, cudaStre
             cudaGraphDestroy(graph);
             return ctx->cuda_fail("cudaGraphInstantiate", e);
         }
-        ctx->graphs.push_back(g);
-        ge = &ctx->graphs.back();
+        if (widen) {
+            cudaGraphExecDestroy(ge->exec);   // a launch in flight still completes
+            cudaGraphDestroy(ge->graph);
+            *ge = g;
+        } else {
+            ctx->graphs.push_back(g);
+            ge = &ctx->graphs.back();
+        }
     }
     PFK_CK(cudaGraphLaunch(ge->exec, st));
+    if (!ge->wide && ge->launches < kWideAfter) ++ge->launches;
     return PFK_OK;
 }
 

@@ -97,9 +97,9 @@ def test_scf_runs_repeat_exactly():
 
 
 def test_first_and_later_builds_take_different_streams():
-    """A context's first build outside a graph runs on four streams, later
-    ones of a short list on twelve, captured ones on branches of one stream:
-    the same bits, and those of one lane."""
+    """A graph, and a context's builds outside graphs, begin on four lanes and
+    take twelve from the 17th launch on (short lists); captured lanes are
+    branches of one stream: the same bits, and those of one lane."""
     P = pfk()
     _, shells = P.shells_for(water_cluster(2, seed=3), "6-31g**", basis_library())
     ref = P.FockEngine(shells)
@@ -112,7 +112,7 @@ def test_first_and_later_builds_take_different_streams():
         eng = P.FockEngine(shells)
         if graph_first:
             assert np.array_equal(eng.fock_rhf(Pa), G)
-        for _ in range(3):
+        for _ in range(19):
             assert all(np.array_equal(a, b) for a, b in zip(eng.fock_uhf(Pa, Pb), U))
             assert all(np.array_equal(a, b) for a, b in zip(eng.jk(Pa, Pb), J))
             assert np.array_equal(eng.fock_rhf(Pa), G)
