@@ -202,10 +202,10 @@ pfk_status pfk_set_density_screening(pfk_ctx *ctx, double dtol);
 /* Concurrent class launches: every later build of this context issues its
  * class kernels on `lanes` streams (1 to 4) forked from the build's stream
  * and joined back before the J/K combine, so that one class's tail and the
- * small classes overlap the others.  Until it is called a build takes 4, or
- * 12 when its lists are short (up to 4 Mi shell quartets).  Classes go, largest
- * (primitive quartets x component quartets) first, to the lane with the
- * least work.  lanes = 1 issues them in class order on the build's stream.
+ * small classes overlap the others.  4 is the default, with which builds of
+ * short lists (up to 4 Mi shell quartets) go on to 12 when they are repeated.
+ * Classes go, largest (primitive quartets x component quartets) first, to the
+ * lane with the least work.  lanes = 1 issues them in class order on the build's stream.
  * The results are bitwise identical for every lane count: the J/K
  * accumulation is in fixed-point integers, whose sums do not depend on the
  * order of the additions.

@@ -339,7 +339,8 @@ class FockEngine:
         self._check(self.lib.pfk_set_primitive_tol(self.h, float(ptol)))
 
     def set_lanes(self, lanes):
-        """Streams the class kernels of a build are spread over (1 to 4)."""
+        """Streams the class kernels of a build are spread over (1 to 4; 4 is
+        the default, which repeated builds of short lists extend to 12)."""
         self._check(self.lib.pfk_set_lanes(self.h, int(lanes)))
 
     def set_density_screening(self, dtol):

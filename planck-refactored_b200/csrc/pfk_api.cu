@@ -96,7 +96,7 @@ struct pfk_ctx {
     std::string err;
     // concurrent class launches: lanes - 1 side streams forked from the
     // build's stream (fork_ev) and joined back (join_ev) around the classes
-    int lanes = 0;                    // 0: by the size of the lists (auto_lanes)
+    int lanes = 0;                    // 0: kMaxLanes, or more by the size of the lists (auto_lanes)
     int auto_lanes = kMaxLanes;       // set by build_lists
     int direct_builds = 0;            // launched outside a capture, up to kWideAfter
     int nside = 0;                    // side streams created so far
@@ -1681,6 +1681,7 @@ pfk_status pfk_set_lanes(pfk_ctx *ctx, int lanes)
 {
     if (!ctx) return PFK_ERR_STATE;
     if (lanes < 1 || lanes > kMaxLanes) return ctx->fail(PFK_ERR_INVALID, "need 1 <= lanes <= 4");
+    if (lanes == kMaxLanes) lanes = 0;           // the default
     if (lanes != ctx->lanes) drop_graphs(ctx);   // captured builds hold the old fork
     ctx->lanes = lanes;
     return PFK_OK;
