@@ -104,9 +104,10 @@ struct pfk_ctx {
     cudaEvent_t fork_ev = nullptr, join_ev[kSmallLanes - 1] = {};
     cublasHandle_t blas = nullptr;   // created by the first pfk_mo_transform
     double mo_ms[3] = {0.0, 0.0, 0.0};   // last pfk_mo_transform: AO tensor, GEMMs, copy out
-    // buffers of the MO transform (mo_run), kept for the next call while they
-    // are within kMoKeepBytes together
-    DevBuf<double> mo_E, mo_T1, mo_T2, mo_C, mo_red;
+    // buffers of the MO transform (mo_run), kept for the next call while all
+    // contexts' together are within kMoKeepBytes; mo_kept: counted there
+    DevBuf<double> mo_E, mo_W, mo_T2, mo_C, mo_red;
+    size_t mo_kept = 0;
     // two pinned staging chunks for copying MO blocks into pageable host memory
     void *pin[2] = {nullptr, nullptr};
     cudaEvent_t pin_ev[2] = {nullptr, nullptr};
@@ -883,6 +884,44 @@ pfk_status ensure_work(pfk_ctx *ctx)
     return PFK_OK;
 }
 
+// Gives the MO transform's buffers back, all of them or when the device's
+// contexts would keep more than kMoKeepBytes together.
+constexpr size_t kMoKeepBytes = size_t(4) << 30;
+std::atomic<size_t> g_mo_kept[64];   // by device (mod 64: devices that share an entry share the limit)
+void mo_release(pfk_ctx *ctx, bool all)
+{
+    DevBuf<double> *bufs[] = {&ctx->mo_E, &ctx->mo_W, &ctx->mo_T2, &ctx->mo_C, &ctx->mo_red};
+    std::atomic<size_t> &kept = g_mo_kept[ctx->device & 63];
+    size_t bytes = 0;
+    for (auto *b : bufs) bytes += sizeof(double) * b->n;
+    kept -= ctx->mo_kept;
+    ctx->mo_kept = 0;
+    if (!all && kept.fetch_add(bytes) + bytes <= kMoKeepBytes) {
+        ctx->mo_kept = bytes;
+        return;
+    }
+    if (!all) kept -= bytes;
+    for (auto *b : bufs) b->release();
+}
+
+// Makes every buffer at least so long.  What has to grow is freed before
+// anything is allocated, and if that does not fit, so is the rest (not E with
+// keep_E).
+cudaError_t mo_reserve(pfk_ctx *ctx, bool keep_E, size_t nE, size_t nW, size_t nT2, size_t nC, size_t nred)
+{
+    struct { DevBuf<double> *b; size_t n; } need[] = {
+        {&ctx->mo_E, nE}, {&ctx->mo_W, nW}, {&ctx->mo_T2, nT2}, {&ctx->mo_C, nC}, {&ctx->mo_red, nred}};
+    cudaError_t e = cudaSuccess;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        for (auto &x : need)
+            if (x.b->n < x.n || (attempt > 0 && !(keep_E && x.b == &ctx->mo_E))) x.b->release();
+        for (auto &x : need)
+            if ((e = x.b->reserve(x.n)) != cudaSuccess) break;
+        if (e == cudaSuccess) break;
+    }
+    return e;
+}
+
 // max |P(i,j) - P(j,i)| against 1e-10 max(1, max |P|), and every element
 // finite.  The transposed pairs are compared tile by tile (32 x 32), so both
 // tiles stay in cache: a row-against-column sweep of an 800 x 800 matrix
@@ -1031,7 +1070,7 @@ pfk_status pfk_destroy(pfk_ctx *ctx)
     ctx->d_shell_bf.release();
     ctx->d_shell_nbf.release();
     ctx->d_Dsh.release();
-    for (DevBuf<double> *b : {&ctx->mo_E, &ctx->mo_T1, &ctx->mo_T2, &ctx->mo_C, &ctx->mo_red}) b->release();
+    mo_release(ctx, true);
     for (DevBuf<double> *b : {&ctx->d_P, &ctx->d_Pb, &ctx->d_Pt, &ctx->d_G, &ctx->d_Gb}) b->release();
     for (DevBuf<FxWord> *b : {&ctx->d_J, &ctx->d_K0, &ctx->d_K1}) b->release();
     for (int i = 0; i < kSmallLanes - 1; ++i) {
@@ -1304,8 +1343,9 @@ pfk_status pfk_eri_tensor(pfk_ctx *ctx, double *eri)
 // depend on the order in which blocks finish.
 constexpr int kMp2R = 0, kMp2Same = 1, kMp2Opp = 2;
 
-// out[r][l][s] = out[r][s][l] = in[r][l (l + 1) / 2 + s]: one block per row
-// group r and l, the packed row read once, s across the threads.
+// out[r][l][s] = out[r][s][l] = in[r][l (l + 1) / 2 + s], l >= s: one block per
+// r, the nb^2 elements in order over its threads (the writes are coalesced;
+// the upper half's reads are strided, out of the caches: a row is 63 KB).
 __global__ void __launch_bounds__(128) unpack_pairs_kernel(const double *__restrict__ in, int nb, double *__restrict__ out)
 {
     const size_t np = (size_t)nb * (nb + 1) / 2, r = blockIdx.x;
@@ -1357,17 +1397,9 @@ __global__ void __launch_bounds__(256) mp2_sum_kernel(const double *__restrict__
 // next call with 2, which uses it as it is.
 //
 // The buffers belong to the context: a call that allocated and freed its
-// 2 GB tensor (125 functions) spent about 3 of its 8 ms on that.  Above kMoKeepBytes
-// together they are given back when the call ends (mo_release).
-constexpr size_t kMoKeepBytes = size_t(4) << 30;
-static void mo_release(pfk_ctx *ctx)
-{
-    DevBuf<double> *all[] = {&ctx->mo_E, &ctx->mo_T1, &ctx->mo_T2, &ctx->mo_C, &ctx->mo_red};
-    size_t bytes = 0;
-    for (auto *b : all) bytes += sizeof(double) * b->n;
-    if (bytes > kMoKeepBytes)
-        for (auto *b : all) b->release();
-}
+// 2 GB tensor (125 functions) spent about 3 of its 8 ms on that.  They stay for
+// the next call while what all contexts of the process keep on this device is
+// at most kMoKeepBytes (mo_release); pfk_destroy gives them back.
 static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C2, int n2, const double *C3, int n3,
                          const double *C4, int n4, double *out, const double *eps1, const double *eps2, int mode,
                          double *e_corr, int share = 0)
@@ -1375,7 +1407,7 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
     struct Release {
         pfk_ctx *c;
         bool on;
-        ~Release() { if (on) mo_release(c); }
+        ~Release() { if (on) mo_release(c, false); }
     } release{ctx, share == 0};
     const int nb = ctx->nb;
     if (n1 < 1 || n2 < 1 || n3 < 1 || n4 < 1 || n1 > nb || n2 > nb || n3 > nb || n4 > nb)
@@ -1389,15 +1421,23 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
     if (cublasSetStream(ctx->blas, st) != CUBLAS_STATUS_SUCCESS) return ctx->fail(PFK_ERR_CUDA, "cublasSetStream failed");
     const size_t b = nb, b2 = b * b;
     const size_t np = b * (b + 1) / 2;
-    // buffers allocated before the timed work: the packed AO tensor E
-    // (nb^2 np), T1 (n1 nb np, and T3 after it: n1 n2 n3 nb) and the unpacked
-    // T2 (n1 n2 nb^2, and the result after it).  The packed T2 (n1 n2 np)
-    // overwrites E, or has its place behind the unpacked one when E is kept
-    DevBuf<double> &E = ctx->mo_E, &T1 = ctx->mo_T1, &T2buf = ctx->mo_T2;
+    // buffers allocated before the timed work.  W: the packed AO tensor E
+    // (nb^2 np), over which the packed T2 (n1 n2 np) is written, and T1
+    // (n1 nb np) behind it, then T3 (n1 n2 n3 nb) over both; T2buf: the unpacked
+    // T2 (n1 n2 nb^2), then the result.  With all orbitals in all four blocks
+    // that is 2 nb^4.  An E kept for further calls has a buffer of its own, and
+    // the packed T2 its place behind the unpacked one
     const bool build_E = share != 2;
     const double *hC[4] = {C1, C2, C3, C4};
     const int nk[4] = {n1, n2, n3, n4};
-    PFK_CK(ctx->mo_C.reserve(b * ((size_t)n1 + n2 + n3 + n4)));
+    const size_t nE = b2 * np, nT1 = b * np * n1, nT3 = b * n1 * n2 * n3, nT2 = b2 * (size_t)n1 * n2;
+    const size_t behind = (nE + 31) / 32 * 32;   // 256-byte steps, as an allocation
+    int nsm = 0;
+    PFK_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    const int grid = 8 * std::max(nsm, 1);   // of the MP2 sums: 8 blocks of 256 per SM
+    PFK_CK(mo_reserve(ctx, share == 2, share ? nE : 0, share ? std::max(nT1, nT3) : std::max(behind + nT1, nT3),
+                      nT2 + (share ? np * n1 * n2 : 0), b * ((size_t)n1 + n2 + n3 + n4), eps1 ? 2 * b + grid : 0));
+    double *const E = share ? ctx->mo_E.p : ctx->mo_W.p, *const T1 = share ? ctx->mo_W.p : ctx->mo_W.p + behind;
     double *dC[4];
     size_t c_at = 0;
     for (int k = 0; k < 4; ++k) {
@@ -1416,14 +1456,11 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
         ~EvFree() { for (int k = 0; k < 4; ++k) if (e[k]) cudaEventDestroy(e[k]); }
     } ev_free{ev};
     for (auto &x : ev) PFK_CK(cudaEventCreate(&x));
-    PFK_CK(E.reserve(b2 * np));
-    PFK_CK(T1.reserve(std::max(b * np * n1, b * n1 * n2 * n3)));
-    PFK_CK(T2buf.reserve((b2 + (share ? np : 0)) * (size_t)n1 * n2));
     PFK_CK(cudaEventRecord(ev[0], st));
     pfk_status s = PFK_OK;
     if (build_E) {
-        PFK_CK(cudaMemsetAsync(E.p, 0, sizeof(double) * b2 * np, st));
-        s = run_classes(ctx, ctx->d_P.p, ctx->d_P.p, nullptr, 1, ctx->d_J.p, nullptr, nullptr, E.p, st, false, true);
+        PFK_CK(cudaMemsetAsync(E, 0, sizeof(double) * nE, st));
+        s = run_classes(ctx, ctx->d_P.p, ctx->d_P.p, nullptr, 1, ctx->d_J.p, nullptr, nullptr, E, st, false, true);
         if (s != PFK_OK) return s;
     }
     PFK_CK(cudaEventRecord(ev[1], st));
@@ -1431,12 +1468,12 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
     auto ck = [&](cublasStatus_t r, const char *what) {
         return r == CUBLAS_STATUS_SUCCESS ? PFK_OK : ctx->fail(PFK_ERR_CUDA, std::string(what) + " failed");
     };
-    double *T2 = T2buf.p, *T2p = share ? T2 + b2 * n1 * n2 : E.p, *T3 = T1.p, *O = T2;
-    s = ck(cublasDgemm(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)(b * np), n1, nb, &one, E.p, (int)(b * np), dC[0], nb,
-                       &zero, T1.p, (int)(b * np)),
+    double *T2 = ctx->mo_T2.p, *T2p = share ? T2 + nT2 : E, *T3 = ctx->mo_W.p, *O = T2;
+    s = ck(cublasDgemm(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)(b * np), n1, nb, &one, E, (int)(b * np), dC[0], nb,
+                       &zero, T1, (int)(b * np)),
            "quarter transform 1 (cublasDgemm)");
     if (s != PFK_OK) return s;
-    s = ck(cublasDgemmStridedBatched(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)np, n2, nb, &one, T1.p, (int)np,
+    s = ck(cublasDgemmStridedBatched(ctx->blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)np, n2, nb, &one, T1, (int)np,
                                      (long long)(b * np), dC[1], nb, 0, &zero, T2p, (int)np, (long long)np * n2, n1),
            "quarter transform 2 (cublasDgemmStridedBatched)");
     if (s != PFK_OK) return s;
@@ -1453,10 +1490,6 @@ static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C
     if (s != PFK_OK) return s;
     PFK_CK(cudaEventRecord(ev[2], st));
     if (eps1) {
-        int nsm = 0;
-        PFK_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-        const int grid = 8 * std::max(nsm, 1);   // 8 blocks of 256 per SM
-        PFK_CK(ctx->mo_red.reserve(2 * b + grid));
         double *d_eps = ctx->mo_red.p, *d_sum = d_eps + 2 * b;
         PFK_CK(cudaMemcpyAsync(d_eps, eps1, sizeof(double) * nb, cudaMemcpyHostToDevice, st));
         PFK_CK(cudaMemcpyAsync(d_eps + nb, eps2, sizeof(double) * nb, cudaMemcpyHostToDevice, st));
@@ -1544,7 +1577,7 @@ pfk_status pfk_ump2_energy(pfk_ctx *ctx, const double *Ca, const double *eps_a, 
         s = mo_run(ctx, Cb, n_beta, Cbv, nvb, Cb, n_beta, Cbv, nvb, nullptr, eps_b, eps_b, kMp2Same, &e_bb, 2);
     if (s == PFK_OK)
         s = mo_run(ctx, Ca, n_alpha, Cav, nva, Cb, n_beta, Cbv, nvb, nullptr, eps_a, eps_b, kMp2Opp, &e_ab, 2);
-    mo_release(ctx);
+    mo_release(ctx, false);
     if (s == PFK_OK) *e_corr = e_aa + e_bb + e_ab;
     return s;
 }

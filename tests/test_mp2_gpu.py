@@ -136,3 +136,47 @@ def test_kept_buffers_do_not_leak_between_calls():
         assert np.array_equal(call(kept), call(fresh))
         fresh.close()
     kept.close()
+
+
+def _device_bytes():
+    torch = pytest.importorskip("torch")
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+def test_kept_buffers_are_bounded_over_contexts():
+    """What the transforms leave with their contexts is 4 GiB in the whole
+    process, not in each: four contexts of 125 functions, 1.5 GB each (and
+    cuBLAS's workspaces, under 0.1 GB each)."""
+    P = pfk()
+    mol, shells = P.shells_for(P.workloads.water_cluster(5, seed=2), "6-31g**", basis_library())
+    engines = [P.FockEngine(shells) for _ in range(4)]
+    nb = engines[0].nbasis
+    C = np.linalg.qr(np.random.default_rng(1).normal(size=(nb, nb)))[0]
+    eps = np.concatenate([-2.0 + 0.01 * np.arange(25), 0.5 + 0.01 * np.arange(nb - 25)])
+    before = _device_bytes()
+    e = [eng.rmp2_energy(C, eps, 25) for eng in engines]
+    assert e[1:] == e[:-1]
+    assert 1.0e9 < _device_bytes() - before < 2 ** 32 + 0.4e9
+    assert engines[3].rmp2_energy(C, eps, 25) == e[0] == engines[0].rmp2_energy(C, eps, 25)
+    for eng in engines:
+        eng.close()
+    assert _device_bytes() - before < 0.2e9
+
+
+def test_full_transform_takes_two_tensors():
+    """All orbitals in all four blocks: 2 nb^4 doubles at once, the size of
+    the tensor and the result (cuBLAS's workspace, 0.08 GB, is a tenth of
+    one)."""
+    P = pfk()
+    mol, shells = P.shells_for(P.workloads.water_cluster(4, seed=2), "6-31g**", basis_library())
+    eng = P.FockEngine(shells)
+    nb = eng.nbasis
+    C = np.linalg.qr(np.random.default_rng(1).normal(size=(nb, nb)))[0]
+    small = eng.mo_transform(C[:, :2], C, C[:, :2], C)
+    full = eng.mo_transform(C, C, C, C)
+    assert np.abs(full[:2, :, :2, :] - small).max() < 1e-12
+    kept = _device_bytes()
+    eng.close()
+    assert 1.9 * 8 * nb ** 4 < kept - _device_bytes() < 2.2 * 8 * nb ** 4
