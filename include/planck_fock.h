@@ -139,8 +139,9 @@ pfk_status pfk_eri_tensor(pfk_ctx *ctx, double *eri);
  * there as FP64 GEMMs (cuBLAS); nothing of size nbasis^4 crosses to the
  * host.  With all orbitals in all four blocks 2 nbasis^4 doubles are on the
  * device at once.  The device buffers of this call and of the MP2 energies stay
- * with the context for its next one while the contexts of the process keep at
- * most 4 GiB of them on the device; pfk_destroy frees them. */
+ * with the context for its next one, at most 4 GiB of them, and at most a
+ * sixteenth of the device's memory in all contexts of the process;
+ * pfk_destroy frees them. */
 pfk_status pfk_mo_transform(pfk_ctx *ctx, const double *C1, int n1, const double *C2, int n2, const double *C3,
                             int n3, const double *C4, int n4, double *out);
 

@@ -104,8 +104,8 @@ struct pfk_ctx {
     cudaEvent_t fork_ev = nullptr, join_ev[kSmallLanes - 1] = {};
     cublasHandle_t blas = nullptr;   // created by the first pfk_mo_transform
     double mo_ms[3] = {0.0, 0.0, 0.0};   // last pfk_mo_transform: AO tensor, GEMMs, copy out
-    // buffers of the MO transform (mo_run), kept for the next call while all
-    // contexts' together are within kMoKeepBytes; mo_kept: counted there
+    // buffers of the MO transform (mo_run), kept for the next call within the
+    // limits of mo_release; mo_kept: how much of them is counted there
     DevBuf<double> mo_E, mo_W, mo_T2, mo_C, mo_red;
     size_t mo_kept = 0;
     // two pinned staging chunks for copying MO blocks into pageable host memory
@@ -884,23 +884,33 @@ pfk_status ensure_work(pfk_ctx *ctx)
     return PFK_OK;
 }
 
-// Gives the MO transform's buffers back, all of them or when the device's
-// contexts would keep more than kMoKeepBytes together.
+// Gives the MO transform's buffers back: all of them, or when this context
+// would keep more than kMoKeepBytes or all contexts more than a sixteenth of
+// the device's memory (12 GB of 183: eight contexts of 125 functions; with
+// three at work in turn a call that had to allocate took 4.5 ms instead of 2.4).
 constexpr size_t kMoKeepBytes = size_t(4) << 30;
 std::atomic<size_t> g_mo_kept[64];   // by device (mod 64: devices that share an entry share the limit)
+size_t mo_keep_limit()
+{
+    size_t avail = 0, total = 0;
+    return cudaMemGetInfo(&avail, &total) == cudaSuccess ? total / 16 : 0;
+}
 void mo_release(pfk_ctx *ctx, bool all)
 {
     DevBuf<double> *bufs[] = {&ctx->mo_E, &ctx->mo_W, &ctx->mo_T2, &ctx->mo_C, &ctx->mo_red};
     std::atomic<size_t> &kept = g_mo_kept[ctx->device & 63];
     size_t bytes = 0;
     for (auto *b : bufs) bytes += sizeof(double) * b->n;
+    if (!all && bytes == ctx->mo_kept) return;   // counted already
     kept -= ctx->mo_kept;
     ctx->mo_kept = 0;
-    if (!all && kept.fetch_add(bytes) + bytes <= kMoKeepBytes) {
-        ctx->mo_kept = bytes;
-        return;
+    if (!all && bytes <= kMoKeepBytes) {
+        if (kept.fetch_add(bytes) + bytes <= mo_keep_limit()) {
+            ctx->mo_kept = bytes;
+            return;
+        }
+        kept -= bytes;
     }
-    if (!all) kept -= bytes;
     for (auto *b : bufs) b->release();
 }
 
@@ -1398,8 +1408,7 @@ __global__ void __launch_bounds__(256) mp2_sum_kernel(const double *__restrict__
 //
 // The buffers belong to the context: a call that allocated and freed its
 // 2 GB tensor (125 functions) spent about 3 of its 8 ms on that.  They stay for
-// the next call while what all contexts of the process keep on this device is
-// at most kMoKeepBytes (mo_release); pfk_destroy gives them back.
+// the next call within the limits of mo_release; pfk_destroy gives them back.
 static pfk_status mo_run(pfk_ctx *ctx, const double *C1, int n1, const double *C2, int n2, const double *C3, int n3,
                          const double *C4, int n4, double *out, const double *eps1, const double *eps2, int mode,
                          double *e_corr, int share = 0)
