@@ -20,7 +20,7 @@ using namespace pfk;
 
 namespace pfk {
 ClassLauncher g_class_launchers[kQuartetClasses];   // constant-initialised; filled by the class units
-ClassResident g_class_resident[kQuartetClasses];
+ClassWaves g_class_waves[kQuartetClasses];
 }
 
 namespace {
@@ -2025,8 +2025,7 @@ extern "C" pfk_status pfk_fock_rhf_noalloc(const pfk_basis_desc *basis, const do
 // warp, and that one is slower in a window's order: its 32 quartets are all
 // of the longest, each with primitives of its own to load, to the end, where
 // in the caller's order most lanes drop out.  So up to one wave
-// (g_class_resident) runs as listed, in the builds for that (kLaunchShort),
-// and the windows begin above it.  Windowed / listed time, FP64, at n of the
+// (g_class_waves) runs as listed, and the windows begin above it.  Windowed / listed time, FP64, at n of the
 // wave w: (ss|ss) w = 151552: 2.2 (n = 8192), 1.6 (65536); (ps|ps) Rys 1.9,
 // 1.3 (w = 75776); (pp|pp) w = 37888: 1.4, 0.72; (pp|ps) w = 56832: 1.55, 0.84;
 // (dp|pp) w = 7104: 1.02 (6144), 0.92 (8192), 0.66 (16384); (fp|pp) w = 3552:
@@ -2050,16 +2049,16 @@ struct pfk_eri_batch {
     std::vector<int> pair_nprim;
     long long nq = 0;
     int cls = -1;              // class of the listed quartets
-    // one wave of the listed class per launch flags (-1: not asked for yet)
-    std::atomic<long long> wave[16] = {};
-    long long one_wave(int flags)
+    // the listed class's waves by launch flags, asked for once
+    std::mutex waves_lock;
+    BlockWaves waves[4];
+    bool have_waves[4] = {};
+    BlockWaves waves_of(int flags)
     {
-        long long w = wave[flags].load(std::memory_order_relaxed);
-        if (w < 0) {
-            w = g_class_resident[cls](flags);
-            wave[flags].store(w, std::memory_order_relaxed);
-        }
-        return w;
+        std::lock_guard<std::mutex> hold(waves_lock);
+        if (!have_waves[flags]) waves[flags] = g_class_waves[cls](flags);
+        have_waves[flags] = true;
+        return waves[flags];
     }
 
     pfk_status fail(pfk_status s, const std::string &msg)
@@ -2212,7 +2211,7 @@ pfk_status pfk_eri_batch_set_quartets(pfk_eri_batch *ctx, const int *quartets, l
     PFK_CK(cudaStreamSynchronize(ctx->stream));
     ctx->d_sorted.release();
     ctx->d_pos.release();
-    for (auto &w : ctx->wave) w.store(-1, std::memory_order_relaxed);
+    for (bool &h : ctx->have_waves) h = false;
     if (n <= INT32_MAX) {
         try {
             // (longest first, place) as one key: at most 64^4 primitive quartets
@@ -2275,10 +2274,11 @@ pfk_status pfk_eri_batch_run(pfk_eri_batch *ctx, long long first, long long coun
     a.qstride = 1;
     a.qoffset = 0;
     int flags = (engine == PFK_ENGINE_OS ? kLaunchOS : 0) | (precision == PFK_PREC_MIXED ? kLaunchFP32 : 0);
-    const bool few = count <= ctx->one_wave(flags | kLaunchShort);
+    const BlockWaves w = ctx->waves_of(flags);
+    const bool few = count <= w.few_limit;
     if (few) flags |= kLaunchShort;
     // above a wave, whole windows of the range run in their sorted order, the ends as listed
-    const bool windows = !few && count > ctx->one_wave(flags) && ctx->d_sorted.p;
+    const bool windows = count > (few ? w.few_wave : w.wave) && ctx->d_sorted.p;
     const long long end = first + count;
     long long w0 = (first + kBatchWindow - 1) / kBatchWindow * kBatchWindow;
     long long w1 = end == ctx->nq ? end : end / kBatchWindow * kBatchWindow;

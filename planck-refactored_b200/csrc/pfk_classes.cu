@@ -64,7 +64,8 @@ struct OutBuild {
     void (*kernel)(const uint2 *, long long, JKArgs);
     int threads;
     size_t smem;
-    int per;   // quartets per block
+    int per;         // quartets per block
+    int few_waves;   // up to so many waves this build, if it is the one for short lists
 };
 // the plain Obara-Saika build: left alone the compiler takes 94 registers at
 // L = 1 and 190 at L = 3 to have more of the Boys polynomials in flight, at 5
@@ -83,43 +84,45 @@ OutBuild out_build(int flags)
         if (flags & kLaunchOS)
             return {fp32 ? &eri_os_kernel<LA, LB, LC, LD, 1, float, kOSBlocks<L, float>, false, true>
                          : &eri_os_kernel<LA, LB, LC, LD, 1, double, kOSBlocks<L, double>, false, true>,
-                    128, 0, 128};
+                    128, 0, 128, 1};
     }
     if constexpr (S::N <= kRegMaxComponents) {
         if (fp32)
             return {few ? &eri_reg_kernel<LA, LB, LC, LD, 1, float, true, RegShape<LA, LB, LC, LD, float>::MINB_SHORT>
                         : &eri_reg_kernel<LA, LB, LC, LD, 1, float, true>,
-                    128, 0, 128};
-        return {&eri_reg_kernel<LA, LB, LC, LD, 1, double, true>, 128, 0, 128};
+                    128, 0, 128, 1};
+        return {&eri_reg_kernel<LA, LB, LC, LD, 1, double, true>, 128, 0, 128, 1};
     } else if constexpr (SS::OK) {
         using SF = SplitShape<LA, LB, LC, LD, float>;
         if (fp32)
             return {few ? &eri_split_kernel<LA, LB, LC, LD, 1, float, false, true, SF::MINB_SHORT>
                         : &eri_split_kernel<LA, LB, LC, LD, 1, float, false, true>,
-                    128, SF::SMEM, SF::TEAMS};
+                    128, SF::SMEM, SF::TEAMS, SF::FEW_WAVES};
         return {few ? &eri_split_kernel<LA, LB, LC, LD, 1, double, false, true, SS::MINB_SHORT>
                     : &eri_split_kernel<LA, LB, LC, LD, 1, double, false, true>,
-                128, SS::SMEM, SS::TEAMS};
+                128, SS::SMEM, SS::TEAMS, SS::FEW_WAVES};
     } else {
         using TS = TeamShape<LA, LB, LC, LD>;
         using TF = TeamShape<LA, LB, LC, LD, float>;
-        if (fp32) return {&eri_team_kernel<LA, LB, LC, LD, 1, float>, TF::BLOCK, TF::SMEM, TF::TEAMS};
-        return {&eri_team_kernel<LA, LB, LC, LD, 1>, TS::BLOCK, TS::SMEM, TS::TEAMS};
+        if (fp32) return {&eri_team_kernel<LA, LB, LC, LD, 1, float>, TF::BLOCK, TF::SMEM, TF::TEAMS, 1};
+        return {&eri_team_kernel<LA, LB, LC, LD, 1>, TS::BLOCK, TS::SMEM, TS::TEAMS, 1};
     }
 }
 
 template <int LA, int LB, int LC, int LD>
-long long resident_quartets(int flags)
+BlockWaves block_waves(int flags)
 {
-    const OutBuild o = out_build<LA, LB, LC, LD>(flags);
-    int dev = 0, sms = 0, blocks = 0;
+    const OutBuild few = out_build<LA, LB, LC, LD>(flags | kLaunchShort), many = out_build<LA, LB, LC, LD>(flags);
+    int dev = 0, sms = 0, blocks[2] = {};
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, o.kernel, o.threads, o.smem) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[0], few.kernel, few.threads, few.smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[1], many.kernel, many.threads, many.smem) != cudaSuccess) {
         cudaGetLastError();
-        return 0;
+        return {};
     }
-    return (long long)blocks * sms * o.per;
+    const long long wave = (long long)blocks[0] * sms * few.per;
+    return {wave, wave * few.few_waves, (long long)blocks[1] * sms * many.per};
 }
 
 template <int LA, int LB, int LC, int LD>
@@ -246,7 +249,7 @@ void reg_range()
 {
     constexpr int X = cls_bra(C), Y = cls_ket(C);
     g_class_launchers[C] = &launch_class<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
-    g_class_resident[C] = &resident_quartets<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
+    g_class_waves[C] = &block_waves<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
     if constexpr (C + 1 < PFK_CLASS_END) reg_range<C + 1>();
 }
 

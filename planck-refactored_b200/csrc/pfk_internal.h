@@ -31,7 +31,7 @@ __host__ __device__ constexpr int quartet_class_L(int c)
 // for classes with LA+LB+LC+LD <= kOSMaxL; the other classes run Rys.
 // kLaunchDense picks the Obara-Saika kernel compiled for 4 blocks of 128
 // per SM (single exchange density only).  kLaunchShort, in block mode, picks
-// the build for launches of at most one wave (MINB_SHORT).
+// the build for short lists (MINB_SHORT).
 constexpr int kLaunchFP32 = 1, kLaunchOS = 2, kLaunchDense = 4, kLaunchShort = 8;
 constexpr int kOSMaxL = 4;
 
@@ -44,10 +44,15 @@ using ClassLauncher = void (*)(const uint2 *quartets, long long n, const JKArgs 
 // n < 0 only configures the current device for its kernels.
 extern ClassLauncher g_class_launchers[kQuartetClasses];
 
-// How many quartets of each class the current device works on at once (one
-// wave) in the build that block mode takes for these flags; 0 on an error.
-using ClassResident = long long (*)(int flags);
-extern ClassResident g_class_resident[kQuartetClasses];
+// Block mode on the current device, for launch flags without kLaunchShort: how
+// many quartets the build for short lists works on at once (one wave), the
+// longest list that it is the faster build for, and one wave of the other
+// build.  Zeros on an error.
+struct BlockWaves {
+    long long few_wave, few_limit, wave;
+};
+using ClassWaves = BlockWaves (*)(int flags);
+extern ClassWaves g_class_waves[kQuartetClasses];
 
 // Context internals for the other units: its CUDA device, and recording a
 // failure message (returns s).

@@ -741,16 +741,19 @@ struct SplitShape {
     // M = 18); at M = 27 the spills cost more ((dp|pp) 3.42 -> 3.70).  With 54
     // FP64 accumulators three blocks spill 900 to 1300 bytes into the inner
     // loop, two none: 16384 (fd|pp) blocks 4.00 -> 3.33 ms.  In FP32 three
-    // spill 360 and are the faster build of long lists (16384 (dp|dp) blocks
-    // 11%, (fd|pp) 16%); short ones gain 7% from two.
+    // spill 360, and are the faster build of long lists only (FEW_WAVES).
     static constexpr int MINB = M <= 18 ? 4 : M <= 36 || sizeof(R) == 4 ? 3 : 2;
     // the SPLIT builds (lists far below one wave)
     static constexpr int MINB_SPLIT = M <= 18 ? 4 : M <= 36 ? 3 : 2;
-    // block-mode launches of at most one wave, which lasts as long as its
-    // longest quartet: no spills count, blocks per SM do not.  512 quartets
-    // at 4 blocks per SM instead of 3: (dd|dp) 13%, (fs|dp) 8%, (dd|ps) 7%
-    // slower; 65536: 3 to 22% faster
-    static constexpr int MINB_SHORT = M <= 18 ? 3 : M <= 27 || (M <= 36 && sizeof(R) == 4) ? 3 : 2;
+    // block-mode launches of at most FEW_WAVES times what fits on the chip at
+    // once, where a quartet's own time counts (no spills) and blocks per SM do
+    // not.  4 blocks per SM instead of 3 at M = 18: 512 quartets (dd|dp) 13%,
+    // (fs|dp) 8%, (dd|ps) 7% slower, 1.2 waves of (fs|dp) and (dd|dp) 16% and 14%,
+    // 65536 quartets 3 to 22% faster.  3 instead of 2 at M = 54 in FP32: up to
+    // 5 waves 8 to 23% slower ((fp|dp) 3072, (fd|pp) 12288, (dp|dp) 16384), from
+    // 14 waves 8 to 10% faster
+    static constexpr int MINB_SHORT = M <= 27 || (M <= 36 && sizeof(R) == 4) ? 3 : 2;
+    static constexpr int FEW_WAVES = M > 36 && sizeof(R) == 4 ? 6 : 2;
 };
 
 template <int TEAM>
