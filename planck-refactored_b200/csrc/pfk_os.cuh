@@ -91,19 +91,20 @@ __device__ __forceinline__ double boys_exp(double T)
 // (kBoysMid; gen_boys_table.py).  One polynomial covers the whole range, so
 // the lanes of a warp, whose T are unrelated, run one path of about 40
 // instructions.  M >= 1: the same for T >= TS, then the upward recursion
-// F_{m+1} = ((2m+1) F_m - e^-T) / (2T), whose error growth stays below ~10x
-// for m <= 4 at T >= 2 (TS = 1 for M = 1, 2 up to M = 4, 3 above); for T < TS
-// F_M by interpolation in T (kBoysSmall) and the stable downward recursion
-// F_m = (2T F_{m+1} + e^-T) / (2m+1).  One rsqrt gives both 1/sqrt(T + 16)
+// F_{m+1} = ((2m+1) F_m - e^-T) / (2T), whose error growth is largest at TS
+// (TS = 1 for M = 1, 2.125 for M = 2 and 3, 2.25 for 4, 3.25 above); for T < TS
+// F_M by interpolation in T - TS/2 (kBoysSmall) and the stable downward
+// recursion F_m = (2T F_{m+1} + e^-T) / (2m+1).  One rsqrt gives both 1/sqrt(T + 16)
 // and 1/T: r = 1 / (T sqrt(T + 16)).
 // T >= TA: the large-T limit F_0 = sqrt(pi / 4T), F_{m+1} = (2m+1) F_m /
 // (2T); TA = 34, 38, 42, 44, 46 for M = 0..4 is where the limit's relative
 // error (the dropped e^-T terms) falls to its own rounding level, 60 above.
 //
-// Largest relative error against 40-digit values: 4e-16 (M = 0), 7e-16 (1),
-// 1e-15 (2), 3e-15 (3), 5e-15 (4), 1e-14 (6); with the Taylor series below TS
-// and 1 - e^-T erfcx above, which this replaces, 1e-15 (M <= 1), 8e-15 (4),
-// 2e-14 (6).  The library's exp and erfcx keep their coefficients as
+// Largest relative error against 40-digit values, from 1500 points that lie
+// densest just above TS: 4.6e-16, 8.9e-16, 1.3e-15, 3.1e-15,
+// 6.1e-15, 7.0e-15, 1.7e-14 for M = 0 to 6; with the Taylor series
+// below TS (1, 2, 3) and 1 - e^-T erfcx above, which this replaces,
+// 3.9e-16, 1.1e-15, 1.6e-15, 3.2e-15, 7.2e-15, 9.7e-15, 1.9e-14.  The library's exp and erfcx keep their coefficients as
 // literals, and a warp paid for both branches: with them
 // (ss|ss) issued 160 instructions per primitive quartet, 26% of them FP64.
 // (H2O)32 / 6-31G**: (ss|ss) 3.16 -> 2.17 ms, (ps|ss) 5.56 -> 4.96; C40H82 /
@@ -125,7 +126,7 @@ __device__ __forceinline__ void boys_fm(double T, double *F)
         if (near) {
             const double e = boys_exp(T);
             if (T < TS) {
-                F[M] = poly_even_odd<kBoysSmallDeg[M]>(kBoysSmall[M], T);
+                F[M] = poly_even_odd<kBoysSmallDeg[M]>(kBoysSmall[M], T - 0.5 * TS);
 #pragma unroll
                 for (int m = M - 1; m >= 0; --m) F[m] = fma(2.0 * T, F[m + 1], e) * (1.0 / (2 * m + 1));
             } else {
@@ -139,7 +140,7 @@ __device__ __forceinline__ void boys_fm(double T, double *F)
                 for (int m = 0; m < M; ++m) F[m + 1] = fma(double(2 * m + 1), F[m], -e) * h;
             }
         } else {
-            // erfc(sqrt T) and e^-T are below 1e-17 of every (2m+1) F_m here
+            // what is left out is at most 6e-16 of F_m (m = 4 at T = 46), 2e-16 for m = 0
             F[0] = kHalfSqrtPi * r;
             const double h = 0.5 * r * r;
 #pragma unroll

@@ -19,6 +19,7 @@ import numpy as np
 import pytest
 
 mpmath = pytest.importorskip("mpmath")
+special = pytest.importorskip("scipy.special")
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "planck-refactored_b200", "csrc")
@@ -74,7 +75,7 @@ def boys(M, T):
     F = [0.0] * (M + 1)
     if near and T < ts:
         e = _exp(T)
-        F[M] = _even_odd(small, T)
+        F[M] = _even_odd(small, T - 0.5 * ts)
         for m in range(M - 1, -1, -1):
             F[m] = _fma(2.0 * T, F[m + 1], e) * (1.0 / (2 * m + 1))
         return F
@@ -130,4 +131,48 @@ def test_tables_are_the_generators():
         assert T_["kBoysMid"][M][:g.MID_DEG[M] + 1] == t["mid"][M]
         assert T_["kBoysSmall"][M][:g.SMALL_DEG[M] + 1] == t["small"][M]
     assert T_["kBoysExp"] == t["exp"] and T_["kBoysMidScale"] == t["mid_scale"]
-    assert [int(v) for v in T_["kBoysTA"]] == g.TA and [int(v) for v in T_["kBoysTS"]] == g.TS
+    assert T_["kBoysTA"] == g.TA and T_["kBoysTS"] == g.TS
+
+
+def _former(M, T):
+    """The scheme the polynomials replaced, with the C library's exp and
+    scipy's erfcx: the Taylor series of F_M and downward recursion below 1, 2
+    or 3, F_0 = sqrt(pi)/2 (1 - e^-T erfcx(sqrt T)) / sqrt T and upward
+    recursion above, the large-T limit from TA on."""
+    ts, nt = (1.0, 18) if M <= 1 else (2.0, 25) if M <= 4 else (3.0, 32)
+    F = [0.0] * (M + 1)
+    if T < ts:
+        s = 0.0
+        for k in range(nt - 1, -1, -1):
+            s = s * T + (-1) ** k / (math.factorial(k) * (2 * M + 2 * k + 1))
+        F[M], e = s, math.exp(-T)
+        for m in range(M - 1, -1, -1):
+            F[m] = (2.0 * T * F[m + 1] + e) * (1.0 / (2 * m + 1))
+        return F
+    ist, near = 1.0 / math.sqrt(T), T < T_["kBoysTA"][M]
+    e = math.exp(-T) if near else 0.0
+    F[0] = 0.88622692545275801365 * (1.0 - e * special.erfcx(T * ist) if near else 1.0) * ist
+    h = 0.5 * ist * ist
+    for m in range(M):
+        F[m + 1] = ((2 * m + 1) * F[m] - e) * h
+    return F
+
+
+@pytest.mark.parametrize("M", range(7))
+def test_no_less_accurate_than_the_former_scheme(M):
+    """Largest errors over points that lie densest just above either scheme's
+    switch to the upward recursion, where it amplifies most, and in the small
+    range.  One unit of 2^-53 for the sample at M = 0, whose errors are two to
+    four of them on either side."""
+    rng = np.random.default_rng(70 + M)
+    ts, ta, old = T_["kBoysTS"][M], T_["kBoysTA"][M], 1.0 if M <= 1 else 2.0 if M <= 4 else 3.0
+    Ts = np.concatenate([rng.uniform(ts, ts + 0.3, 500), rng.uniform(old, old + 0.3, 500), rng.uniform(0, ts, 150),
+                         rng.uniform(ts, ts + 3, 150), rng.uniform(ts, ta, 150), rng.uniform(ta, ta + 3, 50)])
+    new = former = 0.0
+    with mpmath.workdps(30):
+        for T in map(float, Ts):
+            ref = [_exact(m, mpmath.mpf(T)) for m in range(M + 1)]
+            err = [max(abs(float((f - r) / r)) for f, r in zip(F, ref)) for F in (boys(M, T), _former(M, T))]
+            new, former = max(new, err[0]), max(former, err[1])
+    print(f"M = {M}: {new:.2e}, former scheme {former:.2e}")
+    assert new <= former + (1.2e-16 if M == 0 else 0.0), (new, former)
