@@ -642,21 +642,6 @@ static int class_components(int c)
     return ncart(pc_la(x)) * ncart(pc_lb(x)) * ncart(pc_la(y)) * ncart(pc_lb(y));
 }
 
-// Lanes of the team that works on one quartet of class c: 1 in the
-// Obara-Saika and register kernels, SplitShape's in the split kernels.
-int class_team(int c)
-{
-    int x = 0;
-    while ((x + 1) * (x + 2) / 2 <= c) ++x;
-    const int y = c - x * (x + 1) / 2;
-    const int na = ncart(pc_la(x)), rest = ncart(pc_lb(x)) * ncart(pc_la(y)) * ncart(pc_lb(y));
-    if (quartet_class_L(c) <= kOSMaxL || na * rest <= 81) return 1;
-    const int group = rest <= 64 ? na : na * ncart(pc_lb(x));
-    int t = 4;
-    while (t < group) t *= 2;
-    return t;
-}
-
 // Segments of a sorted list (Segments) for this context's shard.  A bucket
 // of n quartets of 2^(b-1) < K <= 2^b primitive quartets gets enough lanes per
 // quartet to put kSplitLanes threads on the chip, but leaves every lane at

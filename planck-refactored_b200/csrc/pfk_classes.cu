@@ -12,7 +12,6 @@
 namespace pfk {
 namespace {
 
-constexpr int kRegMaxComponents = 81;   // register path up to (pp|pp)-sized blocks
 // The split kernels' SPLIT build exists for the s..d classes, whose basis sets
 // have contracted shells in molecules small enough to need it.
 template <int LA>
@@ -248,6 +247,10 @@ template <int C>
 void reg_range()
 {
     constexpr int X = cls_bra(C), Y = cls_ket(C);
+    using SS = SplitShape<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
+    constexpr bool split = pc_la(X) + pc_lb(X) + pc_la(Y) + pc_lb(Y) > kOSMaxL && SS::S::N > kRegMaxComponents && SS::OK;
+    static_assert(!split || class_team(C) == SS::TEAM, "list_segments counts in teams of the split kernel's size");
+    static_assert(split || SS::S::N > kRegMaxComponents || class_team(C) == 1, "register and OS kernels: one lane");
     g_class_launchers[C] = &launch_class<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
     g_class_waves[C] = &block_waves<pc_la(X), pc_lb(X), pc_la(Y), pc_lb(Y)>;
     if constexpr (C + 1 < PFK_CLASS_END) reg_range<C + 1>();

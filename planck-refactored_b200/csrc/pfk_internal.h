@@ -35,6 +35,25 @@ __host__ __device__ constexpr int quartet_class_L(int c)
 constexpr int kLaunchFP32 = 1, kLaunchOS = 2, kLaunchDense = 4, kLaunchShort = 8;
 constexpr int kOSMaxL = 4;
 
+// Register kernels take blocks of up to so many components ((pp|pp)).
+constexpr int kRegMaxComponents = 81;
+
+// Lanes of the team that works on one quartet of class c: 1 in the
+// Obara-Saika and register kernels, SplitShape::TEAM in the split kernels (the
+// class units assert that the two agree).
+constexpr int class_team(int c)
+{
+    int x = 0;
+    while ((x + 1) * (x + 2) / 2 <= c) ++x;
+    const int y = c - x * (x + 1) / 2;
+    const int na = ncart(pc_la(x)), rest = ncart(pc_lb(x)) * ncart(pc_la(y)) * ncart(pc_lb(y));
+    if (quartet_class_L(c) <= kOSMaxL || na * rest <= kRegMaxComponents) return 1;
+    const int group = rest <= 64 ? na : na * ncart(pc_lb(x));
+    int t = 4;
+    while (t < group) t *= 2;
+    return t;
+}
+
 // One launcher per quartet class.  nk = number of exchange densities (1 or 2).
 using ClassLauncher = void (*)(const uint2 *quartets, long long n, const JKArgs &args, int nk, int flags,
                                cudaStream_t st);
