@@ -2290,6 +2290,7 @@ int ctx_device(const pfk_ctx *ctx) { return ctx->device; }
 pfk_status fock_rhf_direct(pfk_ctx *ctx, const double *dP, double *dG, cudaStream_t st)
 {
     cudaSetDevice(ctx->device);
+    ctx->direct_builds = kWideAfter;   // an SCF loop repeats its builds
     return rhf_sequence(ctx, dP, dG, st);
 }
 pfk_status ctx_fail(pfk_ctx *ctx, pfk_status s, const std::string &msg) { return ctx->fail(s, msg); }
