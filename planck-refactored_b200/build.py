@@ -1,9 +1,12 @@
 """Build libplanck_fock.so (sm_100a) in-tree.
 
-nvcc compiles the ten bra-class translation units of pfk_classes.cu, the
+nvcc compiles pfk_classes.cu once per quartet class (55 translation units), the
 setup kernels and the C ABI in parallel into _build/, then links the shared
 library next to this file.  Objects are rebuilt when any source under csrc/
-or include/ is newer than them.
+or include/ is newer than they are.  nvcc writes under another name, and what it
+wrote becomes the object when it is complete, with the time at which the
+compilation began: an interrupted build, or a source edited during one, leaves
+nothing that looks current.
 
     python build.py [-j N] [--force]
 """
@@ -12,6 +15,7 @@ import concurrent.futures as cf
 import os
 import subprocess
 import sys
+import time
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 REPO = os.path.dirname(HERE)
@@ -56,12 +60,20 @@ def _newest(src):
 
 
 def _compile(src, obj, extra, verbose):
-    cmd = [NVCC] + ARCH + FLAGS + extra + ["-c", os.path.join(CSRC, src), "-o", obj]
+    part = f"{obj}.{os.getpid()}.part"
+    cmd = [NVCC] + ARCH + FLAGS + extra + ["-c", os.path.join(CSRC, src), "-o", part]
     if verbose:
         cmd.insert(1, "-Xptxas=-v")
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"nvcc failed for {src} {extra}:\n{r.stderr[-6000:]}")
+    began = time.time()
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"nvcc failed for {src} {extra}:\n{r.stderr[-6000:]}")
+        os.utime(part, (began, began))
+        os.replace(part, obj)
+    finally:
+        if os.path.exists(part):
+            os.remove(part)
     return r.stderr
 
 
@@ -80,8 +92,13 @@ def build(jobs=None, force=False, verbose=False):
                 logs[futs[f][1]] = f.result()
     objs = [os.path.join(BUILD, o) for _, o, _ in _units()]
     if todo or not os.path.exists(LIB) or os.path.getmtime(LIB) < max(os.path.getmtime(o) for o in objs):
-        cmd = [NVCC] + ARCH + ["-shared", "-o", LIB] + objs + ["-lcudart", "-lcublas", "-lcusolver"]
-        subprocess.check_call(cmd)
+        part = f"{LIB}.{os.getpid()}.part"
+        try:
+            subprocess.check_call([NVCC] + ARCH + ["-shared", "-o", part] + objs + ["-lcudart", "-lcublas", "-lcusolver"])
+            os.replace(part, LIB)
+        finally:
+            if os.path.exists(part):
+                os.remove(part)
     return LIB, logs
 
 
