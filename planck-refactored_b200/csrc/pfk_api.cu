@@ -80,7 +80,9 @@ struct GraphEntry {
 // lasts as long as one quartet's chain of loads, recurrences and adds (20 to
 // 60 us), so what counts is how many run at once: one water / 6-31G** 175 us a
 // build with 4, 115 with 12; (H2O)5 464 and 447; (H2O)4 / 3-21G 104 and 88.
-// More than 4 were slower for (H2O)32 (49.8 ms with 4, 50.4 with 6, 50.6 with 8).
+// More than 4 were slower for (H2O)32 (49.8 ms with 4, 50.4 with 6, 50.6 with
+// 8).  The line: 12 against 4 take 4.5% less for 1.0 M quartets ((H2O)5), 1.1%
+// less for 3.2 M ((H2O)7), 2% more for 4.4 M ((H2O)9, C6H14 / cc-pVDZ).
 //
 // But 12 branches take 0.1 (water / 3-21G) to 0.45 ms (6-31G**) longer to
 // instantiate than 4 and as much longer to destroy, and eight more streams 0.4
@@ -647,10 +649,21 @@ static int class_components(int c)
 // quartet to put kSplitLanes threads on the chip, but leaves every lane at
 // least kSplitPrims primitive quartets (the lanes' sums cost five shuffles
 // per contracted value).
+//
+// Build times with kSplitLanes at 2^15, 2^16, 2^17: water / 6-31G** 88 us with
+// all; (H2O)5 359, 365, 367 us; pentane / cc-pVDZ 1.67, 1.77, 1.86 ms (2^18:
+// 1.98); C8H18 / 6-31G* 1.27, 1.32, 1.40; (H2O)32 45.9, 46.0, 46.4; but C40H82 /
+// cc-pVDZ 222.6, 222.7, 219.8, where the longest loops are the end of each
+// class's kernel.  One line for all of them keeps the longest build.
 constexpr long long kSplitLanes = 1 << 17;
 // In the split kernels the unit is a team of `team` lanes, of which a block of
 // 128 threads can give a quartet 128 / team at most; a primitive quartet there
 // is 1 to 2 us of dependent steps, so two of them are worth a team.
+//
+// kSplitPrims 4, 8, 16: water / 6-31G** 80, 88, 106 us;
+// (H2O)5 408, 367, 349; ethane / cc-pVDZ 189, 176, 198; pentane 1990, 1862, 1764;
+// no lanes at all 434, 563, 2072, 2931.  kSplitTeamPrims 1, 2, 4, none: water
+// 84, 88, 95, 110; (H2O)5 424, 367, 357, 351; ethane 176, 176, 187, 268.
 constexpr int kSplitPrims = 8, kSplitTeamPrims = 2;
 void list_segments(const pfk_ctx *ctx, const long long *bucket0, long long n, int team, Segments &sg)
 {
