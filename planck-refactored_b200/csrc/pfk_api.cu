@@ -888,10 +888,15 @@ pfk_status ensure_work(pfk_ctx *ctx)
 // three at work in turn a call that had to allocate took 4.5 ms instead of 2.4).
 constexpr size_t kMoKeepBytes = size_t(4) << 30;
 std::atomic<size_t> g_mo_kept[64];   // by device (mod 64: devices that share an entry share the limit)
-size_t mo_keep_limit()
+size_t mo_keep_limit(int device)
 {
-    size_t avail = 0, total = 0;
-    return cudaMemGetInfo(&avail, &total) == cudaSuccess ? total / 16 : 0;
+    static std::atomic<size_t> limit[64];   // asked for once: cudaMemGetInfo takes up to milliseconds
+    std::atomic<size_t> &l = limit[device & 63];
+    if (!l) {
+        size_t avail = 0, total = 0;
+        if (cudaMemGetInfo(&avail, &total) == cudaSuccess) l = total / 16;
+    }
+    return l;
 }
 void mo_release(pfk_ctx *ctx, bool all)
 {
@@ -903,7 +908,7 @@ void mo_release(pfk_ctx *ctx, bool all)
     kept -= ctx->mo_kept;
     ctx->mo_kept = 0;
     if (!all && bytes <= kMoKeepBytes) {
-        if (kept.fetch_add(bytes) + bytes <= mo_keep_limit()) {
+        if (kept.fetch_add(bytes) + bytes <= mo_keep_limit(ctx->device)) {
             ctx->mo_kept = bytes;
             return;
         }
